@@ -109,6 +109,19 @@ __device__ __forceinline__ void neighbor_rows(const DevParams &P, int c, Rows &r
     }
 }
 
+// f(c0, c1) for the cell rows [c0, c1) within `reach` cells of cell c on each axis.
+template <class F>
+__device__ __forceinline__ void for_rows_within(const DevParams &P, int c, int reach, F &&f)
+{
+    const int row = c / P.nz, cz = c - row * P.nz, cx = row / P.ny, cy = row - cx * P.ny;
+    const int z0 = max(cz - reach, 0), z1 = min(cz + reach, P.nz - 1) + 1;
+    for (int x = max(cx - reach, 0); x <= min(cx + reach, P.nx - 1); ++x)
+        for (int y = max(cy - reach, 0); y <= min(cy + reach, P.ny - 1); ++y) {
+            const int base = (x * P.ny + y) * P.nz;
+            f(base + z0, base + z1);
+        }
+}
+
 // ------------------------------------------------------- batched launches
 // Every step kernel has a body taking (params, args, local block index) and a
 // batched wrapper: one launch serves many instances, each with its own
@@ -135,6 +148,27 @@ __device__ __forceinline__ int locate_instance(const int *__restrict__ bstart, i
         const DevParams P = items[inst].P;                                                                \
         const ARGS &A = items[inst].A;                                                                    \
         BODY(P, A, (int)blockIdx.x - bstart[inst]);                                                       \
+    }
+
+// The list rebuild's kernels work on the plan's rebuilding instances only, which
+// the list decision (kb_nl_decide) has written to act: act[0] of them, act[2 + k]
+// the k-th; an instance has `per` consecutive items.  One modest grid for the
+// whole plan walks all their blocks in turn, so a step without a rebuild costs
+// an almost empty launch, and the rebuilding instances of a batch share the
+// whole GPU whatever their number (grids sized per instance, 8 blocks per SM
+// and more for each of 64, cost 15-25 us per idle launch).
+#define FSIM_REBUILD_KERNEL(NAME, ARGS, BODY, BOUNDS, BLOCKS)                                              \
+    __global__ void __launch_bounds__(BOUNDS) NAME(const Item<ARGS> *__restrict__ items,                 \
+                                                   const int *__restrict__ act, int per)                  \
+    {                                                                                                     \
+        int b = blockIdx.x;                                                                               \
+        for (int k = 0, n = act[0] * per; k < n; ++k) {                                                   \
+            const Item<ARGS> &it = items[act[2 + k / per] * per + k % per];                               \
+            const ARGS &A = it.A;                                                                         \
+            const int nb = (BLOCKS);                                                                      \
+            for (; b < nb; b += gridDim.x) BODY(it.P, A, b);                                              \
+            b -= nb;                                                                                      \
+        }                                                                                                 \
     }
 
 // The same kernel in two more launch forms whose parameters sit in the constant
@@ -170,39 +204,26 @@ __device__ __forceinline__ int cell_slot(int *cnt, int c, bool active)
     return base + __popc(peers & ((1u << lane) - 1u));
 }
 
-// the element blocks an item's block `blk` covers: blk, blk + grid, ... (all of
-// them when the item is launched with one block per element block)
-#define FSIM_ELEMENT_BLOCKS(A, blk, b)                                                                     \
-    for (int b = (blk), nb_ = blocks_for((A).n, (int)blockDim.x), st_ = (A).grid ? (A).grid : nb_; b < nb_; \
-         b += st_)
-
 __device__ __forceinline__ void hash_body(const DevParams &P, const HashArgs &A, int blk)
 {
-    if (A.gate && !*A.gate) return; // uniform per block
-    FSIM_ELEMENT_BLOCKS(A, blk, b)
-    {
-        const int s = b * blockDim.x + threadIdx.x;
-        const bool active = s < A.n;
-        int c = 0;
-        if (active) {
-            const float4 p = A.pos[s];
-            c = cell_index(P, p.x, p.y, p.z, A.flags);
-            A.key[s] = c;
-        }
-        const int slot = cell_slot(A.cnt, c, active);
-        if (active) A.slot[s] = slot;
+    const int s = blk * blockDim.x + threadIdx.x;
+    const bool active = s < A.n;
+    int c = 0;
+    if (active) {
+        const float4 p = A.pos[s];
+        c = cell_index(P, p.x, p.y, p.z, A.flags);
+        A.key[s] = c;
     }
+    const int slot = cell_slot(A.cnt, c, active);
+    if (active) A.slot[s] = slot;
 }
 FSIM_BATCHED_KERNEL(kb_hash, HashArgs, hash_body, kBlock)
+FSIM_REBUILD_KERNEL(kg_hash, HashArgs, hash_body, kBlock, blocks_for(A.n, kBlock))
 
 __device__ __forceinline__ void zero_body(const DevParams &, const ZeroArgs &A, int blk)
 {
-    if (A.gate && !*A.gate) return;
-    FSIM_ELEMENT_BLOCKS(A, blk, b)
-    {
-        const int s = b * blockDim.x + threadIdx.x;
-        if (s < A.n) A.p[s] = 0;
-    }
+    const int s = blk * blockDim.x + threadIdx.x;
+    if (s < A.n) A.p[s] = 0;
 }
 FSIM_BATCHED_KERNEL(kb_zero, ZeroArgs, zero_body, kBlock)
 
@@ -242,7 +263,6 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *total)
 // scan pass 1: per-tile sums (one block per 4096-entry tile)
 __device__ __forceinline__ void scan_reduce_body(const DevParams &, const ScanArgs &J, int blk)
 {
-    if (J.gate && !*J.gate) return; // uniform per block
     const int base = blk * kScanTile + threadIdx.x * kScanItems;
     int s = 0;
 #pragma unroll
@@ -253,11 +273,11 @@ __device__ __forceinline__ void scan_reduce_body(const DevParams &, const ScanAr
     if (threadIdx.x == 0) J.partial[blk] = total;
 }
 FSIM_BATCHED_KERNEL(kb_scan_reduce, ScanArgs, scan_reduce_body, kScanThreads)
+FSIM_REBUILD_KERNEL(kg_scan_reduce, ScanArgs, scan_reduce_body, kScanThreads, blocks_for(A.n, kScanTile))
 
 // scan pass 2: exclusive scan of the tile sums (one block per array)
 __device__ __forceinline__ void scan_partials_body(const DevParams &, const ScanArgs &J, int)
 {
-    if (J.gate && !*J.gate) return;
     const int tiles = blocks_for(J.n, kScanTile);
     int carry = 0;
     for (int b0 = 0; b0 < tiles; b0 += kScanThreads) {
@@ -271,11 +291,11 @@ __device__ __forceinline__ void scan_partials_body(const DevParams &, const Scan
     if (threadIdx.x == 0) J.out[J.n] = carry;
 }
 FSIM_BATCHED_KERNEL(kb_scan_partials, ScanArgs, scan_partials_body, kScanThreads)
+FSIM_REBUILD_KERNEL(kg_scan_partials, ScanArgs, scan_partials_body, kScanThreads, A.n > 0 ? 1 : 0)
 
 // scan pass 3: scan inside each tile plus its offset
 __device__ __forceinline__ void scan_apply_body(const DevParams &, const ScanArgs &J, int blk)
 {
-    if (J.gate && !*J.gate) return;
     const int base = blk * kScanTile + threadIdx.x * kScanItems;
     int v[kScanItems];
     int s = 0;
@@ -293,21 +313,19 @@ __device__ __forceinline__ void scan_apply_body(const DevParams &, const ScanArg
     }
 }
 FSIM_BATCHED_KERNEL(kb_scan_apply, ScanArgs, scan_apply_body, kScanThreads)
+FSIM_REBUILD_KERNEL(kg_scan_apply, ScanArgs, scan_apply_body, kScanThreads, blocks_for(A.n, kScanTile))
 
 __device__ __forceinline__ void scatter_body(const DevParams &, const ScatterArgs &A, int blk)
 {
-    if (A.gate && !*A.gate) return;
-    FSIM_ELEMENT_BLOCKS(A, blk, b)
-    {
-        const int s = b * blockDim.x + threadIdx.x;
-        if (s >= A.n) continue;
-        const int c = A.key[s];
-        FSIM_DCHECK(A.start[c] + A.slot[s] >= 0 && A.start[c] + A.slot[s] < A.n, 8192u, continue);
-        A.tmp[A.start[c] + A.slot[s]] = s;
-        if (A.reset) A.reset[c] = 0; // the counts are spent: zero for the next sort
-    }
+    const int s = blk * blockDim.x + threadIdx.x;
+    if (s >= A.n) return;
+    const int c = A.key[s];
+    FSIM_DCHECK(A.start[c] + A.slot[s] >= 0 && A.start[c] + A.slot[s] < A.n, 8192u, return);
+    A.tmp[A.start[c] + A.slot[s]] = s;
+    if (A.reset) A.reset[c] = 0; // the counts are spent: zero for the next sort
 }
 FSIM_BATCHED_KERNEL(kb_scatter, ScatterArgs, scatter_body, kBlock)
+FSIM_REBUILD_KERNEL(kg_scatter, ScatterArgs, scatter_body, kBlock, blocks_for(A.n, kBlock))
 
 // Rank inside the cell by previous position: the new order is sorted by
 // (cell, previous sorted position), a stable and deterministic order.  The
@@ -482,17 +500,17 @@ __device__ __forceinline__ float rcp_approx(float x)
 }
 
 // LIMITER: min(3 du, c0) (fluid, wall) or c0 (solid).  clamp_ps: P* >= 0 (wall).
-// KAHAN: the density-rate sum is Kahan-compensated (mixed form).
-template <bool LIMITER, int VISCID, bool KAHAN = false>
-__device__ __forceinline__ void riemann_pair(const DevParams &P, float dx, float dy, float dz, float r2, float uix,
-                                             float uiy, float uiz, float rhoi, float pi, float ujx, float ujy,
-                                             float ujz, float rhoj, float pj, bool clamp_ps, PairAcc &A)
+// The terms of one pair: drho += x w, a += f (dx, dy, dz).
+// EXACT (mixed form): every rounding spelled out (no contraction freedom left to
+// the compiler), so that every kernel inlining this rounds identically.
+template <bool LIMITER, int VISCID, bool EXACT = false>
+__device__ __forceinline__ void riemann_terms(const DevParams &P, float dx, float dy, float dz, float r2, float uix,
+                                              float uiy, float uiz, float rhoi, float pi, float ujx, float ujy,
+                                              float ujz, float rhoj, float pj, bool clamp_ps, float &x, float &w,
+                                              float &f)
 {
-    if (KAHAN) {
-        // The same terms with every rounding spelled out (no contraction
-        // freedom left to the compiler), so that every kernel inlining this
-        // rounds identically, and a Kahan-compensated density-rate sum.
-        const float w = __fmul_rn(ex2_approx(__fmul_rn(r2, P.exp2_scale)), P.kdiff);
+    if (EXACT) {
+        w = __fmul_rn(ex2_approx(__fmul_rn(r2, P.exp2_scale)), P.kdiff);
         const float inv_r = rsqrt_approx(fmaxf(r2, 1e-30f));
         const float rs_inv = rcp_approx(__fadd_rn(rhoi, rhoj));
         const float a = fmaf(__fsub_rn(uiz, ujz), dz, fmaf(__fsub_rn(uiy, ujy), dy, __fmul_rn(__fsub_rn(uix, ujx), dx)));
@@ -502,21 +520,14 @@ __device__ __forceinline__ void riemann_pair(const DevParams &P, float dx, float
         ps = fmaf(__fmul_rn(__fmul_rn(__fmul_rn(rhoi, rhoj), rs_inv), du), lim, ps);
         if (clamp_ps) ps = fmaxf(ps, 0.0f);
         const float r = __fmul_rn(r2, inv_r);
-        const float x = fmaf(rhoj, a, -__fmul_rn(__fmul_rn(__fsub_rn(pi, pj), r), P.c0_inv));
-        const float y = __fsub_rn(__fmul_rn(__fmul_rn(x, rs_inv), w), A.drho_c);
-        const float t = __fadd_rn(A.drho, y);
-        A.drho_c = __fsub_rn(__fsub_rn(t, A.drho), y);
-        A.drho = t;
-        float f = __fmul_rn(-2.0f, ps);
+        x = __fmul_rn(fmaf(rhoj, a, -__fmul_rn(__fmul_rn(__fsub_rn(pi, pj), r), P.c0_inv)), rs_inv);
+        f = __fmul_rn(-2.0f, ps);
         if (VISCID == 1 || (VISCID == 2 && P.viscid))
             f = fmaf(__fmul_rn(P.mu10, -a), rcp_approx(__fadd_rn(r2, P.eps_h2)), f);
         f = __fmul_rn(f, w);
-        A.ax = fmaf(f, dx, A.ax);
-        A.ay = fmaf(f, dy, A.ay);
-        A.az = fmaf(f, dz, A.az);
         return;
     }
-    const float w = ex2_approx(r2 * P.exp2_scale) * P.kdiff;
+    w = ex2_approx(r2 * P.exp2_scale) * P.kdiff;
     const float inv_r = rsqrt_approx(fmaxf(r2, 1e-30f)); // r2 = 0 (the particle itself) contributes 0
     const float rs_inv = rcp_approx(rhoi + rhoj);
     const float a = (uix - ujx) * dx + (uiy - ujy) * dy + (uiz - ujz) * dz;
@@ -526,10 +537,33 @@ __device__ __forceinline__ void riemann_pair(const DevParams &P, float dx, float
     ps = fmaf(rhoi * rhoj * rs_inv * du, lim, ps);
     if (clamp_ps) ps = fmaxf(ps, 0.0f);
     const float r = r2 * inv_r;
-    A.drho = fmaf((rhoj * a - (pi - pj) * r * P.c0_inv) * rs_inv, w, A.drho);
-    float f = -2.0f * ps;
+    x = (rhoj * a - (pi - pj) * r * P.c0_inv) * rs_inv;
+    f = -2.0f * ps;
     if (VISCID == 1 || (VISCID == 2 && P.viscid)) f = fmaf(P.mu10 * -a, rcp_approx(r2 + P.eps_h2), f);
     f *= w;
+}
+
+// sum += x w with Kahan's compensation c (mixed form), where `in`
+__device__ __forceinline__ void kahan_add(float x, float w, bool in, float &sum, float &c)
+{
+    const float y = __fsub_rn(__fmul_rn(x, w), c), t = __fadd_rn(sum, y);
+    const float d = __fsub_rn(__fsub_rn(t, sum), y);
+    sum = in ? t : sum;
+    c = in ? d : c;
+}
+
+// Adds one pair to the sums.  KAHAN: the density-rate sum is Kahan-compensated
+// (mixed form).
+template <bool LIMITER, int VISCID, bool KAHAN = false>
+__device__ __forceinline__ void riemann_pair(const DevParams &P, float dx, float dy, float dz, float r2, float uix,
+                                             float uiy, float uiz, float rhoi, float pi, float ujx, float ujy,
+                                             float ujz, float rhoj, float pj, bool clamp_ps, PairAcc &A)
+{
+    float x, w, f;
+    riemann_terms<LIMITER, VISCID, KAHAN>(P, dx, dy, dz, r2, uix, uiy, uiz, rhoi, pi, ujx, ujy, ujz, rhoj, pj,
+                                          clamp_ps, x, w, f);
+    if (KAHAN) kahan_add(x, w, true, A.drho, A.drho_c);
+    else A.drho = fmaf(x, w, A.drho);
     A.ax = fmaf(f, dx, A.ax);
     A.ay = fmaf(f, dy, A.ay);
     A.az = fmaf(f, dz, A.az);
@@ -784,26 +818,16 @@ __global__ void __launch_bounds__(SH::warps * 32) kb_fluid_sweep_p(const __grid_
 // keep the order of the last build between builds; the other phases walk a
 // per-step cell index (kb_rank) instead.
 
-// One block per instance at the start of every step: rebuild when forced or
-// when the largest displacement since the last build (fluid: accumulated by
-// the last sweep; solid: measured here) exceeds the allowance.
-__device__ __forceinline__ void nl_decide_body(const DevParams &, const NlDecideArgs &A, int blk)
+// At the start of every step, per instance: rebuild when forced or when the
+// largest displacement since the last build (fluid: accumulated by the last
+// sweep; solid: measured here) exceeds the allowance.  The last instance of the
+// plan to decide lists the rebuilding ones for the rebuild's kernels.
+__device__ __forceinline__ bool nl_decide_instance(const NlDecideArgs &A, unsigned m)
 {
-    __shared__ unsigned wmax[kBlock / 32];
-    unsigned m = 0;
-    for (int i = blk * blockDim.x + threadIdx.x; i < A.ns; i += A.nblocks * blockDim.x) {
-        const float4 p = A.s_pos[i], o = A.s_x0[i];
-        m = max(m, __float_as_uint(dist2(p.x - o.x, p.y - o.y, p.z - o.z)));
-    }
-    m = __reduce_max_sync(kFull, m);
-    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x) return;
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = max(m, wmax[w]);
     NlState &S = *A.nl;
     if (m) atomicMax(&S.maxd2, m); // NaN bits compare above every distance
     __threadfence();
-    if (atomicAdd(&S.ticket, 1u) != (unsigned)A.nblocks - 1u) return;
+    if (atomicAdd(&S.ticket, 1u) != (unsigned)A.nblocks - 1u) return false;
     // the last block: every block's maximum (and the last sweep's) is in maxd2
     __threadfence();
     const float d2 = __uint_as_float(atomicMax(&S.maxd2, 0u));
@@ -816,133 +840,165 @@ __device__ __forceinline__ void nl_decide_body(const DevParams &, const NlDecide
         S.builds += 1;
         S.overflow = 0;
     }
+    __threadfence();
+    return atomicAdd(reinterpret_cast<unsigned *>(A.act + 1), 1u) == (unsigned)A.ninst - 1u;
 }
-FSIM_BATCHED_KERNEL(kb_nl_decide, NlDecideArgs, nl_decide_body, kBlock)
 
-// The list build: the sweep's warp-uniform candidate stream (a warp's lanes of
-// one cell row walk the union of their 9 neighbour rows) over the list grid,
-// testing r^2 < Rs^2; hits collect in a per-lane shared-memory list that is
-// appended to the lane's global list in candidate order.  Per particle: its
-// fluid, then wall, then solid candidates, in row order -- the order in which
-// the stream sweep sums them.
-constexpr int kNlBuildWarps = kNlBuildThreads / 32, kNlBuildCap = 32, kNlBuildChunk = 8;
-
-// Append a lane's pending hits lst[0..cnt) to its list in whole groups of
-// kNlGroup entries (two 16-byte stores: a full sector); the remainder stays
-// pending at the front.  `tot` counts the entries stored so far; the final
-// flush stores the last partial group padded with -1 and makes `tot` exact.
-__device__ __forceinline__ void nl_flush(const NlBuildArgs &A, int (*lst)[32], int lane, int i, int &cnt, int &tot,
-                                         bool last)
+__global__ void __launch_bounds__(kBlock) kb_nl_decide(const Item<NlDecideArgs> *__restrict__ items,
+                                                       const int *__restrict__ bstart, int ninst)
 {
-    const int full = last ? (cnt + kNlGroup - 1) / kNlGroup : cnt / kNlGroup;
-    const int mfull = __reduce_max_sync(kFull, full);
-    for (int g = 0; g < mfull; ++g) {
-        const int grp = tot / kNlGroup + g;
-        if (g < full && grp * kNlGroup < A.cap) {
-            int v[kNlGroup];
+    const int inst = locate_instance(bstart, ninst, blockIdx.x), blk = (int)blockIdx.x - bstart[inst];
+    const NlDecideArgs &A = items[inst].A;
+    __shared__ unsigned wmax[kBlock / 32];
+    __shared__ int last;
+    unsigned m = 0;
+    for (int i = blk * blockDim.x + threadIdx.x; i < A.ns; i += A.nblocks * blockDim.x) {
+        const float4 p = A.s_pos[i], o = A.s_x0[i];
+        m = max(m, __float_as_uint(dist2(p.x - o.x, p.y - o.y, p.z - o.z)));
+    }
+    m = __reduce_max_sync(kFull, m);
+    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = max(m, wmax[w]);
+        last = nl_decide_instance(A, m);
+    }
+    __syncthreads();
+    if (!last || threadIdx.x >= 32) return;
+    __threadfence();
+    int n = 0;
+    for (int k0 = 0; k0 < ninst; k0 += 32) {
+        const int k = k0 + (int)threadIdx.x;
+        const bool rb = k < ninst && *(volatile int *)&items[k].A.nl->rebuild;
+        const unsigned set = __ballot_sync(kFull, rb);
+        if (rb) A.act[2 + n + __popc(set & ((1u << threadIdx.x) - 1u))] = k;
+        n += __popc(set);
+    }
+    if (threadIdx.x == 0) {
+        A.act[0] = n;
+        A.act[1] = 0;
+    }
+}
+
+// The list build, one lane per particle: the list grid's cells are a fraction
+// 1 / reach of the list radius, so the candidates of a particle are the cells
+// within `reach` of its own -- (2 reach + 1)^2 rows (x, y), each one z-contiguous
+// index range.  Particles are sorted on that grid, so a column of cells holds
+// its particles in z order and a warp's lanes are (nearly) consecutive in it:
+// their candidate loads are shifted copies of one another and coalesce.  Hits
+// (r^2 < Rs^2) collect in a two-group ring per lane in shared memory and leave
+// in whole groups.  Per particle: its fluid, then wall, then solid candidates,
+// in row order.
+constexpr int kNlBuildWarps = kNlBuildThreads / 32, kNlBuildRing = 2 * kNlGroup;
+
+// Store group `grp` of the lane's list from the ring (entries past `tot` as -1):
+// two 16-byte stores, a full sector.
+__device__ __forceinline__ void nl_store_group(const NlBuildArgs &A, int (*ring)[32], int lane, int i, int grp, int tot)
+{
+    if (grp * kNlGroup >= A.cap) return;
+    int v[kNlGroup];
 #pragma unroll
-            for (int q = 0; q < kNlGroup; ++q) {
-                const int k = g * kNlGroup + q;
-                v[q] = k < cnt ? lst[k][lane] : -1;
-            }
-            int4 *dst = reinterpret_cast<int4 *>(A.list + ((size_t)grp * A.n + i) * kNlGroup);
-            __stcs(dst, make_int4(v[0], v[1], v[2], v[3])); // streaming: keep the positions in L2
-            __stcs(dst + 1, make_int4(v[4], v[5], v[6], v[7]));
-        }
+    for (int q = 0; q < kNlGroup; ++q) {
+        const int k = grp * kNlGroup + q;
+        v[q] = k < tot ? ring[k & (kNlBuildRing - 1)][lane] : -1;
     }
-    if (last) {
-        tot += cnt;
-        cnt = 0;
-        return;
-    }
-    const int rem = cnt - full * kNlGroup; // < kNlGroup; moves down from index >= kNlGroup (or stays put)
-    for (int q = 0; q < rem; ++q) lst[q][lane] = lst[full * kNlGroup + q][lane];
-    tot += full * kNlGroup;
-    cnt = rem;
+    int4 *dst = reinterpret_cast<int4 *>(A.list + ((size_t)grp * A.n + i) * kNlGroup);
+    __stcs(dst, make_int4(v[0], v[1], v[2], v[3])); // streaming: keep the positions in L2
+    __stcs(dst + 1, make_int4(v[4], v[5], v[6], v[7]));
 }
 
 template <int SP>
-__device__ __forceinline__ void nl_gather(const DevParams &P, const NlBuildArgs &A, int (*lst)[32], int lane, int i,
-                                          int &cnt, int &tot, bool in, int cx, int cy, int z0, int z1, float4 pr)
+__device__ __forceinline__ void nl_gather(const DevParams &P, const NlBuildArgs &A, int (*ring)[32], int lane, int i,
+                                          bool valid, int &tot, int cx, int cy, int cz, float4 pr)
 {
-    const int *start = SP == 0 ? A.start_f : SP == 1 ? A.start_v : A.start_s;
-    const float4 *pos = SP == 0 ? A.posr : SP == 1 ? A.v_posr : A.s_pos;
-    const int tag = (int)((unsigned)SP << kNlSpeciesShift);
-    for (int ox = -1; ox <= 1; ++ox) {
-        const int x = cx + ox;
-        if (x < 0 || x >= P.nx) continue;
-        for (int oy = -1; oy <= 1; ++oy) {
-            const int y = cy + oy;
-            if (y < 0 || y >= P.ny) continue;
-            const int base = (x * P.ny + y) * P.nz;
-            int j = start[base + z0];
-            const int je = start[base + z1];
-            while (j < je) {
-                if (__reduce_max_sync(kFull, cnt) > kNlBuildCap - kNlBuildChunk)
-                    nl_flush(A, lst, lane, i, cnt, tot, false);
-                const int jend = min(j + kNlBuildChunk, je);
-#pragma unroll 4
-                for (; j < jend; ++j) {
-                    FSIM_DCHECK(j < (SP == 0 ? A.n : SP == 1 ? A.nv : A.ns), 2u, continue);
-                    const float4 q = pos[j]; // same address in every lane: a broadcast
-                    const float r2 = dist2(q.x - pr.x, q.y - pr.y, q.z - pr.z);
-                    if (in && r2 < A.R2s) lst[cnt++][lane] = j | tag;
+    const int *__restrict__ start = SP == 0 ? A.start_f : SP == 1 ? A.start_v : A.start_s;
+    const float4 *__restrict__ pos = SP == 0 ? A.posr : SP == 1 ? A.v_posr : A.s_pos;
+    const int K = A.reach;
+#pragma unroll 1
+    for (int ox = -K; ox <= K; ++ox) {
+        const int x = cx + ox, mx = max(abs(ox) - 1, 0);
+        const bool inx = valid && x >= 0 && x < P.nx;
+#pragma unroll 1
+        for (int oy = -K; oy <= K; ++oy) {
+            const int y = cy + oy, my = max(abs(oy) - 1, 0);
+            int zr = K; // cells of this row that can hold a point within reach
+            while ((zr - 1) * (zr - 1) + mx * mx + my * my >= K * K) --zr;
+            int j = 0, je = 0;
+            if (inx && y >= 0 && y < P.ny) {
+                const int base = (x * P.ny + y) * P.nz;
+                j = start[base + max(cz - zr, 0)];
+                je = start[base + min(cz + zr, P.nz - 1) + 1];
+            }
+            for (; j < je; j += kNlGroup) {
+                const int grp = tot / kNlGroup;
+#pragma unroll
+                for (int c = 0; c < kNlGroup; ++c) {
+                    if (j + c < je) {
+                        FSIM_DCHECK(j + c < (SP == 0 ? A.n : SP == 1 ? A.nv : A.ns), 2u, continue);
+                        const float4 q = pos[j + c];
+                        const float r2 = dist2(q.x - pr.x, q.y - pr.y, q.z - pr.z);
+                        if (r2 < A.R2s) {
+                            ring[tot & (kNlBuildRing - 1)][lane] = j + c;
+                            ++tot;
+                        }
+                    }
                 }
+                if (tot / kNlGroup != grp) nl_store_group(A, ring, lane, i, grp, tot);
             }
         }
     }
 }
 
-__device__ __forceinline__ void nl_build_block(const DevParams &P, const NlBuildArgs &A, int blk);
-
 __device__ __forceinline__ void nl_build_body(const DevParams &P, const NlBuildArgs &A, int blk)
 {
-    if (!A.nl->rebuild) return; // uniform per block
-    FSIM_ELEMENT_BLOCKS(A, blk, b) nl_build_block(P, A, b);
-}
-
-__device__ __forceinline__ void nl_build_block(const DevParams &P, const NlBuildArgs &A, int blk)
-{
-    __shared__ int lists[kNlBuildWarps][kNlBuildCap][32];
+    __shared__ int rings[kNlBuildWarps][kNlBuildRing][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = (blk * kNlBuildWarps + warp) * 32 + lane;
     const bool valid = i < A.n;
-    int(*lst)[32] = lists[warp];
+    int(*ring)[32] = rings[warp];
     const float4 pr = valid ? A.posr[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const int cell = valid ? A.cell_f[i] : 0;
-    const int row = cell / P.nz, cz = cell - row * P.nz;
-    int cnt = 0, tot = 0;
-    unsigned remaining = __ballot_sync(kFull, valid);
-    while (remaining) {
-        const int leader = __ffs(remaining) - 1;
-        const int grow = __shfl_sync(kFull, row, leader);
-        const unsigned grp = __ballot_sync(kFull, valid && row == grow);
-        remaining &= ~grp;
-        const bool in = (grp >> lane) & 1u;
-        const int zlo = __reduce_min_sync(kFull, in ? cz : INT_MAX);
-        const int zhi = __reduce_max_sync(kFull, in ? cz : INT_MIN);
-        const int z0 = max(zlo - 1, 0), z1 = min(zhi + 1, P.nz - 1) + 1;
-        const int cx = grow / P.ny, cy = grow - cx * P.ny;
-        nl_gather<0>(P, A, lst, lane, i, cnt, tot, in, cx, cy, z0, z1, pr);
-        nl_gather<1>(P, A, lst, lane, i, cnt, tot, in, cx, cy, z0, z1, pr);
-        nl_gather<2>(P, A, lst, lane, i, cnt, tot, in, cx, cy, z0, z1, pr);
+    const int row = cell / P.nz, cz = cell - row * P.nz, cx = row / P.ny, cy = row - cx * P.ny;
+    // each species' entries start on a group; the last fluid group is filled up
+    // with the particle itself, which contributes nothing to its own sums, so
+    // that the sweep takes whole fluid groups
+    int tot = 0;
+    nl_gather<0>(P, A, ring, lane, i, valid, tot, cx, cy, cz, pr);
+    const int nf = tot;
+    if (tot % kNlGroup) {
+        while (tot % kNlGroup) ring[tot++ & (kNlBuildRing - 1)][lane] = i;
+        nl_store_group(A, ring, lane, i, tot / kNlGroup - 1, tot);
     }
-    nl_flush(A, lst, lane, i, cnt, tot, true);
-    if (valid) {
-        A.cnt[i] = tot;
-        if (tot > A.cap) {
-            atomicAdd(&A.nl->overflow, 1);
-            atomicOr(A.flags, FLAG_LIST_OVERFLOW);
-        }
+    const int v0 = tot;
+    nl_gather<1>(P, A, ring, lane, i, valid, tot, cx, cy, cz, pr);
+    const int nv = tot - v0;
+    if (tot % kNlGroup) {
+        nl_store_group(A, ring, lane, i, tot / kNlGroup, tot);
+        tot = (tot / kNlGroup + 1) * kNlGroup;
+    }
+    const int s0 = tot;
+    nl_gather<2>(P, A, ring, lane, i, valid, tot, cx, cy, cz, pr);
+    const int ns = tot - s0;
+    if (tot % kNlGroup) nl_store_group(A, ring, lane, i, tot / kNlGroup, tot);
+    if (!valid) return;
+    A.cnt[i] = make_int2(min(nf, A.cap), max(min(nv, A.cap - v0), 0) | max(min(ns, A.cap - s0), 0) << 16);
+    if (nf + nv + ns > A.cap - kNlPad) {
+        atomicAdd(&A.nl->overflow, 1);
+        atomicOr(A.flags, FLAG_LIST_OVERFLOW);
     }
 }
-FSIM_BATCHED_KERNEL(kb_nl_build, NlBuildArgs, nl_build_body, kNlBuildWarps * 32)
 
-// The list sweep: one thread per particle walks its list, tests r^2 < R^2
-// and sums the Riemann pair terms in list order (fluid, then wall, then solid
-// candidates, as the stream sweep sums them), then fluidUpdate
-// (src/fluid.cu:234-269) as in the stream sweep; the particle's squared
-// displacement since the build goes into the instance's running maximum.
+FSIM_REBUILD_KERNEL(kg_nl_build, NlBuildArgs, nl_build_body, kNlBuildWarps * 32, blocks_for(A.n, kNlBuildThreads))
+
+// The list sweep: every particle's list in order (fluid, then wall, then solid
+// entries, as the stream sweep sums them), r^2 < R^2, the Riemann pair terms, then
+// fluidUpdate (src/fluid.cu:234-269) as in the stream sweep; the particle's
+// squared displacement since the build goes into the instance's running maximum.
+// With one lane per particle it is bound by the L1's wavefronts (a scattered
+// 32-byte record per entry: 21 wavefronts per warp and entry of a possible 8)
+// and by issue.  Measured, 4.2 M / 1 M / 32 k particles: 1.16 / 0.31 / 0.060 ms
+// with a test and branch per entry, 1.05 / 0.27 / 0.029 ms branch-free with the
+// next group prefetched and (above 262,144 particles) lists of the fine grid.
 // One 32-byte (position, velocity) record with a single 256-bit load through
 // the read-only path (32-byte aligned: records start on 256-byte allocations).
 __device__ __forceinline__ void load_record(const float4 *p, float4 &a, float4 &b)
@@ -952,70 +1008,212 @@ __device__ __forceinline__ void load_record(const float4 *p, float4 &a, float4 &
         : "l"(p));
 }
 
-template <int VISCID, bool CHECK>
-__device__ __forceinline__ void fluid_sweep_nl_pairs(const DevParams &P, const FluidSweepArgs &A, int i, float4 pr,
-                                                     float4 vp, PairAcc &acc)
-{
-    const int m = min(A.nl_cnt[i], A.nl_cap);
-    const int4 *__restrict__ l = reinterpret_cast<const int4 *>(A.nl_list) + (size_t)i * (kNlGroup / 4);
-    const size_t stride = (size_t)A.n * (kNlGroup / 4); // int4 per group row
-    const unsigned ci = CHECK ? A.nl_cxyz_f[i] : 0u;
-    for (int k0 = 0; k0 < m; k0 += kNlGroup) {
-        // one group: a whole 32-byte sector of the lane's list, read once per
-        // sweep, so loaded evict-first: the lists (1.6 GB at the 4M case) would
-        // otherwise push the neighbour records out of L1 and L2
-        const int4 a = __ldcs(l + (size_t)(k0 / kNlGroup) * stride), b = __ldcs(l + (size_t)(k0 / kNlGroup) * stride + 1);
-        const int grp[kNlGroup] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-        for (int q = 0; q < kNlGroup; ++q) {
-            if (k0 + q >= m) break;
-            const unsigned e = (unsigned)grp[q];
-            const int sp = (int)(e >> kNlSpeciesShift), j = (int)(e & kNlIndexMask);
-            FSIM_DCHECK(sp == 0 ? j < A.n : sp == 1 ? j < A.nl_nv : sp == 2 && j < A.nl_ns, 1u, continue);
-            if (sp == 2) {
-                const float4 q4 = A.s_pos[j];
-                const float dx = q4.x - pr.x, dy = q4.y - pr.y, dz = q4.z - pr.z;
-                const float r2 = dist2(dx, dy, dz);
-                if (r2 < P.R2 && (!CHECK || cells_adjacent(ci, A.nl_cxyz_s[j]))) {
-                    const float4 np = A.s_np[j], sv = A.s_vel[j];
-                    const float k2 = 2.0f * ((vp.x - sv.x) * np.x + (vp.y - sv.y) * np.y + (vp.z - sv.z) * np.z);
-                    riemann_pair<false, VISCID>(P, dx, dy, dz, r2, vp.x, vp.y, vp.z, pr.w, vp.w, vp.x - k2 * np.x,
-                                                vp.y - k2 * np.y, vp.z - k2 * np.z, pr.w, np.w, false, acc);
-                }
-            } else if (sp == 1) {
-                const float4 q4 = A.v_posr[j];
-                const float dx = q4.x - pr.x, dy = q4.y - pr.y, dz = q4.z - pr.z;
-                const float r2 = dist2(dx, dy, dz);
-                if (r2 < P.R2 && (!CHECK || cells_adjacent(ci, A.nl_cxyz_v[j]))) {
-                    const float4 u = A.v_velp[j];
-                    riemann_pair<true, VISCID>(P, dx, dy, dz, r2, vp.x, vp.y, vp.z, pr.w, vp.w, u.x, u.y, u.z, q4.w,
-                                               u.w, true, acc);
-                }
-            } else {
-                float4 q4, u;
-                load_record(A.rec + 2 * (size_t)j, q4, u); // position and velocity: one sector
-                const float dx = q4.x - pr.x, dy = q4.y - pr.y, dz = q4.z - pr.z;
-                const float r2 = dist2(dx, dy, dz);
-                if (r2 < P.R2 && (!CHECK || cells_adjacent(ci, A.nl_cxyz_f[j]))) {
-                    riemann_pair<true, VISCID>(P, dx, dy, dz, r2, vp.x, vp.y, vp.z, pr.w, vp.w, u.x, u.y, u.z, q4.w,
-                                               u.w, false, acc);
-                }
+// One pair of the list sweep: whether it counts, its difference vector and its
+// terms (drho += x w, a += f d).
+struct ListPair {
+    bool in;
+    float dx, dy, dz, x, w, f;
+};
+
+// How a particle's pair terms are summed, always in list order.
+//  * One lane (LANES false): the lane walks its whole list.  The sums are
+//    predicated on `in` instead of branched around: no divergence, the loads of
+//    later entries issue ahead of an entry's arithmetic, and a neighbour out of
+//    range adds nothing, whatever its state holds.
+//  * 2^lane_shift lanes (at least four) of an instance too small to fill the
+//    GPU with one lane per particle: each takes every 2^lane_shift-th entry, and
+//    after each round of one entry per lane the terms go through shared memory
+//    to the first four lanes, which own one of the four sums each and add the
+//    round's terms in list order -- the same additions in the same order as one
+//    lane makes, so the number of lanes never changes a result.
+// KAHAN (mixed form): the density rate is Kahan-compensated.
+template <bool LANES, bool KAHAN>
+struct ListSum {
+    PairAcc acc;           // LANES: sum c of lane c < 4 in acc.ax, its compensation in acc.drho_c
+    float (*sh)[32];       // LANES: the warp's terms: f, x, dx, dy, dz, w
+    int lane, g, G;
+
+    __device__ __forceinline__ void add(const ListPair &p)
+    {
+        if (!LANES) {
+            if (KAHAN) kahan_add(p.x, p.w, p.in, acc.drho, acc.drho_c);
+            asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\t@p fma.rn.f32 %0, %4, %5, %0;\n\t"
+                "@p fma.rn.f32 %1, %4, %6, %1;\n\t@p fma.rn.f32 %2, %4, %7, %2;\n\t}"
+                : "+f"(acc.ax), "+f"(acc.ay), "+f"(acc.az)
+                : "r"((int)p.in), "f"(p.f), "f"(p.dx), "f"(p.dy), "f"(p.dz));
+            if (!KAHAN)
+                asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %1, 0;\n\t@p fma.rn.f32 %0, %2, %3, %0;\n\t}"
+                    : "+f"(acc.drho)
+                    : "r"((int)p.in), "f"(p.x), "f"(p.w));
+            return;
+        }
+        // a term out of range is stored as 0 x 0
+        __syncwarp();
+        sh[0][lane] = p.in ? p.f : 0.0f;
+        sh[1][lane] = p.in ? p.x : 0.0f;
+        sh[2][lane] = p.in ? p.dx : 0.0f;
+        sh[3][lane] = p.in ? p.dy : 0.0f;
+        sh[4][lane] = p.in ? p.dz : 0.0f;
+        sh[5][lane] = p.in ? p.w : 0.0f;
+        __syncwarp();
+        if (g < 4) {
+            const float *l = &sh[g == 3 ? 1 : 0][lane - g], *r = &sh[2 + g][lane - g];
+#pragma unroll 4
+            for (int k = 0; k < G; ++k) {
+                if (KAHAN && g == 3) kahan_add(l[k], r[k], true, acc.ax, acc.drho_c);
+                else acc.ax = __fmaf_rn(l[k], r[k], acc.ax);
             }
         }
     }
+    // the particle's sums, on its lane 0 (all lanes call it)
+    __device__ __forceinline__ PairAcc total()
+    {
+        if (!LANES) return acc;
+        const int l0 = lane - g;
+        PairAcc t;
+        t.ax = __shfl_sync(kFull, acc.ax, l0);
+        t.ay = __shfl_sync(kFull, acc.ax, l0 + 1);
+        t.az = __shfl_sync(kFull, acc.ax, l0 + 2);
+        t.drho = __shfl_sync(kFull, acc.ax, l0 + 3);
+        t.drho_c = 0.0f;
+        return t;
+    }
+};
+
+// Walk particle i's list: f(species, j) gives the pair with entry j, and the
+// sums take the pairs in list order.  Fluid entries come in whole groups (the
+// last one filled up with the particle itself, which adds nothing).
+template <bool LANES, bool KAHAN, class FF, class FV, class FS>
+__device__ __forceinline__ void walk_list(const FluidSweepArgs &A, int i, bool valid, ListSum<LANES, KAHAN> &sum,
+                                          FF &&fluid, FV &&wall, FS &&solid)
+{
+    const int2 cnt = valid ? A.nl_cnt[i] : make_int2(0, 0);
+    const int ngf = (cnt.x + kNlGroup - 1) / kNlGroup, nv = cnt.y & 0xffff, ns = (int)((unsigned)cnt.y >> 16);
+    const int ngv = (nv + kNlGroup - 1) / kNlGroup;
+    if (!LANES) {
+        // the lists are read once per sweep, evict-first: they (1.6 GB at the 4M
+        // case) would otherwise push the neighbour records out of L1 and L2; the
+        // next group's entries load while this group's pairs are summed
+        const size_t stride = (size_t)A.n * (kNlGroup / 4); // int4 per group row
+        const int4 *__restrict__ l = reinterpret_cast<const int4 *>(A.nl_list) + (size_t)i * (kNlGroup / 4);
+        int4 a, b;
+        if (ngf) {
+            a = __ldcs(l);
+            b = __ldcs(l + 1);
+        }
+        for (int k = 0; k < ngf; ++k) {
+            const int e[kNlGroup] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            l += stride;
+            if (k + 1 < ngf) {
+                a = __ldcs(l);
+                b = __ldcs(l + 1);
+            }
+#pragma unroll
+            for (int q = 0; q < kNlGroup; ++q) {
+                FSIM_DCHECK(e[q] >= 0 && e[q] < A.n, 1u, continue);
+                sum.add(fluid(e[q]));
+            }
+        }
+        for (int k = 0; k < nv; ++k) {
+            const int j = A.nl_list[((size_t)(ngf + k / kNlGroup) * A.n + i) * kNlGroup + k % kNlGroup];
+            FSIM_DCHECK(j >= 0 && j < A.nl_nv, 1u, continue);
+            sum.add(wall(j));
+        }
+        for (int k = 0; k < ns; ++k) {
+            const int j = A.nl_list[((size_t)(ngf + ngv + k / kNlGroup) * A.n + i) * kNlGroup + k % kNlGroup];
+            FSIM_DCHECK(j >= 0 && j < A.nl_ns, 1u, continue);
+            sum.add(solid(j));
+        }
+        return;
+    }
+    // rounds of one entry per lane; the warp's particles may need different
+    // numbers of them, and all lanes take part in every round
+    auto rounds = [&](int count, int grp, auto &&pair) {
+        const int most = __reduce_max_sync(kFull, count);
+        for (int e = sum.g; e - sum.g < most; e += sum.G) {
+            ListPair p = {};
+            if (e < count) p = pair(A.nl_list[((size_t)(grp + e / kNlGroup) * A.n + i) * kNlGroup + e % kNlGroup]);
+            sum.add(p);
+        }
+    };
+    rounds(cnt.x, 0, fluid);
+    rounds(nv, ngf, wall);
+    rounds(ns, ngf + ngv, solid);
 }
 
-template <int VISCID>
-__device__ __forceinline__ void fluid_sweep_nl_body(const DevParams &P, const FluidSweepArgs &A, int blk)
+// Particle i's pairs in the plain form.
+template <int VISCID, bool CHECK, bool LANES>
+__device__ __forceinline__ void fluid_sweep_nl_pairs(const DevParams &P, const FluidSweepArgs &A, int i, bool valid,
+                                                     float4 pr, float4 vp, ListSum<LANES, false> &sum)
 {
-    const int i = blk * blockDim.x + threadIdx.x;
+    const unsigned ci = CHECK && valid ? A.nl_cxyz_f[i] : 0u;
+    auto rel = [&](float4 q, ListPair &p) {
+        p.dx = q.x - pr.x;
+        p.dy = q.y - pr.y;
+        p.dz = q.z - pr.z;
+        return dist2(p.dx, p.dy, p.dz);
+    };
+    walk_list<LANES, false>(
+        A, i, valid, sum,
+        [&](int j) {
+            ListPair p;
+            float4 q, u;
+            load_record(A.rec + 2 * (size_t)j, q, u); // position and velocity: one sector
+            const float r2 = rel(q, p);
+            p.in = r2 < P.R2 && (!CHECK || cells_adjacent(ci, A.nl_cxyz_f[j]));
+            riemann_terms<true, VISCID>(P, p.dx, p.dy, p.dz, r2, vp.x, vp.y, vp.z, pr.w, vp.w, u.x, u.y, u.z, q.w, u.w,
+                                        false, p.x, p.w, p.f);
+            return p;
+        },
+        [&](int j) {
+            ListPair p;
+            const float4 q = A.v_posr[j], u = A.v_velp[j];
+            const float r2 = rel(q, p);
+            p.in = r2 < P.R2 && (!CHECK || cells_adjacent(ci, A.nl_cxyz_v[j]));
+            riemann_terms<true, VISCID>(P, p.dx, p.dy, p.dz, r2, vp.x, vp.y, vp.z, pr.w, vp.w, u.x, u.y, u.z, q.w, u.w,
+                                        true, p.x, p.w, p.f);
+            return p;
+        },
+        [&](int j) {
+            ListPair p;
+            const float4 q = A.s_pos[j], np = A.s_np[j], sv = A.s_vel[j];
+            const float r2 = rel(q, p);
+            p.in = r2 < P.R2 && (!CHECK || cells_adjacent(ci, A.nl_cxyz_s[j]));
+            const float k2 = 2.0f * ((vp.x - sv.x) * np.x + (vp.y - sv.y) * np.y + (vp.z - sv.z) * np.z);
+            riemann_terms<false, VISCID>(P, p.dx, p.dy, p.dz, r2, vp.x, vp.y, vp.z, pr.w, vp.w, vp.x - k2 * np.x,
+                                         vp.y - k2 * np.y, vp.z - k2 * np.z, pr.w, np.w, false, p.x, p.w, p.f);
+            return p;
+        });
+}
+
+// the warp's term rows of the lanes form (dynamic shared memory)
+__device__ __forceinline__ float (*lane_terms())[32]
+{
+    extern __shared__ float sweep_terms[][32];
+    return sweep_terms + kSweepTermRows * (threadIdx.x >> 5);
+}
+
+template <int VISCID, bool LANES>
+__device__ __forceinline__ void fluid_sweep_nl_lanes(const DevParams &P, const FluidSweepArgs &A, int blk)
+{
+    const int t = blk * blockDim.x + threadIdx.x, sh = LANES ? A.lane_shift : 0, i = t >> sh;
+    ListSum<LANES, false> sum;
+    sum.acc = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    sum.lane = threadIdx.x & 31;
+    sum.G = 1 << sh;
+    sum.g = t & (sum.G - 1);
+    if (LANES) sum.sh = lane_terms();
     const bool valid = i < A.n;
-    unsigned d2bits = 0u;
+    float4 pr = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vp = pr;
     if (valid) {
-        const float4 pr = A.posr[i], vp = A.velp[i];
-        PairAcc acc = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        if (A.nl_cxyz_f) fluid_sweep_nl_pairs<VISCID, true>(P, A, i, pr, vp, acc);
-        else fluid_sweep_nl_pairs<VISCID, false>(P, A, i, pr, vp, acc);
+        pr = A.posr[i];
+        vp = A.velp[i];
+    }
+    if (A.nl_cxyz_f) fluid_sweep_nl_pairs<VISCID, true, LANES>(P, A, i, valid, pr, vp, sum);
+    else fluid_sweep_nl_pairs<VISCID, false, LANES>(P, A, i, valid, pr, vp, sum);
+    const PairAcc acc = sum.total();
+    unsigned d2bits = 0u;
+    if (valid && sum.g == 0) {
         const float4 x = fluid_update_store(P, A, i, pr, vp, acc);
         const float4 o = A.x0[i];
         d2bits = __float_as_uint(dist2(x.x - o.x, x.y - o.y, x.z - o.z));
@@ -1023,15 +1221,21 @@ __device__ __forceinline__ void fluid_sweep_nl_body(const DevParams &P, const Fl
     const unsigned wmax = __reduce_max_sync(kFull, d2bits);
     if ((threadIdx.x & 31) == 0 && wmax) atomicMax(&A.nl->maxd2, wmax);
 }
+template <int VISCID>
+__device__ __forceinline__ void fluid_sweep_nl_body(const DevParams &P, const FluidSweepArgs &A, int blk)
+{
+    if (A.lane_shift) fluid_sweep_nl_lanes<VISCID, true>(P, A, blk); // uniform over the launch
+    else fluid_sweep_nl_lanes<VISCID, false>(P, A, blk);
+}
 
 // launch shapes of the list sweep: threads per block, minimum blocks per SM
 template <int BS, int MINB>
 struct NlShape {
     static constexpr int threads = BS, min_blocks = MINB;
 };
-using NlShape0 = NlShape<128, 16>; // at most 32 registers: 16 blocks (64 warps) per SM
-using NlShape1 = NlShape<128, 12>; // at most 40 registers: 12 blocks (48 warps) per SM
-using NlShape2 = NlShape<256, 5>;  // at most 51 registers: 5 blocks (40 warps) per SM
+using NlShape0 = NlShape<128, 8>;  // at most 64 registers: 8 blocks (32 warps) per SM
+using NlShape1 = NlShape<128, 9>;  // at most 56 registers: 9 blocks (36 warps) per SM
+using NlShape2 = NlShape<256, 4>;  // at most 64 registers: 4 blocks (32 warps) per SM
 static_assert(kShapeWarps[0] * 32 == NlShape0::threads && kShapeWarps[1] * 32 == NlShape1::threads &&
                   kShapeWarps[2] * 32 == NlShape2::threads,
               "list-sweep shapes follow the block sizes of fsim_types.h");
@@ -1107,16 +1311,14 @@ FSIM_BATCHED_KERNEL(kb_virt, VirtArgs, virt_body, kBlock)
 // gradient sum over the other virtual particles, normalised, zero when its
 // squared length is below EPS_FOR_SUM.  Walls never move: computed once.
 __global__ void k_virt_normal(const DevParams P, const float4 *__restrict__ v_posr, const int *__restrict__ v_cell,
-                              const int *__restrict__ start_v, float4 *__restrict__ v_normal, int n)
+                              const int *__restrict__ start_v, float4 *__restrict__ v_normal, int n, int reach)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 xi = v_posr[i];
-    Rows rows;
-    neighbor_rows(P, v_cell[i], rows);
     float nx = 0.0f, ny = 0.0f, nz = 0.0f;
-    for (int r = 0; r < rows.count; ++r) {
-        for (int j = start_v[rows.base[r] + rows.z0], je = start_v[rows.base[r] + rows.z1]; j < je; ++j) {
+    for_rows_within(P, v_cell[i], reach, [&](int c0, int c1) {
+        for (int j = start_v[c0], je = start_v[c1]; j < je; ++j) {
             if (j == i) continue;
             const float4 q = v_posr[j];
             const float dx = q.x - xi.x, dy = q.y - xi.y, dz = q.z - xi.z;
@@ -1128,7 +1330,7 @@ __global__ void k_virt_normal(const DevParams P, const float4 *__restrict__ v_po
                 nz -= dz * w;
             }
         }
-    }
+    });
     const float l2 = nx * nx + ny * ny + nz * nz;
     if (l2 < FSIM_EPS_FOR_SUM) {
         nx = ny = nz = 0.0f;
@@ -1580,6 +1782,28 @@ __device__ __forceinline__ void unpack_cell(unsigned c, int &cx, int &cy, int &c
     cz = (int)(c >> 21);
 }
 
+// A pair's difference vector in the mixed form from the packed codes d (as
+// cell_codes unpacks them): true when the cells are neighbours.  Where they
+// are not, the codes come out as those of the own cell, so that what is
+// addressed by them stays in bounds.
+__device__ __forceinline__ bool mixed_rel(const DevParams &P, const OwnMixed &o, unsigned d, float4 q, float &dx,
+                                          float &dy, float &dz, int &bx, int &by, int &bz)
+{
+    // every field in {0, 1, 2}: no bit above the low two of a field, and not both of those
+    constexpr unsigned kLow = 3u * kCellBias;
+    const bool near = (d & ~kLow) == 0u && (d & (d >> 1) & kCellBias) == 0u;
+    d = near ? d : kCellBias;
+    bx = (int)(d & 3u);
+    by = (int)((d >> 11) & 3u);
+    bz = (int)(d >> 21);
+    // = shifted(o.b*, b* - 1, cdx); the small codes to float through the bits of 2^23 + b
+    auto f = [](int b) { return __fsub_rn(__int_as_float(0x4b000000 | b), 8388608.0f); };
+    dx = q.x - fmaf(-f(bx), P.cdx[0], o.bx);
+    dy = q.y - fmaf(-f(by), P.cdx[1], o.by);
+    dz = q.z - fmaf(-f(bz), P.cdx[2], o.bz);
+    return near;
+}
+
 // Neighbour lists in the mixed form.  The particles keep the order of the last
 // list build between builds; each step re-bins every offset to the cell it now
 // lies in (in place), and the per-step cell index (kb_rank) gives every
@@ -1589,95 +1813,91 @@ __device__ __forceinline__ void unpack_cell(unsigned c, int &cx, int &cy, int &c
 // and a pair is taken exactly as the mixed cell walk takes it: the two cells
 // are neighbours, and r^2 < R^2 with the offset of i shifted by the cell
 // difference (`shifted`), so both sum bit-identical pair terms (in list order).
-template <int VISCID>
-__device__ __forceinline__ void fluid_sweep_nlm_pairs(const DevParams &P, const FluidSweepArgs &A, int i,
+template <int VISCID, bool LANES>
+__device__ __forceinline__ void fluid_sweep_nlm_pairs(const DevParams &P, const FluidSweepArgs &A, int i, bool valid,
                                                       const OwnMixed &o, float4 pa, float4 vp, unsigned ci,
-                                                      PairAcc &acc)
+                                                      ListSum<LANES, true> &sum)
 {
     const unsigned cb = kCellBias - ci;
-    const int m = min(A.nl_cnt[i], A.nl_cap);
-    const int4 *__restrict__ l = reinterpret_cast<const int4 *>(A.nl_list) + (size_t)i * (kNlGroup / 4);
-    const size_t stride = (size_t)A.n * (kNlGroup / 4);
     const int nynz = P.ny * P.nz;
-    for (int k0 = 0; k0 < m; k0 += kNlGroup) {
-        const int4 a = __ldcs(l + (size_t)(k0 / kNlGroup) * stride), b = __ldcs(l + (size_t)(k0 / kNlGroup) * stride + 1);
-        const int grp[kNlGroup] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-        for (int q = 0; q < kNlGroup; ++q) {
-            if (k0 + q >= m) break;
-            const unsigned e = (unsigned)grp[q];
-            const int sp = (int)(e >> kNlSpeciesShift), j = (int)(e & kNlIndexMask);
-            FSIM_DCHECK(sp == 0 ? j < A.n : sp == 1 ? j < A.nl_nv : sp == 2 && j < A.nl_ns, 1u, continue);
-            if (sp == 2) {
-                const float4 q4 = A.s_pos[j];
-                const float dx = q4.x - pa.x, dy = q4.y - pa.y, dz = q4.z - pa.z;
-                const float r2 = dist2(dx, dy, dz);
-                if (r2 < P.R2 && cells_adjacent(ci, A.nl_cxyz_s[j])) {
-                    const float4 np = A.s_np[j], sv = A.s_vel[j];
-                    const float k2 = __fmul_rn(2.0f, fmaf(__fsub_rn(vp.z, sv.z), np.z,
-                                                          fmaf(__fsub_rn(vp.y, sv.y), np.y,
-                                                               __fmul_rn(__fsub_rn(vp.x, sv.x), np.x))));
-                    riemann_pair<false, VISCID, true>(P, dx, dy, dz, r2, vp.x, vp.y, vp.z, o.rho, o.p,
-                                                      fmaf(-k2, np.x, vp.x), fmaf(-k2, np.y, vp.y),
-                                                      fmaf(-k2, np.z, vp.z), o.rho, np.w, false, acc);
-                }
-                continue;
-            }
-            float4 q4, u;
-            unsigned cj;
-            if (sp == 1) {
-                q4 = A.v_posr[j];
-                u = A.v_velp[j];
-                cj = A.nl_cxyz_v[j];
-            } else {
-                load_record(A.rec + 2 * (size_t)j, q4, u);
-                cj = __float_as_uint(u.w);
-            }
+    walk_list<LANES, true>(
+        A, i, valid, sum,
+        [&](int j) {
+            ListPair p;
+            float4 q, u;
+            load_record(A.rec + 2 * (size_t)j, q, u);
             int bx, by, bz;
-            if (!cell_codes(cj, cb, bx, by, bz)) continue;
-            // = shifted(o.b*, b* - 1, cdx)
-            const float dx = q4.x - fmaf(-(float)bx, P.cdx[0], o.bx);
-            const float dy = q4.y - fmaf(-(float)by, P.cdx[1], o.by);
-            const float dz = q4.z - fmaf(-(float)bz, P.cdx[2], o.bz);
-            const float r2 = dist2(dx, dy, dz);
-            if (!(r2 < P.R2)) continue;
-            float rhoj, pj;
-            if (sp == 0) {
-                const float2 ref = A.cm[o.cbase + bx * nynz + by * P.nz + bz];
-                const float2 dev = half2_floats(q4.w);
-                rhoj = fmaf(P.rho0, fmaf(dev.x, kDeltaUnit, ref.x), P.rho0);
-                pj = fmaf(dev.y, P.p_unit, ref.y);
-            } else {
-                rhoj = q4.w;
-                pj = u.w;
-            }
-            riemann_pair<true, VISCID, true>(P, dx, dy, dz, r2, vp.x, vp.y, vp.z, o.rho, o.p, u.x, u.y, u.z, rhoj, pj,
-                                             sp == 1, acc);
-        }
-    }
+            const bool near = mixed_rel(P, o, __float_as_uint(u.w) + cb, q, p.dx, p.dy, p.dz, bx, by, bz);
+            const float r2 = dist2(p.dx, p.dy, p.dz);
+            p.in = near && r2 < P.R2;
+            const float2 ref = A.cm[o.cbase + bx * nynz + by * P.nz + bz];
+            const float2 dev = half2_floats(q.w);
+            riemann_terms<true, VISCID, true>(P, p.dx, p.dy, p.dz, r2, vp.x, vp.y, vp.z, o.rho, o.p, u.x, u.y, u.z,
+                                              fmaf(P.rho0, fmaf(dev.x, kDeltaUnit, ref.x), P.rho0),
+                                              fmaf(dev.y, P.p_unit, ref.y), false, p.x, p.w, p.f);
+            return p;
+        },
+        [&](int j) {
+            ListPair p;
+            const float4 q = A.v_posr[j], u = A.v_velp[j];
+            int bx, by, bz;
+            const bool near = mixed_rel(P, o, A.nl_cxyz_v[j] + cb, q, p.dx, p.dy, p.dz, bx, by, bz);
+            const float r2 = dist2(p.dx, p.dy, p.dz);
+            p.in = near && r2 < P.R2;
+            riemann_terms<true, VISCID, true>(P, p.dx, p.dy, p.dz, r2, vp.x, vp.y, vp.z, o.rho, o.p, u.x, u.y, u.z,
+                                              q.w, u.w, true, p.x, p.w, p.f);
+            return p;
+        },
+        [&](int j) {
+            ListPair p;
+            const float4 q = A.s_pos[j], np = A.s_np[j], sv = A.s_vel[j];
+            p.dx = q.x - pa.x;
+            p.dy = q.y - pa.y;
+            p.dz = q.z - pa.z;
+            const float r2 = dist2(p.dx, p.dy, p.dz);
+            p.in = r2 < P.R2 && cells_adjacent(ci, A.nl_cxyz_s[j]);
+            const float k2 = __fmul_rn(2.0f, fmaf(__fsub_rn(vp.z, sv.z), np.z,
+                                                  fmaf(__fsub_rn(vp.y, sv.y), np.y,
+                                                       __fmul_rn(__fsub_rn(vp.x, sv.x), np.x))));
+            riemann_terms<false, VISCID, true>(P, p.dx, p.dy, p.dz, r2, vp.x, vp.y, vp.z, o.rho, o.p,
+                                               fmaf(-k2, np.x, vp.x), fmaf(-k2, np.y, vp.y), fmaf(-k2, np.z, vp.z),
+                                               o.rho, np.w, false, p.x, p.w, p.f);
+            return p;
+        });
 }
 
-template <int VISCID>
-__device__ __forceinline__ void fluid_sweep_nlm_body(const DevParams &P, const FluidSweepArgs &A, int blk)
+template <int VISCID, bool LANES>
+__device__ __forceinline__ void fluid_sweep_nlm_lanes(const DevParams &P, const FluidSweepArgs &A, int blk)
 {
-    const int i = blk * blockDim.x + threadIdx.x;
+    const int t = blk * blockDim.x + threadIdx.x, sh = LANES ? A.lane_shift : 0, i = t >> sh;
+    ListSum<LANES, true> sum;
+    sum.acc = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    sum.lane = threadIdx.x & 31;
+    sum.G = 1 << sh;
+    sum.g = t & (sum.G - 1);
+    if (LANES) sum.sh = lane_terms();
     const bool valid = i < A.n;
-    unsigned d2bits = 0u;
+    float4 off = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vp = off;
+    unsigned ci = 0;
+    OwnMixed o = {};
     if (valid) {
-        const float4 off = A.posr[i], vp = A.velp[i];
-        const unsigned ci = A.nl_cxyz_f[i];
-        int cx, cy, cz;
-        unpack_cell(ci, cx, cy, cz);
-        OwnMixed o;
-        o.bx = __fadd_rn(off.x, P.cdx[0]);
-        o.by = __fadd_rn(off.y, P.cdx[1]);
-        o.bz = __fadd_rn(off.z, P.cdx[2]);
+        off = A.posr[i];
+        vp = A.velp[i];
+        ci = A.nl_cxyz_f[i];
         o.cbase = A.cell_f[i] - P.ny * P.nz - P.nz - 1;
-        o.rho = fmaf(P.rho0, vp.w, P.rho0);
-        o.p = eos_delta(P, vp.w);
-        const float4 pa = mixed_abs(P, off, cx, cy, cz, o.rho);
-        PairAcc acc = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        fluid_sweep_nlm_pairs<VISCID>(P, A, i, o, pa, vp, ci, acc);
+    }
+    int cx, cy, cz;
+    unpack_cell(ci, cx, cy, cz);
+    o.bx = __fadd_rn(off.x, P.cdx[0]);
+    o.by = __fadd_rn(off.y, P.cdx[1]);
+    o.bz = __fadd_rn(off.z, P.cdx[2]);
+    o.rho = fmaf(P.rho0, vp.w, P.rho0);
+    o.p = eos_delta(P, vp.w);
+    const float4 pa = mixed_abs(P, off, cx, cy, cz, o.rho);
+    fluid_sweep_nlm_pairs<VISCID, LANES>(P, A, i, valid, o, pa, vp, ci, sum);
+    const PairAcc acc = sum.total();
+    unsigned d2bits = 0u;
+    if (valid && sum.g == 0) {
         const float4 x = mixed_abs(P, fluid_update_store_m(P, A, i, off, vp, o.rho, acc, cx, cy, cz), cx, cy, cz,
                                    0.0f);
         const float4 x0 = A.x0[i];
@@ -1686,11 +1906,17 @@ __device__ __forceinline__ void fluid_sweep_nlm_body(const DevParams &P, const F
     const unsigned wmax = __reduce_max_sync(kFull, d2bits);
     if ((threadIdx.x & 31) == 0 && wmax) atomicMax(&A.nl->maxd2, wmax);
 }
+template <int VISCID>
+__device__ __forceinline__ void fluid_sweep_nlm_body(const DevParams &P, const FluidSweepArgs &A, int blk)
+{
+    if (A.lane_shift) fluid_sweep_nlm_lanes<VISCID, true>(P, A, blk); // uniform over the launch
+    else fluid_sweep_nlm_lanes<VISCID, false>(P, A, blk);
+}
 
 // launch shapes of the mixed list sweep (more registers than the plain one)
-using NlmShape0 = NlShape<128, 8>;  // at most 64 registers
-using NlmShape1 = NlShape<128, 10>; // at most 48 registers (a few spills)
-using NlmShape2 = NlShape<256, 3>;  // at most 85 registers
+using NlmShape0 = NlShape<128, 8>; // at most 64 registers
+using NlmShape1 = NlShape<128, 7>; // at most 72 registers
+using NlmShape2 = NlShape<256, 3>; // at most 85 registers
 static_assert(NlmShape0::threads == NlShape0::threads && NlmShape1::threads == NlShape1::threads &&
                   NlmShape2::threads == NlShape2::threads,
               "mixed list-sweep shapes use the block sizes of the plain ones");
@@ -1722,17 +1948,13 @@ __global__ void __launch_bounds__(SH::threads, SH::min_blocks)
 // the new order, the positions of the build).
 __device__ __forceinline__ void mixed_abs_body(const DevParams &P, const MixedAbsArgs &A, int blk)
 {
-    if (A.gate && !*A.gate) return; // uniform per block
-    FSIM_ELEMENT_BLOCKS(A, blk, b)
-    {
-        const int s = b * blockDim.x + threadIdx.x;
-        if (s >= A.n) continue;
-        int cx, cy, cz;
-        cell_xyz(P, A.cell[s], cx, cy, cz);
-        A.out[s] = mixed_abs(P, A.posr[s], cx, cy, cz, 0.0f);
-    }
+    const int s = blk * blockDim.x + threadIdx.x;
+    if (s >= A.n) return;
+    int cx, cy, cz;
+    cell_xyz(P, A.cell[s], cx, cy, cz);
+    A.out[s] = mixed_abs(P, A.posr[s], cx, cy, cz, 0.0f);
 }
-FSIM_BATCHED_KERNEL(kb_mixed_abs, MixedAbsArgs, mixed_abs_body, kBlock)
+FSIM_REBUILD_KERNEL(kg_mixed_abs, MixedAbsArgs, mixed_abs_body, kBlock, blocks_for(A.n, kBlock))
 
 // getVirtData (src/virt.cu:9-75) in the mixed form.
 __device__ __forceinline__ void virt_mixed_body(const DevParams &P, const VirtArgs &A, int blk)
@@ -2530,7 +2752,7 @@ __global__ void k_neighbor_counts(const DevParams P, const DevParams Pv, const f
                                   const int *__restrict__ cell_f, const int *__restrict__ start_f,
                                   const int *__restrict__ ids_f, const float4 *__restrict__ s_pos,
                                   const int *__restrict__ start_s, const int *__restrict__ ids_s,
-                                  const float4 *__restrict__ v_posr, const int *__restrict__ start_v,
+                                  const float4 *__restrict__ v_posr, const int *__restrict__ start_v, int reach_v,
                                   int *__restrict__ out, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2550,37 +2772,44 @@ __global__ void k_neighbor_counts(const DevParams P, const DevParams Pv, const f
             cs += dist2(q.x - p.x, q.y - p.y, q.z - p.z) < P.R2;
         }
     }
-    Rows vrows;
-    neighbor_rows(Pv, ids_f ? cell_index(Pv, p.x, p.y, p.z, nullptr) : cell_f[i], vrows);
-    for (int r = 0; r < vrows.count; ++r) {
-        const int c0 = vrows.base[r] + vrows.z0, c1 = vrows.base[r] + vrows.z1;
+    for_rows_within(Pv, ids_f ? cell_index(Pv, p.x, p.y, p.z, nullptr) : cell_f[i], reach_v, [&](int c0, int c1) {
         for (int j = start_v[c0]; j < start_v[c1]; ++j) {
             const float4 q = v_posr[j];
             cv += dist2(q.x - p.x, q.y - p.y, q.z - p.z) < P.R2;
         }
-    }
+    });
     out[3 * i] = cf;
     out[3 * i + 1] = cs;
     out[3 * i + 2] = cv;
 }
 
+// f(species, j) for every entry of particle i's list (0 fluid, 1 wall, 2 solid).
+template <class F>
+__device__ __forceinline__ void for_list_entries(const int *__restrict__ list, int2 cnt, int i, int n, F &&f)
+{
+    const int count[3] = {cnt.x, cnt.y & 0xffff, (int)((unsigned)cnt.y >> 16)};
+    int grp = 0; // the species' first group
+    for (int sp = 0; sp < 3; ++sp) {
+        for (int k = 0; k < count[sp]; ++k)
+            f(sp, list[((size_t)(grp + k / kNlGroup) * n + i) * kNlGroup + k % kNlGroup]);
+        grp += (count[sp] + kNlGroup - 1) / kNlGroup;
+    }
+}
+
 // The same counts of a neighbour-list instance, from its lists (which hold
 // every pair within the impact distance while no rebuild is due).
 __global__ void k_neighbor_counts_nl(const DevParams P, const float4 *__restrict__ fposr, const int *__restrict__ list,
-                                     const int *__restrict__ cnt, int cap, const float4 *__restrict__ s_pos,
+                                     const int2 *__restrict__ cnt, const float4 *__restrict__ s_pos,
                                      const float4 *__restrict__ v_posr, int *__restrict__ out, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = fposr[i];
     int c[3] = {0, 0, 0};
-    const int m = min(cnt[i], cap);
-    for (int k = 0; k < m; ++k) {
-        const unsigned e = (unsigned)list[((size_t)(k / kNlGroup) * n + i) * kNlGroup + k % kNlGroup];
-        const int sp = (int)(e >> kNlSpeciesShift), j = (int)(e & kNlIndexMask);
+    for_list_entries(list, cnt[i], i, n, [&](int sp, int j) {
         const float4 q = sp == 0 ? fposr[j] : sp == 1 ? v_posr[j] : s_pos[j];
         if (dist2(q.x - p.x, q.y - p.y, q.z - p.z) < P.R2) ++c[sp == 0 ? 0 : sp == 2 ? 1 : 2];
-    }
+    });
     out[3 * i] = c[0];
     out[3 * i + 1] = c[1];
     out[3 * i + 2] = c[2];
@@ -2597,7 +2826,8 @@ __global__ void k_neighbor_counts_mixed(const DevParams P, const DevParams Pv, c
                                         const int *__restrict__ ids_f, const float4 *__restrict__ s_pos,
                                         const int *__restrict__ start_s, const int *__restrict__ ids_s,
                                         const float4 *__restrict__ v_posr, const int *__restrict__ start_v,
-                                        const unsigned *__restrict__ v_cxyz, int *__restrict__ out, int n)
+                                        const unsigned *__restrict__ v_cxyz, int reach_v, int *__restrict__ out,
+                                        int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -2630,10 +2860,7 @@ __global__ void k_neighbor_counts_mixed(const DevParams P, const DevParams Pv, c
                     }
             }
     if (v_cxyz) {
-        Rows vrows;
-        neighbor_rows(Pv, cell_index(Pv, pa.x, pa.y, pa.z, nullptr), vrows);
-        for (int r = 0; r < vrows.count; ++r) {
-            const int c0 = vrows.base[r] + vrows.z0, c1 = vrows.base[r] + vrows.z1;
+        for_rows_within(Pv, cell_index(Pv, pa.x, pa.y, pa.z, nullptr), reach_v, [&](int c0, int c1) {
             for (int j = start_v[c0]; j < start_v[c1]; ++j) {
                 int jx, jy, jz;
                 unpack_cell(v_cxyz[j], jx, jy, jz);
@@ -2643,7 +2870,7 @@ __global__ void k_neighbor_counts_mixed(const DevParams P, const DevParams Pv, c
                 cv += dist2(q.x - shifted(obx, ox, P.cdx[0]), q.y - shifted(oby, oy, P.cdx[1]),
                             q.z - shifted(obz, oz, P.cdx[2])) < P.R2;
             }
-        }
+        });
     }
     out[3 * i] = cf;
     out[3 * i + 1] = cs;
@@ -2654,7 +2881,7 @@ __global__ void k_neighbor_counts_mixed(const DevParams P, const DevParams Pv, c
 // with the list sweep's pair rule.
 __global__ void k_neighbor_counts_nlm(const DevParams P, const float4 *__restrict__ fposr,
                                       const int *__restrict__ cell_f, const unsigned *__restrict__ cxyz_f,
-                                      const int *__restrict__ list, const int *__restrict__ cnt, int cap,
+                                      const int *__restrict__ list, const int2 *__restrict__ cnt,
                                       const float4 *__restrict__ s_pos, const unsigned *__restrict__ cxyz_s,
                                       const float4 *__restrict__ v_posr, const unsigned *__restrict__ cxyz_v,
                                       int *__restrict__ out, int n)
@@ -2668,24 +2895,21 @@ __global__ void k_neighbor_counts_nlm(const DevParams P, const float4 *__restric
     const float obx = __fadd_rn(off.x, P.cdx[0]), oby = __fadd_rn(off.y, P.cdx[1]), obz = __fadd_rn(off.z, P.cdx[2]);
     const unsigned ci = cxyz_f[i];
     int c[3] = {0, 0, 0};
-    const int m = min(cnt[i], cap);
-    for (int k = 0; k < m; ++k) {
-        const unsigned e = (unsigned)list[((size_t)(k / kNlGroup) * n + i) * kNlGroup + k % kNlGroup];
-        const int sp = (int)(e >> kNlSpeciesShift), j = (int)(e & kNlIndexMask);
+    for_list_entries(list, cnt[i], i, n, [&](int sp, int j) {
         if (sp == 2) {
             const float4 q = s_pos[j];
             if (dist2(q.x - pa.x, q.y - pa.y, q.z - pa.z) < P.R2 && cells_adjacent(ci, cxyz_s[j])) ++c[1];
-            continue;
+            return;
         }
         const float4 q = sp == 0 ? fposr[j] : v_posr[j];
         int jx, jy, jz;
         unpack_cell(sp == 0 ? cxyz_f[j] : cxyz_v[j], jx, jy, jz);
         const int ox = jx - cx, oy = jy - cy, oz = jz - cz;
-        if (abs(ox) > 1 || abs(oy) > 1 || abs(oz) > 1) continue;
+        if (abs(ox) > 1 || abs(oy) > 1 || abs(oz) > 1) return;
         if (dist2(q.x - shifted(obx, ox, P.cdx[0]), q.y - shifted(oby, oy, P.cdx[1]),
                   q.z - shifted(obz, oz, P.cdx[2])) < P.R2)
             ++c[sp == 0 ? 0 : 2];
-    }
+    });
     out[3 * i] = c[0];
     out[3 * i + 1] = c[1];
     out[3 * i + 2] = c[2];
@@ -2983,6 +3207,12 @@ __global__ void __launch_bounds__(kBlock) k_conservation_solid(const DevParams P
 namespace fsim_rt {
 
 #define FSIM_LAUNCH(KB, ARGS, THREADS) KB<<<g, THREADS, 0, st>>>(items_of<ARGS>(pl, L), tb, n)
+// a launch of the list rebuild (L.act: the plan's rebuilding instances) or a plain batched one
+#define FSIM_LAUNCH_G(KB, KG, ARGS, THREADS)                                                               \
+    if (L.act)                                                                                             \
+        KG<<<g, THREADS, 0, st>>>(items_of<ARGS>(pl, L), L.act, L.per);                                    \
+    else                                                                                                   \
+        FSIM_LAUNCH(KB, ARGS, THREADS)
 // one instance by value; up to ParamBlock<ARGS>::kMax as a parameter block; else the item array
 #define FSIM_LAUNCH_P(KB, ARGS, THREADS)                                                                    \
     if (n == 1) {                                                                                          \
@@ -3067,18 +3297,20 @@ fsim_status enqueue_plan(const Plan &pl, cudaStream_t st, int shape_arg, cudaEve
         if (per_launch) CK(cudaEventRecord(per_launch[2 * k], st));
         switch (L.kind) {
         case L_ZERO: FSIM_LAUNCH(kb_zero, ZeroArgs, kBlock); break;
-        case L_HASH: FSIM_LAUNCH(kb_hash, HashArgs, kBlock); break;
-        case L_SCAN_REDUCE: FSIM_LAUNCH(kb_scan_reduce, ScanArgs, kScanThreads); break;
-        case L_SCAN_PARTIALS: FSIM_LAUNCH(kb_scan_partials, ScanArgs, kScanThreads); break;
-        case L_SCAN_APPLY: FSIM_LAUNCH(kb_scan_apply, ScanArgs, kScanThreads); break;
-        case L_SCATTER: FSIM_LAUNCH(kb_scatter, ScatterArgs, kBlock); break;
+        case L_HASH: FSIM_LAUNCH_G(kb_hash, kg_hash, HashArgs, kBlock); break;
+        case L_SCAN_REDUCE: FSIM_LAUNCH_G(kb_scan_reduce, kg_scan_reduce, ScanArgs, kScanThreads); break;
+        case L_SCAN_PARTIALS: FSIM_LAUNCH_G(kb_scan_partials, kg_scan_partials, ScanArgs, kScanThreads); break;
+        case L_SCAN_APPLY: FSIM_LAUNCH_G(kb_scan_apply, kg_scan_apply, ScanArgs, kScanThreads); break;
+        case L_SCATTER: FSIM_LAUNCH_G(kb_scatter, kg_scatter, ScatterArgs, kBlock); break;
         case L_GATHER_F: FSIM_LAUNCH(kb_gather_fluid, GatherFluidArgs, kBlock); break;
         case L_GATHER_S: FSIM_LAUNCH(kb_gather_solid, GatherSolidArgs, kBlock); break;
         case L_RANK_F:
         case L_RANK_S: FSIM_LAUNCH(kb_rank, RankArgs, kBlock); break;
         case L_NL_DECIDE: FSIM_LAUNCH(kb_nl_decide, NlDecideArgs, kBlock); break;
-        case L_NL_BUILD: FSIM_LAUNCH(kb_nl_build, NlBuildArgs, kNlBuildWarps * 32); break;
-        case L_MIXED_ABS: FSIM_LAUNCH(kb_mixed_abs, MixedAbsArgs, kBlock); break;
+        case L_NL_BUILD:
+            kg_nl_build<<<g, kNlBuildWarps * 32, 0, st>>>(items_of<NlBuildArgs>(pl, L), L.act, L.per);
+            break;
+        case L_MIXED_ABS: kg_mixed_abs<<<g, kBlock, 0, st>>>(items_of<MixedAbsArgs>(pl, L), L.act, L.per); break;
         case L_MIXED_REC: FSIM_LAUNCH(kb_mixed_records, CellRefArgs, kBlock); break;
         case L_COUPLE: FSIM_LAUNCH(kb_couple, CoupleArgs, kBlock); break;
         case L_VIRT: FSIM_LAUNCH(kb_virt, VirtArgs, kBlock); break;
@@ -3089,20 +3321,21 @@ fsim_status enqueue_plan(const Plan &pl, cudaStream_t st, int shape_arg, cudaEve
                 if (tune_ev) CK(cudaEventRecord(tune_ev[2 * tr], st));
                 const int *tbs = reinterpret_cast<const int *>(pl.arena + L.shape_table_off[shape]);
                 const int gs = L.shape_blocks[shape], thr = kShapeWarps[shape] * 32;
+                const size_t sm = L.lane_shift ? sizeof(float) * 32 * kSweepTermRows * kShapeWarps[shape] : 0;
                 if (L.variant >= kSweepNlVariant) {
                     const bool mx = L.variant >= kSweepNlMixedVariant;
                     const int v = L.variant - (mx ? kSweepNlMixedVariant : kSweepNlVariant);
                     if (n == 1) {
                         const Item<FluidSweepArgs> &it = host_item<FluidSweepArgs>(pl, L);
-                        (mx ? nlm1 : nl1)[v][shape]<<<gs, thr, 0, st>>>(it.P, it.A);
+                        (mx ? nlm1 : nl1)[v][shape]<<<gs, thr, sm, st>>>(it.P, it.A);
                     } else if (n <= kSweepParamItems) {
                         static thread_local SweepBatchParams B;
                         B.n = n;
                         std::memcpy(B.bstart, pl.host.data() + L.shape_table_off[shape], sizeof(int) * (n + 1));
                         std::memcpy(B.it, pl.host.data() + L.items_off, sizeof(Item<FluidSweepArgs>) * n);
-                        (mx ? nlmp : nlp)[v][shape]<<<gs, thr, 0, st>>>(B);
+                        (mx ? nlmp : nlp)[v][shape]<<<gs, thr, sm, st>>>(B);
                     } else {
-                        (mx ? nlmb : nlb)[v][shape]<<<gs, thr, 0, st>>>(items_of<FluidSweepArgs>(pl, L), tbs, n);
+                        (mx ? nlmb : nlb)[v][shape]<<<gs, thr, sm, st>>>(items_of<FluidSweepArgs>(pl, L), tbs, n);
                     }
                 } else if (n == 1) {
                     const Item<FluidSweepArgs> &it = host_item<FluidSweepArgs>(pl, L);
@@ -3206,9 +3439,9 @@ void launch_k_iota(int grid, cudaStream_t st, int *a, int n)
     k_iota<<<grid, kBlock, 0, st>>>(a, n);
 }
 
-void launch_k_virt_normal(int grid, cudaStream_t st, const DevParams P, const float4 *v_posr, const int *v_cell, const int *start_v, float4 *v_normal, int n)
+void launch_k_virt_normal(int grid, cudaStream_t st, const DevParams P, const float4 *v_posr, const int *v_cell, const int *start_v, float4 *v_normal, int n, int reach)
 {
-    k_virt_normal<<<grid, kBlock, 0, st>>>(P, v_posr, v_cell, start_v, v_normal, n);
+    k_virt_normal<<<grid, kBlock, 0, st>>>(P, v_posr, v_cell, start_v, v_normal, n, reach);
 }
 
 void launch_k_fluid_to_mixed(int grid, cudaStream_t st, const DevParams P, float4 *posr, float4 *velp, int *cell, int n, unsigned *flags)
@@ -3251,24 +3484,24 @@ void launch_k_probe(int grid, cudaStream_t st, const DevParams P, const ProbeArg
     k_probe<<<grid, kBlock, 0, st>>>(P, A);
 }
 
-void launch_k_neighbor_counts(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, int *out, int n)
+void launch_k_neighbor_counts(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, int reach_v, int *out, int n)
 {
-    k_neighbor_counts<<<grid, kBlock, 0, st>>>(P, Pv, fposr, cell_f, start_f, ids_f, s_pos, start_s, ids_s, v_posr, start_v, out, n);
+    k_neighbor_counts<<<grid, kBlock, 0, st>>>(P, Pv, fposr, cell_f, start_f, ids_f, s_pos, start_s, ids_s, v_posr, start_v, reach_v, out, n);
 }
 
-void launch_k_neighbor_counts_nl(int grid, cudaStream_t st, const DevParams P, const float4 *fposr, const int *list, const int *cnt, int cap, const float4 *s_pos, const float4 *v_posr, int *out, int n)
+void launch_k_neighbor_counts_nl(int grid, cudaStream_t st, const DevParams P, const float4 *fposr, const int *list, const int2 *cnt, const float4 *s_pos, const float4 *v_posr, int *out, int n)
 {
-    k_neighbor_counts_nl<<<grid, kBlock, 0, st>>>(P, fposr, list, cnt, cap, s_pos, v_posr, out, n);
+    k_neighbor_counts_nl<<<grid, kBlock, 0, st>>>(P, fposr, list, cnt, s_pos, v_posr, out, n);
 }
 
-void launch_k_neighbor_counts_mixed(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, const unsigned *v_cxyz, int *out, int n)
+void launch_k_neighbor_counts_mixed(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, const unsigned *v_cxyz, int reach_v, int *out, int n)
 {
-    k_neighbor_counts_mixed<<<grid, kBlock, 0, st>>>(P, Pv, fposr, cell_f, start_f, ids_f, s_pos, start_s, ids_s, v_posr, start_v, v_cxyz, out, n);
+    k_neighbor_counts_mixed<<<grid, kBlock, 0, st>>>(P, Pv, fposr, cell_f, start_f, ids_f, s_pos, start_s, ids_s, v_posr, start_v, v_cxyz, reach_v, out, n);
 }
 
-void launch_k_neighbor_counts_nlm(int grid, cudaStream_t st, const DevParams P, const float4 *fposr, const int *cell_f, const unsigned *cxyz_f, const int *list, const int *cnt, int cap, const float4 *s_pos, const unsigned *cxyz_s, const float4 *v_posr, const unsigned *cxyz_v, int *out, int n)
+void launch_k_neighbor_counts_nlm(int grid, cudaStream_t st, const DevParams P, const float4 *fposr, const int *cell_f, const unsigned *cxyz_f, const int *list, const int2 *cnt, const float4 *s_pos, const unsigned *cxyz_s, const float4 *v_posr, const unsigned *cxyz_v, int *out, int n)
 {
-    k_neighbor_counts_nlm<<<grid, kBlock, 0, st>>>(P, fposr, cell_f, cxyz_f, list, cnt, cap, s_pos, cxyz_s, v_posr, cxyz_v, out, n);
+    k_neighbor_counts_nlm<<<grid, kBlock, 0, st>>>(P, fposr, cell_f, cxyz_f, list, cnt, s_pos, cxyz_s, v_posr, cxyz_v, out, n);
 }
 
 void launch_k_gather_f4(int grid, cudaStream_t st, const int *ids, const float4 *src, int n, float4 *dst)

@@ -101,9 +101,10 @@ struct fsim_sim {
     bool nl_check = false;        // pairs also need neighbouring impact-grid cells (f_cxyz, v_icxyz, s_cxyz)
     unsigned *f_cxyz = nullptr, *v_icxyz = nullptr;
     DevParams Pl;                 // the list grid's parameters (else unused)
-    int ncell_l = 0, nl_cap = 0;
+    int ncell_l = 0, nl_cap = 0, nl_reach = 1;
     float nl_R2s = 0.0f, nl_move2 = 0.0f;
-    int *nl_list = nullptr, *nl_cnt = nullptr;
+    int *nl_list = nullptr;
+    int2 *nl_cnt = nullptr;
     NlState *nl_state = nullptr;
     float4 *f_x0 = nullptr, *s_x0 = nullptr;
     int *f_ids = nullptr, *f_lcell = nullptr, *f_lcnt = nullptr, *f_lstart = nullptr;
@@ -301,6 +302,7 @@ void free_plan(Plan *pl)
     }
     if (pl->tgraph) cudaGraphDestroy(pl->tgraph);
     if (pl->arena) cudaFree(pl->arena);
+    if (pl->act) cudaFree(pl->act);
     delete pl;
 }
 
@@ -359,17 +361,22 @@ void add_sweep_launch(Plan &pl, ArenaBuilder &ab, const std::vector<Item<FluidSw
 // the list decision; on a rebuild, the counting sort of fluid and solid on the
 // list grid, else an unpermuted copy; the per-step impact-grid index; on a
 // rebuild, the list build.
-// Blocks a gated launch gets per instance at most (8 per SM of a GB300; the
-// list build, whose blocks carry uneven work, 32 per SM): each loops over its
-// element blocks when its instance rebuilds and returns at once when it does
-// not.  A grid shared by a batch's instances (equally, or in proportion to
-// their particles) measured slower: in a batch some member rebuilds in most
-// steps, and its sort and build then ran on a fraction of the GPU.
-constexpr int kGatedGrid = 8 * 152, kGatedBuildGrid = 32 * 152;
+// Blocks of a launch of the list rebuild, for the whole plan (each loops): 4 per
+// SM of a GB300 for the sort, 2 of the scans' 1024 threads, 12 for the build.
+constexpr int kRebuildGrid = 4 * 152, kRebuildScanGrid = 2 * 152, kRebuildBuildGrid = 12 * 152;
 
-int gated_grid(int grid, long long n, int block)
+// A launch that works on the rebuilding instances only (`per` items each).
+template <class Args>
+void add_rebuild_launch(Plan &pl, ArenaBuilder &ab, int kind, const std::vector<Item<Args>> &items,
+                        const std::vector<int> &blocks_per_item, int grid, int per)
 {
-    return n > 0 ? (int)std::min<long long>(grid, blocks_for(n, block)) : 0;
+    const size_t before = pl.launches.size();
+    add_launch(pl, ab, kind, items, blocks_per_item);
+    if (pl.launches.size() == before) return;
+    Launch &L = pl.launches.back();
+    L.act = pl.act;
+    L.per = per;
+    L.blocks = std::min(L.blocks, grid);
 }
 
 void plan_cell_nl(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, int pf, int ps)
@@ -378,7 +385,7 @@ void plan_cell_nl(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, 
     std::vector<int> db;
     for (fsim_sim *h : m) {
         const int nb = std::min(64, std::max(1, blocks_for(h->ns, kBlock)));
-        NlDecideArgs a{h->nl_state, h->s_pos[ps], h->s_x0, h->ns, h->nl_move2, nb};
+        NlDecideArgs a{h->nl_state, h->s_pos[ps], h->s_x0, h->ns, h->nl_move2, nb, pl.act, (int)m.size()};
         Item<NlDecideArgs> it{h->P, a};
         di.push_back(it);
         db.push_back(nb);
@@ -391,54 +398,45 @@ void plan_cell_nl(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, 
         std::vector<Item<MixedAbsArgs>> ai;
         std::vector<int> abk;
         for (fsim_sim *h : m) {
-            const int ag = gated_grid(kGatedGrid, h->nf, kBlock);
-            const Item<MixedAbsArgs> it{h->P, MixedAbsArgs{h->f_posr[pf], h->f_cell, h->f_rec, h->nf,
-                                                           &h->nl_state->rebuild, ag}};
+            const Item<MixedAbsArgs> it{h->P, MixedAbsArgs{h->f_posr[pf], h->f_cell, h->f_rec, h->nf}};
             ai.push_back(it);
-            abk.push_back(ag);
+            abk.push_back(blocks_for(h->nf, kBlock));
         }
-        add_launch(pl, ab, L_MIXED_ABS, ai, abk);
+        add_rebuild_launch(pl, ab, L_MIXED_ABS, ai, abk, kRebuildGrid, 1);
     }
-    // list-grid sort, run only when the decision says rebuild
-    std::vector<Item<ZeroArgs>> zi;
+    // list-grid sort of the instances that rebuild (the counts start at zero;
+    // the scatter zeroes them again)
     std::vector<Item<HashArgs>> hi;
     std::vector<Item<ScanArgs>> si;
     std::vector<Item<ScatterArgs>> ci;
-    std::vector<int> zb, hb, sb, sp, cb;
+    std::vector<int> hb, sb, sp, cb;
     for (fsim_sim *h : m) {
-        const int *gate = &h->nl_state->rebuild;
         for (int s_ = 0; s_ < 2; ++s_) {
             const int n = s_ ? h->ns : h->nf;
             int *lcnt = s_ ? h->s_lcnt : h->f_lcnt, *lstart = s_ ? h->s_lstart : h->f_lstart;
-            const int zn = n ? h->ncell_l : 0, zg = gated_grid(kGatedGrid, zn, kBlock);
-            const Item<ZeroArgs> z{h->Pl, ZeroArgs{lcnt, zn, gate, zg}};
-            zi.push_back(z);
-            zb.push_back(zg);
-            const int hg = gated_grid(kGatedGrid, n, kBlock);
             const float4 *fpos = mixed ? h->f_rec : h->f_posr[pf];
-            const HashArgs ha = s_ ? HashArgs{h->s_pos[ps], h->ns, h->s_key, h->s_slot, lcnt, h->d_flags, gate, hg}
-                                   : HashArgs{fpos, h->nf, h->f_key, h->f_slot, lcnt, h->d_flags, gate, hg};
+            const HashArgs ha = s_ ? HashArgs{h->s_pos[ps], h->ns, h->s_key, h->s_slot, lcnt, h->d_flags}
+                                   : HashArgs{fpos, h->nf, h->f_key, h->f_slot, lcnt, h->d_flags};
             const Item<HashArgs> hh{h->Pl, ha};
             hi.push_back(hh);
-            hb.push_back(hg);
-            const Item<ScanArgs> sc{h->Pl,
-                                    ScanArgs{lcnt, lstart, h->ncell_l, h->scan_partials + (s_ ? kMaxScanTiles : 0), gate}};
+            hb.push_back(blocks_for(n, kBlock));
+            const Item<ScanArgs> sc{h->Pl, ScanArgs{lcnt, lstart, n ? h->ncell_l : 0,
+                                                    h->scan_partials + (s_ ? kMaxScanTiles : 0)}};
             si.push_back(sc);
             sb.push_back(n ? blocks_for(h->ncell_l, kScanTile) : 0);
             sp.push_back(n ? 1 : 0);
-            const ScatterArgs ca = s_ ? ScatterArgs{h->s_key, h->s_slot, lstart, h->s_tmp, h->ns, gate, hg}
-                                      : ScatterArgs{h->f_key, h->f_slot, lstart, h->f_tmp, h->nf, gate, hg};
+            const ScatterArgs ca = s_ ? ScatterArgs{h->s_key, h->s_slot, lstart, h->s_tmp, h->ns, lcnt}
+                                      : ScatterArgs{h->f_key, h->f_slot, lstart, h->f_tmp, h->nf, lcnt};
             const Item<ScatterArgs> cc{h->Pl, ca};
             ci.push_back(cc);
-            cb.push_back(hg);
+            cb.push_back(blocks_for(n, kBlock));
         }
     }
-    add_launch(pl, ab, L_ZERO, zi, zb);
-    add_launch(pl, ab, L_HASH, hi, hb);
-    add_launch(pl, ab, L_SCAN_REDUCE, si, sb);
-    add_launch(pl, ab, L_SCAN_PARTIALS, si, sp);
-    add_launch(pl, ab, L_SCAN_APPLY, si, sb);
-    add_launch(pl, ab, L_SCATTER, ci, cb);
+    add_rebuild_launch(pl, ab, L_HASH, hi, hb, kRebuildGrid, 2);
+    add_rebuild_launch(pl, ab, L_SCAN_REDUCE, si, sb, kRebuildScanGrid, 2);
+    add_rebuild_launch(pl, ab, L_SCAN_PARTIALS, si, sp, kRebuildScanGrid, 2);
+    add_rebuild_launch(pl, ab, L_SCAN_APPLY, si, sb, kRebuildScanGrid, 2);
+    add_rebuild_launch(pl, ab, L_SCATTER, ci, cb, kRebuildGrid, 2);
     std::vector<Item<GatherFluidArgs>> gf;
     std::vector<Item<GatherSolidArgs>> gs;
     std::vector<int> gfb, gsb;
@@ -464,11 +462,9 @@ void plan_cell_nl(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, 
     add_launch(pl, ab, L_GATHER_F, gf, gfb);
     add_launch(pl, ab, L_GATHER_S, gs, gsb);
     // the per-step impact-grid index of the particles as they now lie
-    zi.clear();
     hi.clear();
     si.clear();
     ci.clear();
-    zb.clear();
     hb.clear();
     sb.clear();
     sp.clear();
@@ -487,22 +483,20 @@ void plan_cell_nl(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, 
                 hmi.push_back(hm);
                 hmb.push_back(blocks_for(n, kBlock));
             } else {
-                const HashArgs ha = s_ ? HashArgs{h->s_pos[1 - ps], h->ns, h->s_key, h->s_slot, cnt, h->d_flags,
-                                                  nullptr}
-                                       : HashArgs{h->f_posr[1 - pf], h->nf, h->f_key, h->f_slot, cnt, h->d_flags,
-                                                  nullptr};
+                const HashArgs ha = s_ ? HashArgs{h->s_pos[1 - ps], h->ns, h->s_key, h->s_slot, cnt, h->d_flags}
+                                       : HashArgs{h->f_posr[1 - pf], h->nf, h->f_key, h->f_slot, cnt, h->d_flags};
                 const Item<HashArgs> hh{h->P, ha};
                 hi.push_back(hh);
                 hb.push_back(blocks_for(n, kBlock));
             }
             const Item<ScanArgs> sc{h->P,
-                                    ScanArgs{cnt, start, h->ncell, h->scan_partials + (s_ ? kMaxScanTiles : 0), nullptr}};
+                                    ScanArgs{cnt, start, h->ncell, h->scan_partials + (s_ ? kMaxScanTiles : 0)}};
             si.push_back(sc);
             sb.push_back(n ? blocks_for(h->ncell, kScanTile) : 0);
             sp.push_back(n ? 1 : 0);
             // the scatter zeroes the counts again (set to zero at creation)
-            const ScatterArgs ca = s_ ? ScatterArgs{h->s_key, h->s_slot, start, h->s_tmp, h->ns, nullptr, 0, cnt}
-                                      : ScatterArgs{h->f_key, h->f_slot, start, h->f_tmp, h->nf, nullptr, 0, cnt};
+            const ScatterArgs ca = s_ ? ScatterArgs{h->s_key, h->s_slot, start, h->s_tmp, h->ns, cnt}
+                                      : ScatterArgs{h->f_key, h->f_slot, start, h->f_tmp, h->nf, cnt};
             const Item<ScatterArgs> cc{h->P, ca};
             ci.push_back(cc);
             cb.push_back(blocks_for(n, kBlock));
@@ -542,16 +536,15 @@ void plan_cell_nl(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, 
     std::vector<Item<NlBuildArgs>> bi;
     std::vector<int> bb;
     for (fsim_sim *h : m) {
-        const int bg = gated_grid(kGatedBuildGrid, h->nf, kNlBuildThreads);
         const NlBuildArgs ba{h->f_x0,   h->f_lcell,  h->f_lstart, mixed ? h->v_abs : h->v_posr, h->v_start,
                              h->s_x0,   h->s_lstart, h->nf,       h->nl_cap,  h->nl_list,
                              h->nl_cnt, h->nl_state, h->d_flags,  h->nl_R2s,  h->nv,
-                             h->ns,     bg};
+                             h->ns,     h->nl_reach};
         const Item<NlBuildArgs> bt{h->Pl, ba};
         bi.push_back(bt);
-        bb.push_back(bg);
+        bb.push_back(blocks_for(h->nf, kNlBuildThreads));
     }
-    add_launch(pl, ab, L_NL_BUILD, bi, bb);
+    add_rebuild_launch(pl, ab, L_NL_BUILD, bi, bb, kRebuildBuildGrid, 1);
 }
 
 // The cell phase: counting sort of fluid and solid (parity pf -> 1-pf, ps -> 1-ps).
@@ -658,6 +651,17 @@ void plan_virt(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, int
     add_launch(pl, ab, m.empty() || !m[0]->mixed ? L_VIRT : L_VIRT_M, it, nb);
 }
 
+// Lanes that share a particle of the list sweep (log2), by the fluid particles
+// of the whole plan.  One lane walks a list of ~12 groups, a chain of memory
+// latencies: while the particles leave most of the GPU's 152 x 2048 threads idle
+// more lanes shorten it, and beyond that they only repeat the per-particle work.
+// Sweep with 1 / 4 / 8 / 16 lanes: 1.4 k particles 26 / 22 / 17 / 14 us, 32 k 29 /
+// 31 / 38 / 55 us (64 and 63 us before the branch-free walk).
+int sweep_lane_shift(long long n)
+{
+    return n <= 8192 ? 4 : n <= 16384 ? 2 : 0;
+}
+
 // fluid sweep + update (parity pf -> 1-pf)
 void plan_fluid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, int pf, int ps)
 {
@@ -665,6 +669,9 @@ void plan_fluid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, in
     std::vector<int> nb[kSweepShapes];
     bool any_check = false;
     int nvisc = 0;
+    long long total = 0;
+    for (fsim_sim *h : m) total += h->nf;
+    const int lane_shift = !m.empty() && m[0]->nl ? sweep_lane_shift(total) : 0;
     for (fsim_sim *h : m) {
         FluidSweepArgs A;
         A.posr = h->f_posr[pf];
@@ -698,8 +705,9 @@ void plan_fluid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, in
         A.nl_cxyz_v = h->nl_check ? h->v_icxyz : nullptr;
         A.nl_cxyz_s = h->nl_check ? h->s_cxyz : nullptr;
         A.rec = h->f_rec;
+        A.lane_shift = lane_shift;
         it.push_back({h->P, A});
-        for (int sh = 0; sh < kSweepShapes; ++sh) nb[sh].push_back(blocks_for(h->nf, kShapeWarps[sh] * 32));
+        for (int sh = 0; sh < kSweepShapes; ++sh) nb[sh].push_back(blocks_for((long long)h->nf << A.lane_shift, kShapeWarps[sh] * 32));
         if (h->nf) {
             any_check = any_check || h->check_z;
             nvisc += h->P.viscid ? 1 : 0;
@@ -712,7 +720,10 @@ void plan_fluid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, in
     add_sweep_launch(pl, ab, it, nb,
                      nl ? (mixed ? kSweepNlMixedVariant : kSweepNlVariant) + visc_mode
                         : mixed ? 6 + visc_mode : (any_check ? 3 : 0) + visc_mode);
-    if (pl.launches.size() > before) pl.sweep_index = (int)before;
+    if (pl.launches.size() > before) {
+        pl.sweep_index = (int)before;
+        pl.launches.back().lane_shift = lane_shift;
+    }
 }
 
 // solid sub-steps (in place on parity ps; the fluid is read at parity pf):
@@ -826,6 +837,17 @@ fsim_status build_plan(const std::vector<fsim_sim *> &m, unsigned phases, int pf
     pl->pf = pf;
     pl->ps = ps;
     ArenaBuilder ab;
+    if ((phases & (1u << FSIM_PHASE_CELL)) && !m.empty() && m[0]->nl) {
+        cudaError_t e = cudaMalloc((void **)&pl->act, sizeof(int) * (2 + m.size()));
+        if (e == cudaSuccess) e = cudaMemset(pl->act, 0, sizeof(int) * (2 + m.size()));
+        if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy); // the plan runs on a stream of its own
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            fsim_set_error("plan allocation failed: %s", cudaGetErrorString(e));
+            free_plan(pl);
+            return FSIM_ENOMEM;
+        }
+    }
     if (phases & (1u << FSIM_PHASE_CELL)) {
         plan_cell(*pl, ab, m, pf, ps);
         pf ^= 1;
@@ -1007,7 +1029,7 @@ fsim_status check_flags(fsim_sim *h)
     }
     if (flags & FLAG_LIST_OVERFLOW) {
         fsim_set_error("a fluid particle has more than %d neighbour-list candidates (results invalid); "
-                       "lower gb300_neighbor_skin or set it to 0", h->nl_cap);
+                       "lower gb300_neighbor_skin or set it to 0", h->nl_cap - kNlPad);
         return FSIM_ENUMERIC;
     }
     if (flags & FLAG_CELL_OVERFULL) {
@@ -1062,12 +1084,12 @@ fsim_status sort_virtual(fsim_sim *h, const float *vpos_host, float4 *vpos_dev =
     CK_LAUNCH();
     Plan pl;
     ArenaBuilder ab;
-    add_launch(pl, ab, L_ZERO, std::vector<Item<ZeroArgs>>{{G, ZeroArgs{cnt, gcells, nullptr}}},
+    add_launch(pl, ab, L_ZERO, std::vector<Item<ZeroArgs>>{{G, ZeroArgs{cnt, gcells}}},
                {blocks_for(gcells, kBlock)});
     add_launch(pl, ab, L_HASH,
-               std::vector<Item<HashArgs>>{{G, HashArgs{tmp_pos, n, key, slot, cnt, h->d_flags, nullptr}}},
+               std::vector<Item<HashArgs>>{{G, HashArgs{tmp_pos, n, key, slot, cnt, h->d_flags}}},
                {blocks_for(n, kBlock)});
-    const std::vector<Item<ScanArgs>> sc{{G, ScanArgs{cnt, h->v_start, gcells, h->scan_partials, nullptr}}};
+    const std::vector<Item<ScanArgs>> sc{{G, ScanArgs{cnt, h->v_start, gcells, h->scan_partials}}};
     add_launch(pl, ab, L_SCAN_REDUCE, sc, {blocks_for(gcells, kScanTile)});
     add_launch(pl, ab, L_SCAN_PARTIALS, sc, {1});
     add_launch(pl, ab, L_SCAN_APPLY, sc, {blocks_for(gcells, kScanTile)});
@@ -1086,7 +1108,8 @@ fsim_status sort_virtual(fsim_sim *h, const float *vpos_host, float4 *vpos_dev =
     if (e == cudaSuccess && (st = enqueue_plan(pl, h->stream, 0)) == FSIM_OK) {
         e = cudaMemsetAsync(h->v_velp, 0, sizeof(float4) * n, h->stream);
         // the normal sums the walls within R: any grid of cells >= R finds them
-        launch_k_virt_normal(blocks_for(n, kBlock), h->stream, G, h->v_posr, h->v_cell, h->v_start, h->v_normal, n);
+        launch_k_virt_normal(blocks_for(n, kBlock), h->stream, G, h->v_posr, h->v_cell, h->v_start, h->v_normal, n,
+                             h->nl ? h->nl_reach : 1);
         if (h->nl) launch_k_cells_of(blocks_for(n, kBlock), h->stream, h->P, h->v_posr, n, h->v_icell, h->v_icxyz);
         if (e == cudaSuccess) e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
@@ -1232,7 +1255,8 @@ fsim_status alloc_state(fsim_sim *h)
         return st;
     // virtual
     if ((st = dalloc(h, &h->v_posr, nv)) || (st = dalloc(h, &h->v_velp, nv)) || (st = dalloc(h, &h->v_normal, nv)) ||
-        (st = dalloc(h, &h->v_orig, nv)) || (st = dalloc(h, &h->v_cell, nv)) || (st = dalloc(h, &h->v_start, nc + 1)))
+        (st = dalloc(h, &h->v_orig, nv)) || (st = dalloc(h, &h->v_cell, nv)) ||
+        (st = dalloc(h, &h->v_start, (h->nl ? h->ncell_l : nc) + 1)))
         return st;
     // fluid neighbour lists
     if (h->nl) {
@@ -1251,9 +1275,11 @@ fsim_status alloc_state(fsim_sim *h)
         NlState init{};
         init.force = 1; // the first step builds
         CK(cudaMemcpyAsync(h->nl_state, &init, sizeof init, cudaMemcpyHostToDevice, h->stream));
-        CK(cudaMemsetAsync(h->nl_cnt, 0, sizeof(int) * (nf ? nf : 1), h->stream));
+        CK(cudaMemsetAsync(h->nl_cnt, 0, sizeof(int2) * (nf ? nf : 1), h->stream));
         CK(cudaMemsetAsync(h->f_x0, 0, sizeof(float4) * (nf ? nf : 1), h->stream));
         CK(cudaMemsetAsync(h->s_x0, 0, sizeof(float4) * (ns ? ns : 1), h->stream));
+        CK(cudaMemsetAsync(h->f_lcnt, 0, sizeof(int) * ncl, h->stream));
+        CK(cudaMemsetAsync(h->s_lcnt, 0, sizeof(int) * ncl, h->stream));
         CK(cudaMemsetAsync(h->f_lstart, 0, sizeof(int) * (ncl + 1), h->stream));
         CK(cudaMemsetAsync(h->s_lstart, 0, sizeof(int) * (ncl + 1), h->stream));
         // the per-step cell index starts from zero counts; each sort's scatter
@@ -1273,7 +1299,7 @@ fsim_status alloc_state(fsim_sim *h)
     CK(cudaMemsetAsync(h->f_cell, 0, sizeof(int) * (nf ? nf : 1), h->stream));
     CK(cudaMemsetAsync(h->f_start, 0, sizeof(int) * (nc + 1), h->stream));
     CK(cudaMemsetAsync(h->s_start, 0, sizeof(int) * (nc + 1), h->stream));
-    CK(cudaMemsetAsync(h->v_start, 0, sizeof(int) * (nc + 1), h->stream));
+    CK(cudaMemsetAsync(h->v_start, 0, sizeof(int) * ((h->nl ? h->ncell_l : nc) + 1), h->stream));
     CK(cudaMemsetAsync(h->s_np, 0, sizeof(float4) * (ns ? ns : 1), h->stream));
     return FSIM_OK;
 }
@@ -1346,12 +1372,36 @@ namespace {
 // on all three axes) that is the set {r < R}, else (nl_check) the list sweep
 // also compares the pair's packed cell coordinates.  The list grid has cells
 // of at least Rs (1 + 1e-3) on the reference grid's origin.
+// The list grid's cells per axis (at least Rs (1 + 1e-3) / reach wide) and its
+// reach, the finest of 3, 2, 1 whose cells stay few enough.  The finer the
+// cells, the fewer candidates a build tests (about 310 against 730 per
+// particle) and the more a warp's lanes walk alike.  Instances of up to 262,144
+// fluid particles keep reach 1: there the sweep is bound by latency and not by
+// the L1, so the order gains it nothing.
+int list_grid(const fsim_derived &d, double Rs, size_t nf, size_t ns, size_t nv, int n[3])
+{
+    for (int reach = nf > 262144 ? 3 : 1;; --reach) {
+        double cells = 1.0;
+        bool fits = true;
+        for (int a = 0; a < 3; ++a) {
+            const double L = (double)d.cell_max[a] - (double)d.cell_min[a];
+            const double c = std::max(1.0, std::floor(reach * L / (Rs * (1.0 + 1e-3))));
+            n[a] = (int)std::min(c, 1e9);
+            cells *= c;
+            // FP32 rounding of the cell coordinate against the 1e-3 margin
+            fits = fits && 8e-7 * c < 0.5e-3 * reach;
+        }
+        const double most = std::min((double)kMaxScanTiles * kScanTile, 64.0 * ((double)nf + ns + nv) + 65536.0);
+        if (reach == 1 || (fits && cells <= most)) return reach;
+    }
+}
+
 void setup_lists(fsim_sim *h)
 {
     h->nl = false;
     h->nl_check = false;
     const double skin = h->cfg.neighbor_skin;
-    if (!(skin > 0.0) || h->nf > kNlIndexMask || h->nv > kNlIndexMask || h->ns > kNlIndexMask) return;
+    if (!(skin > 0.0) || h->nf > kNlIndexMax || h->nv > kNlIndexMax || h->ns > kNlIndexMax) return;
     const double R = std::sqrt((double)h->der.impact_distance_square);
     for (int a = 0; a < 3; ++a) {
         const double margin = (double)h->der.interval[a] / R - 1.0;
@@ -1372,14 +1422,15 @@ void setup_lists(fsim_sim *h)
     if (!(move > 0.0)) return;
     DevParams Pl = h->P;
     int n[3];
+    const int reach = list_grid(h->der, Rs, h->nf, h->ns, h->nv, n);
     for (int a = 0; a < 3; ++a) {
         const double L = (double)h->der.cell_max[a] - (double)h->der.cell_min[a];
-        n[a] = std::max(1, (int)std::floor(L / (Rs * (1.0 + 1e-3))));
         Pl.cinv[a] = (float)(n[a] / L);
         Pl.cdx[a] = (float)(L / n[a]);
         // the cells must still hold Rs with the FP32 inverse the kernels use
-        if (!(1.0 / (double)Pl.cinv[a] >= Rs * (1.0 + 5e-4))) return;
+        if (!(reach / (double)Pl.cinv[a] >= Rs * (1.0 + 5e-4))) return;
     }
+    h->nl_reach = reach;
     Pl.nx = n[0];
     Pl.ny = n[1];
     Pl.nz = n[2];
@@ -1391,7 +1442,9 @@ void setup_lists(fsim_sim *h)
     // list capacity: 1.5x a full sphere of radius Rs at the particle spacing
     const double dx = h->cfg.particle_diameter;
     const double full = 4.0 / 3.0 * 3.14159265358979 * std::pow(Rs / dx, 3.0);
-    h->nl_cap = ((int)std::ceil(1.5 * full) + 16 + kNlGroup - 1) & ~(kNlGroup - 1); // whole groups
+    const double cap = std::ceil(1.5 * full) + 16 + kNlGroup - 1;
+    if (!(cap + kNlPad < kNlCapMax)) return;
+    h->nl_cap = ((int)cap & ~(kNlGroup - 1)) + kNlPad; // whole groups
     h->nl = true;
 }
 
@@ -1951,11 +2004,11 @@ extern "C" fsim_status fsim_neighbor_counts(fsim_handle h, int *out, size_t byte
         launch_k_neighbor_counts_mixed(g, h->stream, h->P, h->nl ? h->Pl : h->P, h->f_posr[h->f_cur], h->f_cell,
                                        h->f_start, h->nl ? h->f_ids : nullptr, h->s_pos[h->s_cur], h->s_start,
                                        h->nl ? h->s_ids : nullptr, h->v_posr, h->v_start,
-                                       h->nl ? h->v_icxyz : nullptr, d_counts, h->nf);
+                                       h->nl ? h->v_icxyz : nullptr, h->nl_reach, d_counts, h->nf);
     else
         launch_k_neighbor_counts(g, h->stream, h->P, h->nl ? h->Pl : h->P, h->f_posr[h->f_cur], h->f_cell,
                                  h->f_start, h->nl ? h->f_ids : nullptr, h->s_pos[h->s_cur], h->s_start,
-                                 h->nl ? h->s_ids : nullptr, h->v_posr, h->v_start, d_counts, h->nf);
+                                 h->nl ? h->s_ids : nullptr, h->v_posr, h->v_start, h->nl_reach, d_counts, h->nf);
     CK_LAUNCH();
     // reorder to input order in place is not possible; copy sorted and unpermute on the host
     std::vector<int> sorted(3 * (size_t)h->nf), orig(h->nf);
@@ -2032,11 +2085,11 @@ extern "C" fsim_status fsim_list_counts(fsim_handle h, int *out, size_t bytes)
     int *d_counts = (int *)h->staging; // 3 * nf words fit the staging buffer
     if (h->mixed)
         launch_k_neighbor_counts_nlm(blocks_for(h->nf, kBlock), h->stream, h->P, h->f_posr[h->f_cur], h->f_cell,
-                                     h->f_cxyz, h->nl_list, h->nl_cnt, h->nl_cap, h->s_pos[h->s_cur], h->s_cxyz,
+                                     h->f_cxyz, h->nl_list, h->nl_cnt, h->s_pos[h->s_cur], h->s_cxyz,
                                      h->v_posr, h->v_icxyz, d_counts, h->nf);
     else
         launch_k_neighbor_counts_nl(blocks_for(h->nf, kBlock), h->stream, h->P, h->f_posr[h->f_cur], h->nl_list,
-                                    h->nl_cnt, h->nl_cap, h->s_pos[h->s_cur], h->v_posr, d_counts, h->nf);
+                                    h->nl_cnt, h->s_pos[h->s_cur], h->v_posr, d_counts, h->nf);
     CK_LAUNCH();
     std::vector<int> sorted(3 * (size_t)h->nf), orig(h->nf);
     CK(cudaMemcpyAsync(sorted.data(), d_counts, bytes, cudaMemcpyDeviceToHost, h->stream));
@@ -2314,6 +2367,7 @@ struct SnapHeader {
     fsim_config cfg;
 };
 constexpr char kSnapMagic[8] = {'F', 'S', 'I', 'M', 'S', 'N', 'P', '1'};
+constexpr uint32_t kSnapVersion = 3;     // version 2 loads too (snap_arrays_v2)
 constexpr size_t kSnapHeaderBytes = 512; // header padded; arrays start 16-byte aligned
 static_assert(sizeof(SnapHeader) <= kSnapHeaderBytes, "snapshot header");
 
@@ -2321,6 +2375,9 @@ struct SnapArray {
     void *dev;
     size_t bytes;
 };
+// places of some arrays in snap_arrays
+enum { kSnapWallPos = 9, kSnapWallVel = 10, kSnapWallOrig = 12, kSnapWallStart = 14, kSnapFluidListStart = 17,
+       kSnapSolidListStart = 20, kSnapListState = 22, kSnapWallAbs = 23 };
 // A neighbour-list instance also saves what its lists were built from (the
 // positions and list-grid cells of the last build, the particles' order then)
 // and its list state; loading rebuilds the same lists from them.
@@ -2331,7 +2388,7 @@ std::vector<SnapArray> snap_arrays(fsim_sim *h, int pf, int ps)
         {h->f_posr[pf], 16 * nf}, {h->f_velp[pf], 16 * nf}, {h->f_orig[pf], 4 * nf},   {h->f_cell, 4 * nf},
         {h->s_pos[ps], 16 * ns},  {h->s_vel[ps], 16 * ns},  {h->s_ref[ps], 16 * ns},   {h->s_type[ps], 4 * ns},
         {h->s_orig[ps], 4 * ns},  {h->v_posr, 16 * nv},     {h->v_velp, 16 * nv},      {h->v_normal, 16 * nv},
-        {h->v_orig, 4 * nv},      {h->v_cell, 4 * nv},      {h->v_start, 4 * (nc + 1)}};
+        {h->v_orig, 4 * nv},      {h->v_cell, 4 * nv},      {h->v_start, 4 * ((h->nl ? h->ncell_l : nc) + 1)}};
     if (h->nl) {
         const size_t ncl = h->ncell_l;
         const std::vector<SnapArray> b = {{h->f_x0, 16 * nf},           {h->f_lcell, 4 * nf},
@@ -2342,6 +2399,89 @@ std::vector<SnapArray> snap_arrays(fsim_sim *h, int pf, int ps)
         if (h->mixed) a.push_back({h->v_abs, 16 * nv});
     }
     return a;
+}
+
+// Version 2 of the format, of a neighbour-list instance: the same arrays, but
+// the particles and walls were sorted on a list grid of cells as wide as the
+// list radius.  What describes that order comes back as {nullptr, bytes}.
+std::vector<SnapArray> snap_arrays_v2(fsim_sim *h)
+{
+    std::vector<SnapArray> a = snap_arrays(h, 0, 0);
+    if (!h->nl) return a;
+    const double R = std::sqrt((double)h->der.impact_distance_square), Rs = R * (1.0 + h->cfg.neighbor_skin);
+    size_t ncl = 1;
+    for (int k = 0; k < 3; ++k) {
+        const double L = (double)h->der.cell_max[k] - (double)h->der.cell_min[k];
+        ncl *= (size_t)std::max(1, (int)std::floor(L / (Rs * (1.0 + 1e-3))));
+    }
+    a[kSnapWallStart].bytes = 4 * ((size_t)h->ncell + 1);
+    a[kSnapFluidListStart].bytes = a[kSnapSolidListStart].bytes = 4 * (ncl + 1);
+    for (size_t k = kSnapWallPos; k < a.size(); ++k) a[k].dev = nullptr;
+    return a;
+}
+
+size_t snap_payload(const std::vector<SnapArray> &arrays)
+{
+    size_t b = 0;
+    for (const SnapArray &a : arrays) b += (a.bytes + 15) & ~size_t(15);
+    return b;
+}
+
+// The walls and list state of a version-2 snapshot of a neighbour-list
+// instance: the walls sorted anew with their densities, velocities and
+// pressures, and a list build forced at the next step.
+fsim_status restore_v2_lists(fsim_sim *h, const char *in)
+{
+    const std::vector<SnapArray> arrays = snap_arrays_v2(h);
+    std::vector<const char *> at;
+    for (const SnapArray &a : arrays) {
+        at.push_back(in);
+        in += (a.bytes + 15) & ~size_t(15);
+    }
+    const char *posr = at[kSnapWallPos], *velp = at[kSnapWallVel], *orig = at[kSnapWallOrig],
+               *abs = h->mixed ? at[kSnapWallAbs] : posr;
+    const size_t nv = h->nv;
+    std::vector<float> xyz(3 * nv);
+    std::vector<float4> u(nv), by_input(nv), sorted(nv);
+    std::vector<float> rho(nv);
+    for (size_t k = 0; k < nv; ++k) {
+        int o;
+        float4 x, r, v;
+        std::memcpy(&o, orig + 4 * k, 4);
+        std::memcpy(&r, posr + 16 * k, 16);
+        std::memcpy(&x, abs + 16 * k, 16);
+        std::memcpy(&v, velp + 16 * k, 16);
+        if (o < 0 || o >= h->nv) {
+            fsim_set_error("corrupt snapshot (wall ids)");
+            return FSIM_EIO;
+        }
+        xyz[3 * (size_t)o] = x.x;
+        xyz[3 * (size_t)o + 1] = x.y;
+        xyz[3 * (size_t)o + 2] = x.z;
+        rho[o] = r.w;
+        by_input[o] = v;
+    }
+    fsim_status st;
+    if (nv) {
+        if ((st = sort_virtual(h, xyz.data()))) return st;
+        if (h->mixed && (st = walls_to_mixed(h))) return st;
+        std::vector<int> order(nv);
+        CK(cudaStreamSynchronize(h->stream));
+        CK(cudaMemcpy(order.data(), h->v_orig, sizeof(int) * nv, cudaMemcpyDeviceToHost));
+        CK(cudaMemcpy(sorted.data(), h->v_posr, sizeof(float4) * nv, cudaMemcpyDeviceToHost));
+        for (size_t k = 0; k < nv; ++k) {
+            sorted[k].w = rho[order[k]];
+            u[k] = by_input[order[k]];
+        }
+        CK(cudaMemcpy(h->v_posr, sorted.data(), sizeof(float4) * nv, cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(h->v_velp, u.data(), sizeof(float4) * nv, cudaMemcpyHostToDevice));
+    }
+    NlState saved, fresh{};
+    std::memcpy(&saved, at[kSnapListState], sizeof saved);
+    fresh.builds = saved.builds;
+    fresh.force = 1;
+    CK(cudaMemcpy(h->nl_state, &fresh, sizeof fresh, cudaMemcpyHostToDevice));
+    return FSIM_OK;
 }
 
 // Build the lists from the saved build state (positions and cells of the last
@@ -2360,20 +2500,25 @@ fsim_status nl_restore(fsim_sim *h)
     }
     Plan pl;
     ArenaBuilder ab;
-    add_launch(pl, ab, L_NL_BUILD,
+    const int only[3] = {1, 0, 0}; // one rebuilding instance, the plan's first
+    CK(cudaMalloc((void **)&pl.act, sizeof only));
+    add_rebuild_launch(pl, ab, L_NL_BUILD,
                std::vector<Item<NlBuildArgs>>{{h->Pl, NlBuildArgs{h->f_x0, h->f_lcell, h->f_lstart, vpos,
                                                                   h->v_start, h->s_x0, h->s_lstart, h->nf, h->nl_cap,
                                                                   h->nl_list, h->nl_cnt, h->nl_state, h->d_flags,
-                                                                  h->nl_R2s, h->nv, h->ns}}},
-               {blocks_for(h->nf, kNlBuildThreads)});
+                                                                  h->nl_R2s, h->nv, h->ns, h->nl_reach}}},
+               {blocks_for(h->nf, kNlBuildThreads)}, kRebuildBuildGrid, 1);
     pl.host = ab.bytes;
-    CK(cudaMalloc((void **)&pl.arena, ab.bytes.size()));
-    cudaError_t e = cudaMemcpy(pl.arena, ab.bytes.data(), ab.bytes.size(), cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMalloc((void **)&pl.arena, std::max<size_t>(ab.bytes.size(), 1));
+    if (e == cudaSuccess) e = cudaMemcpy(pl.act, only, sizeof only, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(pl.arena, ab.bytes.data(), ab.bytes.size(), cudaMemcpyHostToDevice);
     fsim_status st = FSIM_OK;
     if (e == cudaSuccess) st = enqueue_plan(pl, h->stream, 0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     cudaFree(pl.arena);
+    cudaFree(pl.act);
     pl.arena = nullptr;
+    pl.act = nullptr;
     if (e != cudaSuccess) {
         fsim_set_error("rebuilding the neighbour lists failed: %s", cudaGetErrorString(e));
         return FSIM_ECUDA;
@@ -2382,18 +2527,12 @@ fsim_status nl_restore(fsim_sim *h)
     CK(cudaMemcpy(h->nl_state, &saved, sizeof saved, cudaMemcpyHostToDevice));
     return FSIM_OK;
 }
-size_t snap_payload(fsim_sim *h)
-{
-    size_t b = 0;
-    for (const SnapArray &a : snap_arrays(h, 0, 0)) b += (a.bytes + 15) & ~size_t(15);
-    return b;
-}
 } // namespace
 
 extern "C" fsim_status fsim_snapshot_bytes(fsim_handle h, size_t *bytes)
 {
     if (!h || !bytes) return FSIM_EINVAL;
-    *bytes = kSnapHeaderBytes + snap_payload(h);
+    *bytes = kSnapHeaderBytes + snap_payload(snap_arrays(h, 0, 0));
     return FSIM_OK;
 }
 
@@ -2402,7 +2541,7 @@ extern "C" fsim_status fsim_snapshot_save(fsim_handle h, long long step, void *b
     NvtxRange nvtx_("fsim_snapshot_save");
     if (!h || !buf) return FSIM_EINVAL;
     if (h->batch) batch_wait(h);
-    const size_t need = kSnapHeaderBytes + snap_payload(h);
+    const size_t need = kSnapHeaderBytes + snap_payload(snap_arrays(h, 0, 0));
     if (bytes != need) {
         fsim_set_error("a snapshot of this instance takes %zu bytes, got %zu", need, bytes);
         return FSIM_EINVAL;
@@ -2411,7 +2550,7 @@ extern "C" fsim_status fsim_snapshot_save(fsim_handle h, long long step, void *b
     SnapHeader hd;
     std::memset(&hd, 0, sizeof hd);
     std::memcpy(hd.magic, kSnapMagic, 8);
-    hd.version = 2;
+    hd.version = kSnapVersion;
     hd.config_bytes = sizeof(fsim_config);
     hd.step = step;
     hd.n_fluid = h->nf;
@@ -2446,15 +2585,17 @@ extern "C" fsim_status fsim_snapshot_load(const void *buf, size_t bytes, int dev
         return FSIM_EIO;
     }
     std::memcpy(&hd, buf, sizeof hd);
-    if (std::memcmp(hd.magic, kSnapMagic, 8) || hd.version != 2 || hd.config_bytes != sizeof(fsim_config) ||
+    if (std::memcmp(hd.magic, kSnapMagic, 8) || (hd.version != 2 && hd.version != kSnapVersion) || hd.config_bytes != sizeof(fsim_config) ||
         hd.n_fluid < 0 || hd.n_solid < 0 || hd.n_virt < 0) {
-        fsim_set_error("not a version-2 fluidsim snapshot");
+        fsim_set_error("not a version-2 or version-3 fluidsim snapshot");
         return FSIM_EIO;
     }
     fsim_sim *h = nullptr;
     fsim_status st = new_handle(&hd.cfg, hd.n_fluid, hd.n_solid, hd.n_virt, device, &h);
     if (st) return st;
-    if (h->ncell != hd.ncell || bytes != kSnapHeaderBytes + snap_payload(h) ||
+    // (no array is allocated yet: only the sizes count here)
+    const bool v2 = hd.version == 2;
+    if (h->ncell != hd.ncell || bytes != kSnapHeaderBytes + snap_payload(v2 ? snap_arrays_v2(h) : snap_arrays(h, 0, 0)) ||
         hd.payload_bytes != bytes - kSnapHeaderBytes) {
         fsim_set_error("snapshot size does not match its header");
         delete h;
@@ -2472,8 +2613,8 @@ extern "C" fsim_status fsim_snapshot_load(const void *buf, size_t bytes, int dev
     std::vector<float> ref(3 * (size_t)ns);
     const char *ref_src = nullptr, *orig_src = nullptr;
     cudaError_t e = cudaSuccess;
-    for (const SnapArray &a : snap_arrays(h, 0, 0)) {
-        if (a.bytes && e == cudaSuccess) e = cudaMemcpy(a.dev, in + off, a.bytes, cudaMemcpyHostToDevice);
+    for (const SnapArray &a : v2 ? snap_arrays_v2(h) : snap_arrays(h, 0, 0)) {
+        if (a.dev && a.bytes && e == cudaSuccess) e = cudaMemcpy(a.dev, in + off, a.bytes, cudaMemcpyHostToDevice);
         if (a.dev == h->s_ref[0]) ref_src = in + off;
         if (a.dev == h->s_orig[0]) orig_src = in + off;
         off += (a.bytes + 15) & ~size_t(15);
@@ -2514,7 +2655,7 @@ extern "C" fsim_status fsim_snapshot_load(const void *buf, size_t bytes, int dev
             return st ? st : FSIM_ECUDA;
         }
     }
-    if (h->nl && (st = nl_restore(h))) {
+    if (h->nl && (st = v2 ? restore_v2_lists(h, in + kSnapHeaderBytes) : nl_restore(h))) {
         free_all(h);
         delete h;
         return st;
@@ -3092,17 +3233,22 @@ extern "C" fsim_status fsim_estimate_bytes(const fsim_config *cfg, int n_fluid, 
     if (cfg->precision == FSIM_PRECISION_MIXED) b += nc * sizeof(float2); // per-cell references
     if (cfg->neighbor_skin > 0.0f) {
         // fluid neighbour lists (as setup_lists sizes them) and the list-grid
-        // sort, build state and per-step index (at most as many cells as nc):
+        // sort, build state and per-step index:
         // lists, list counts, ids, list cells, packed cells; x0, the 32-byte
         // records and the positions in the index's order; the mixed form's
         // carried cells and absolute wall positions
         const double rs = std::sqrt((double)d.impact_distance_square) * (1.0 + cfg->neighbor_skin) /
                           (double)cfg->particle_diameter;
-        const size_t cap = (((size_t)std::ceil(1.5 * 4.18879 * rs * rs * rs) + 16 + kNlGroup - 1) & ~size_t(kNlGroup - 1));
-        b += nf * (cap + 4) * sizeof(int) + nf * 4 * sizeof(float4);
+        const size_t cap = (((size_t)std::ceil(1.5 * 4.18879 * rs * rs * rs) + 16 + kNlGroup - 1) & ~size_t(kNlGroup - 1)) + kNlPad;
+        b += nf * (cap + 5) * sizeof(int) + nf * 4 * sizeof(float4);
         b += ns * (sizeof(float4) + 2 * sizeof(int)) + nv * 2 * sizeof(int);
         if (cfg->precision == FSIM_PRECISION_MIXED) b += nf * sizeof(int) + nv * sizeof(float4);
-        b += nc * sizeof(int) * 2 + (nc + 1) * sizeof(int) * 2 + sizeof(NlState);
+        int n[3];
+        const double skin = cfg->neighbor_skin;
+        list_grid(d, std::sqrt((double)d.impact_distance_square) * (1.0 + skin), nf, ns, nv, n);
+        const size_t ncl = (size_t)n[0] * n[1] * n[2];
+        b += (ncl * 2 + (ncl + 1) * 2) * sizeof(int) + sizeof(NlState);
+        if (ncl > nc) b += (ncl - nc) * sizeof(int); // the walls' starts
     }
     b += 2 * kMaxScanTiles * sizeof(int) + sizeof(unsigned);
     size_t words = 3 * nf;

@@ -77,25 +77,16 @@ struct Item {
 
 // ---- argument blocks of the batched kernels (one Item per instance)
 // cell phase: hash (plain / mixed), count reset, scans, scatter, gathers
-// `gate` (neighbour-list instances): when set, the kernel runs only in steps
-// whose *gate is non-zero (a list rebuild); the other steps skip it.  `grid`
-// (0: one block per blockDim.x elements): the blocks launched for the item,
-// each looping over the element blocks -- a small grid, so that a gated launch
-// that has nothing to do costs little.
 struct HashArgs {
     const float4 *pos;
     int n;
     int *key, *slot, *cnt;
     unsigned *flags;
-    const int *gate;
-    int grid;
 };
 
 struct ZeroArgs {
     int *p;
     int n;
-    const int *gate;
-    int grid;
 };
 
 struct ScanArgs {
@@ -103,23 +94,21 @@ struct ScanArgs {
     int *out;
     int n;
     int *partial;
-    const int *gate;
 };
 
 struct ScatterArgs {
     const int *key, *slot, *start;
     int *tmp;
     int n;
-    const int *gate;
-    int grid;
     // the sort's cell counts, which the hash filled and the scan has read:
     // zeroed here cell by cell (every counted cell holds a particle), so that
     // the next sort needs no zeroing launch (nullptr: left as they are)
     int *reset;
 };
 
-// With a gate, a step that does not rebuild copies the state unpermuted; a
-// step that does also records the new positions in x0_out.
+// `gate` (neighbour-list instances): a step whose *gate is zero does not rebuild
+// and copies the state unpermuted; a step that does rebuild also records the new
+// positions in x0_out.
 struct GatherFluidArgs {
     const int *tmp, *key, *start;
     int n;
@@ -146,8 +135,6 @@ struct MixedAbsArgs {
     const int *cell;
     float4 *out;
     int n;
-    const int *gate;
-    int grid;
 };
 
 struct GatherSolidArgs {
@@ -188,14 +175,16 @@ struct NlDecideArgs {
     int ns;
     float move2; // squared displacement allowed since the build: ((Rs - R) / 2 - rounding slack)^2
     int nblocks;
+    int *act;    // the plan's rebuilding instances: count, decided instances, indices
+    int ninst;   // instances of the plan
 };
 
 // list build: every fluid particle's candidates within the list radius among
-// fluid, wall and solid particles of its 27 cells of the list grid (whose
-// cells are at least the list radius), in cell-row order; entry = index |
-// species << kNlSpeciesShift, in groups of kNlGroup: entry e of particle i at
+// fluid, wall and solid particles of the list grid's cells around it; entries
+// are slots, in groups of kNlGroup: entry e of particle i at
 // ((e / kNlGroup) * n + i) * kNlGroup + e % kNlGroup, so that a lane writes and
-// reads a whole 32-byte sector per group and a warp's group is 1 KB contiguous
+// reads a whole 32-byte sector per group and a warp's group is 1 KB contiguous.
+// Each species' entries start on a whole group: fluid, then wall, then solid.
 struct NlBuildArgs {
     const float4 *posr;       // fluid positions at the build (sorted on the list grid)
     const int *cell_f, *start_f;
@@ -204,16 +193,18 @@ struct NlBuildArgs {
     const float4 *s_pos;
     const int *start_s;
     int n, cap;
-    int *list, *cnt;
+    int *list;
+    int2 *cnt;                // (fluid entries, wall entries | solid entries << 16)
     NlState *nl;
     unsigned *flags;
     float R2s; // list radius^2
     int nv, ns;
-    int grid;  // blocks launched (each loops over warps of particles; 0: one block per 4 warps)
+    int reach; // cells of the list grid that cover the list radius
 };
-constexpr int kNlSpeciesShift = 30; // list entry: index | species << 30 (0 fluid, 1 wall, 2 solid)
-constexpr int kNlGroup = 8;         // list entries per 32-byte group (the capacity is a multiple)
-constexpr int kNlIndexMask = (1 << kNlSpeciesShift) - 1;
+constexpr int kNlGroup = 8;                // list entries per 32-byte group (the capacity is a multiple)
+constexpr int kNlPad = 2 * kNlGroup;       // capacity set aside for the species' group boundaries
+constexpr int kNlIndexMax = (1 << 30) - 1; // particles of a species
+constexpr int kNlCapMax = 32768;           // entries of a species fit 16 bits
 
 // fused fluid sweep + update (plain and mixed)
 struct FluidSweepArgs {
@@ -232,7 +223,8 @@ struct FluidSweepArgs {
     const float2 *cm; // mixed form: per-cell (density deviation, pressure) references
     // neighbour-list sweep: the lists, the positions of the last build and the
     // instance's list state (largest displacement since the build)
-    const int *nl_list, *nl_cnt;
+    const int *nl_list;
+    const int2 *nl_cnt;
     int nl_cap, nl_nv, nl_ns; // list capacity; wall and solid counts
     const float4 *x0;
     NlState *nl;
@@ -244,6 +236,9 @@ struct FluidSweepArgs {
     // the step-start (posr, velp) of every fluid slot side by side: one
     // 32-byte sector per fluid neighbour, fetched with one 256-bit load
     const float4 *rec;
+    // list sweep: 2^lane_shift lanes share a particle (the same for all
+    // instances of a launch; results do not depend on it)
+    int lane_shift;
 };
 
 // The cell walks below take `ids_*`: nullptr when the particles are sorted by
@@ -468,6 +463,8 @@ constexpr int kIndexMask = (1 << kCodeShift) - 1;
 // launch shapes of the fluid sweep the autotuner chooses among
 constexpr int kSweepShapes = 3;
 
+constexpr int kSweepTermRows = 6; // list sweep with lanes: shared-memory rows of a warp's pair terms
+
 constexpr int kShapeWarps[kSweepShapes] = {4, 4, 8}; // warps per block of sweep shapes 0..2
 
 // L_SWEEP variants: 0-5 stream sweep (CHECK_Z * 3 + VISCID mode), 6-8 mixed
@@ -494,11 +491,14 @@ struct Launch {
     int kind;
     size_t items_off, table_off; // arena offsets
     int ninst, blocks, variant;
+    int lane_shift = 0;                   // L_SWEEP: lanes per particle of the list sweep (log2)
     size_t shape_table_off[kSweepShapes]; // L_SWEEP: block prefix table per launch shape
     int shape_blocks[kSweepShapes];
     size_t table2_off, barrier_off;       // L_SOLID_FUSED: thread-per-particle table, grid barrier
     int max_sub;
     unsigned polls;                       // L_SOLID_FUSED: barrier wait limit, 0 = the default
+    const int *act = nullptr;             // launches of the list rebuild: the plan's rebuilding instances
+    int per = 1;                          //   and the items each instance has
 };
 
 struct Plan {
@@ -507,6 +507,7 @@ struct Plan {
     int pf_after = 0, ps_after = 0;
     std::vector<Launch> launches;
     char *arena = nullptr;
+    int *act = nullptr;           // list instances: the rebuilding ones of the step (see NlDecideArgs)
     std::vector<char> host; // host image of the arena (one-instance launches pass items by value)
     cudaGraphExec_t graph = nullptr;
     int sweep_index = -1;         // launch index of the fluid sweep
@@ -571,7 +572,7 @@ int fused_grid(bool mixed, int want);
 // One launch of a utility kernel (kBlock threads per block) on `st`.
 void launch_k_pack_f4(int grid, cudaStream_t st, const float *xyz, const float *w, int n, float wconst, float4 *out);
 void launch_k_iota(int grid, cudaStream_t st, int *a, int n);
-void launch_k_virt_normal(int grid, cudaStream_t st, const DevParams P, const float4 *v_posr, const int *v_cell, const int *start_v, float4 *v_normal, int n);
+void launch_k_virt_normal(int grid, cudaStream_t st, const DevParams P, const float4 *v_posr, const int *v_cell, const int *start_v, float4 *v_normal, int n, int reach);
 void launch_k_fluid_to_mixed(int grid, cudaStream_t st, const DevParams P, float4 *posr, float4 *velp, int *cell, int n, unsigned *flags);
 void launch_k_offsets_in_cells(int grid, cudaStream_t st, const DevParams P, float4 *pos, const int *cell, int n);
 void launch_k_unpermute_mixed(int grid, cudaStream_t st, const DevParams P, const float4 *pos, const float4 *velp, const int *cell, const int *orig, int n, int what, float *out);
@@ -580,10 +581,10 @@ void launch_k_unpermute_words(int grid, cudaStream_t st, const int *src, const i
 void launch_k_permute_in_mixed(int grid, cudaStream_t st, const DevParams P, float4 *pos, float4 *velp, const int *cell, const int *orig, int n, int what, const float *in);
 void launch_k_permute_in_f4(int grid, cudaStream_t st, float4 *dst, const int *orig, int n, int comp, int width, const float *in);
 void launch_k_probe(int grid, cudaStream_t st, const DevParams P, const ProbeArgs A);
-void launch_k_neighbor_counts(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, int *out, int n);
-void launch_k_neighbor_counts_nl(int grid, cudaStream_t st, const DevParams P, const float4 *fposr, const int *list, const int *cnt, int cap, const float4 *s_pos, const float4 *v_posr, int *out, int n);
-void launch_k_neighbor_counts_mixed(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, const unsigned *v_cxyz, int *out, int n);
-void launch_k_neighbor_counts_nlm(int grid, cudaStream_t st, const DevParams P, const float4 *fposr, const int *cell_f, const unsigned *cxyz_f, const int *list, const int *cnt, int cap, const float4 *s_pos, const unsigned *cxyz_s, const float4 *v_posr, const unsigned *cxyz_v, int *out, int n);
+void launch_k_neighbor_counts(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, int reach_v, int *out, int n);
+void launch_k_neighbor_counts_nl(int grid, cudaStream_t st, const DevParams P, const float4 *fposr, const int *list, const int2 *cnt, const float4 *s_pos, const float4 *v_posr, int *out, int n);
+void launch_k_neighbor_counts_mixed(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, const unsigned *v_cxyz, int reach_v, int *out, int n);
+void launch_k_neighbor_counts_nlm(int grid, cudaStream_t st, const DevParams P, const float4 *fposr, const int *cell_f, const unsigned *cxyz_f, const int *list, const int2 *cnt, const float4 *s_pos, const unsigned *cxyz_s, const float4 *v_posr, const unsigned *cxyz_v, int *out, int n);
 void launch_k_gather_f4(int grid, cudaStream_t st, const int *ids, const float4 *src, int n, float4 *dst);
 void launch_k_pack_records(int grid, cudaStream_t st, const float4 *posr, const float4 *velp, const unsigned *cxyz, int n, float4 *rec);
 void launch_k_nl_displacement(int grid, cudaStream_t st, const DevParams P, const float4 *posr, const int *cell, const float4 *x0, int n, NlState *nl);
