@@ -109,6 +109,40 @@ __device__ __forceinline__ void neighbor_rows(const DevParams &P, int c, Rows &r
     }
 }
 
+// The index ranges of the 9 rows, all read at once: a walk that reads a row's
+// range when it gets there adds a memory latency per row, and where the walks
+// are short or empty (most walls and most of a solid see no fluid) those
+// latencies are its whole time.  z0: the rows' first cell.  With SPLIT also
+// where each row's second and third cell begin.
+template <bool SPLIT = false>
+struct RowRanges {
+    int b[9], e[9], b1[SPLIT ? 9 : 1], b2[SPLIT ? 9 : 1];
+    int cx, cy, cz, z0;
+    __device__ __forceinline__ RowRanges(const DevParams &P, int c, const int *__restrict__ start)
+    {
+        const int row = c / P.nz;
+        cz = c - row * P.nz;
+        cx = row / P.ny;
+        cy = row - cx * P.ny;
+        z0 = max(cz - 1, 0);
+        const int z1 = min(cz + 1, P.nz - 1) + 1;
+#pragma unroll
+        for (int r = 0; r < 9; ++r) {
+            const int x = cx + r / 3 - 1, y = cy + r % 3 - 1;
+            b[r] = e[r] = 0;
+            if (x >= 0 && x < P.nx && y >= 0 && y < P.ny) {
+                const int base = (x * P.ny + y) * P.nz;
+                b[r] = start[base + z0];
+                e[r] = start[base + z1];
+                if (SPLIT) {
+                    b1[r] = start[base + min(z0 + 1, z1)];
+                    b2[r] = start[base + min(z0 + 2, z1)];
+                }
+            }
+        }
+    }
+};
+
 // f(c0, c1) for the cell rows [c0, c1) within `reach` cells of cell c on each axis.
 template <class F>
 __device__ __forceinline__ void for_rows_within(const DevParams &P, int c, int reach, F &&f)
@@ -1265,32 +1299,61 @@ __global__ void __launch_bounds__(SH::threads, SH::min_blocks) kb_fluid_sweep_nl
 // getVirtData (src/virt.cu:9-75): nearest fluid particle's rho, hydrostatically
 // corrected p and velocity mirrored about the (static) wall normal.  Ties in
 // distance go to the smaller input id.
+// Bound by latency: all row ranges load at once, candidates four at a time (a
+// row's last one stands in past its end: a repeated candidate changes nothing),
+// and particle ids only to break a tie in distance -- read for every new nearest,
+// two dependent loads that one lane or another of a warp waited for at nearly
+// every candidate, they were most of the walk's time.
+struct NearestFluid {
+    float best = FSIM_LARGE_FLOAT;
+    int t = -1;
+    // the particle of walk slot t
+    __device__ __forceinline__ int particle(const VirtArgs &A) const
+    {
+        const int j = t < 0 || !A.ids_f ? t : A.ids_f[t];
+        FSIM_DCHECK(j >= -1 && j < A.nf, 32u, return -1);
+        return j;
+    }
+    // candidate slot tc at squared distance d2: true when it becomes the nearest
+    __device__ __forceinline__ bool take(const VirtArgs &A, int tc, float d2)
+    {
+        if (!(d2 <= best) || tc == t) return false;
+        if (d2 == best && t >= 0) {
+            const NearestFluid c{d2, tc};
+            const int jc = c.particle(A), jt = particle(A);
+            if (jc < 0 || (jt >= 0 && A.forig[jc] > A.forig[jt])) return false;
+        }
+        best = d2;
+        t = tc;
+        return true;
+    }
+};
+// the position of walk slot t
+__device__ __forceinline__ float4 walk_pos(const VirtArgs &A, int t)
+{
+    return A.fpos_t ? A.fpos_t[t] : A.fposr[A.ids_f ? A.ids_f[t] : t];
+}
 __device__ __forceinline__ void virt_body(const DevParams &P, const VirtArgs &A, int blk)
 {
     const int i = blk * blockDim.x + threadIdx.x;
     if (i >= A.n) return;
     const float4 xi = A.v_posr_in[i];
-    Rows rows;
-    neighbor_rows(P, A.v_cell[i], rows);
-    float best = FSIM_LARGE_FLOAT;
-    int best_j = -1, best_orig = INT_MAX;
-    for (int r = 0; r < rows.count; ++r) {
-        for (int t = A.start_f[rows.base[r] + rows.z0], te = A.start_f[rows.base[r] + rows.z1]; t < te; ++t) {
-            // with the index's position copy, the particle id only for a new best
-            const float4 q = A.fpos_t ? A.fpos_t[t] : A.fposr[A.ids_f ? A.ids_f[t] : t];
-            const float d2 = dist2(q.x - xi.x, q.y - xi.y, q.z - xi.z);
-            if (d2 <= best) {
-                const int j = A.ids_f ? A.ids_f[t] : t;
-                FSIM_DCHECK(j >= 0 && j < A.nf, 32u, continue);
-                const int o = A.forig[j];
-                if (d2 < best || o < best_orig) {
-                    best = d2;
-                    best_j = j;
-                    best_orig = o;
-                }
+    const RowRanges<> R(P, A.v_cell[i], A.start_f);
+    NearestFluid N;
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+        for (int t = R.b[r], last = R.e[r] - 1; t <= last; t += 4) {
+            float d2[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float4 q = walk_pos(A, min(t + c, last));
+                d2[c] = dist2(q.x - xi.x, q.y - xi.y, q.z - xi.z);
             }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) N.take(A, min(t + c, last), d2[c]);
         }
     }
+    const int best_j = N.particle(A);
     float rho = P.rho0, p = 0.0f, ux = 0.0f, uy = 0.0f, uz = 0.0f;
     if (best_j >= 0) {
         const float4 q = A.fposr[best_j], u = A.fvelp[best_j];
@@ -1370,6 +1433,37 @@ __device__ __forceinline__ float group_sum(float v)
 // solidCoupleUpdate (src/solid.cu:262-344): solid normal from the solid
 // neighbours' kernel gradients, solid pressure as the Shepard average of the
 // fluid pressure.  kCoupleGroup lanes per solid particle.
+// A lane's share of the normal: the solid candidates of the rows, two at a time
+// (two chains of index and position loads in flight), summed in walk order.
+__device__ __forceinline__ void couple_normal(const DevParams &P, const CoupleArgs &A, const RowRanges<> &S, float4 xi,
+                                              int g, float &nx, float &ny, float &nz)
+{
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+        for (int ts = S.b[r] + g; ts < S.e[r]; ts += 2 * kCoupleGroup) {
+            float4 q[2];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const int t = min(ts + c * kCoupleGroup, S.e[r] - 1);
+                const int j = A.ids_s ? A.ids_s[t] : t;
+                q[c] = xi; // own position: adds nothing
+                FSIM_DCHECK(j >= 0 && j < A.n, 128u, continue);
+                q[c] = A.s_pos[j];
+            }
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const float dx = q[c].x - xi.x, dy = q[c].y - xi.y, dz = q[c].z - xi.z;
+                const float r2 = dist2(dx, dy, dz);
+                if (r2 < P.R2 && ts + c * kCoupleGroup < S.e[r]) {
+                    const float w = __expf(-r2 * P.h_inv2) * P.kdiff;
+                    nx -= dx * w;
+                    ny -= dy * w;
+                    nz -= dz * w;
+                }
+            }
+        }
+    }
+}
 __device__ __forceinline__ void couple_body(const DevParams &P, const CoupleArgs &A, int blk)
 {
     const int t = blk * blockDim.x + threadIdx.x;
@@ -1378,11 +1472,10 @@ __device__ __forceinline__ void couple_body(const DevParams &P, const CoupleArgs
     float nx = 0.0f, ny = 0.0f, nz = 0.0f, psum = 0.0f, wsum = 0.0f;
     if (valid) {
         const float4 xi = A.s_pos[i];
-        Rows rows;
-        neighbor_rows(P, A.s_cell[i], rows);
-        for (int r = 0; r < rows.count; ++r) {
-            const int c0 = rows.base[r] + rows.z0, c1 = rows.base[r] + rows.z1;
-            for (int tf = A.start_f[c0] + g, te = A.start_f[c1]; tf < te; tf += kCoupleGroup) {
+        const RowRanges<> F(P, A.s_cell[i], A.start_f), S(P, A.s_cell[i], A.start_s);
+#pragma unroll
+        for (int r = 0; r < 9; ++r) {
+            for (int tf = F.b[r] + g; tf < F.e[r]; tf += kCoupleGroup) {
                 const float4 q = A.fpos_t ? A.fpos_t[tf] : A.fposr[A.ids_f ? A.ids_f[tf] : tf];
                 const float dx = q.x - xi.x, dy = q.y - xi.y, dz = q.z - xi.z;
                 const float r2 = dist2(dx, dy, dz);
@@ -1394,20 +1487,8 @@ __device__ __forceinline__ void couple_body(const DevParams &P, const CoupleArgs
                     psum += A.fvelp[j].w * w;
                 }
             }
-            for (int ts = A.start_s[c0] + g, te = A.start_s[c1]; ts < te; ts += kCoupleGroup) {
-                const int j = A.ids_s ? A.ids_s[ts] : ts;
-                FSIM_DCHECK(j >= 0 && j < A.n, 128u, continue);
-                const float4 q = A.s_pos[j];
-                const float dx = q.x - xi.x, dy = q.y - xi.y, dz = q.z - xi.z;
-                const float r2 = dist2(dx, dy, dz);
-                if (r2 < P.R2) {
-                    const float w = __expf(-r2 * P.h_inv2) * P.kdiff;
-                    nx -= dx * w;
-                    ny -= dy * w;
-                    nz -= dz * w;
-                }
-            }
         }
+        couple_normal(P, A, S, xi, g, nx, ny, nz);
     }
     nx = group_sum<kCoupleGroup>(nx);
     ny = group_sum<kCoupleGroup>(ny);
@@ -1962,43 +2043,32 @@ __device__ __forceinline__ void virt_mixed_body(const DevParams &P, const VirtAr
     const int i = blk * blockDim.x + threadIdx.x;
     if (i >= A.n) return;
     const float4 xi = A.v_posr_in[i]; // offset from the wall particle's cell
-    int cx, cy, cz;
-    cell_xyz(P, A.v_cell[i], cx, cy, cz);
-    float best = FSIM_LARGE_FLOAT;
-    int best_j = -1, best_orig = INT_MAX;
+    const RowRanges<true> R(P, A.v_cell[i], A.start_f);
+    NearestFluid N;
     float bsx = 0.0f, bsy = 0.0f, bsz = 0.0f;
-    const int z0 = max(cz - 1, 0), z1 = min(cz + 1, P.nz - 1) + 1;
-    for (int ox = -1; ox <= 1; ++ox) {
-        const int x = cx + ox;
-        if (x < 0 || x >= P.nx) continue;
-        const float psx = fmaf(-(float)ox, P.cdx[0], xi.x);
-        for (int oy = -1; oy <= 1; ++oy) {
-            const int y = cy + oy;
-            if (y < 0 || y >= P.ny) continue;
-            const float psy = fmaf(-(float)oy, P.cdx[1], xi.y);
-            const int rb = (x * P.ny + y) * P.nz;
-            for (int z = z0; z < z1; ++z) {
-                const float psz = fmaf(-(float)(z - cz), P.cdx[2], xi.z);
-                for (int t = A.start_f[rb + z], te = A.start_f[rb + z + 1]; t < te; ++t) {
-                    const float4 q = A.fpos_t ? A.fpos_t[t] : A.fposr[A.ids_f ? A.ids_f[t] : t];
-                    const float d2 = dist2(q.x - psx, q.y - psy, q.z - psz);
-                    if (d2 <= best) {
-                        const int j = A.ids_f ? A.ids_f[t] : t;
-                        FSIM_DCHECK(j >= 0 && j < A.nf, 32u, continue);
-                        const int o = A.forig[j];
-                        if (d2 < best || o < best_orig) {
-                            best = d2;
-                            best_j = j;
-                            best_orig = o;
-                            bsx = psx;
-                            bsy = psy;
-                            bsz = psz;
-                        }
-                    }
-                }
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+        const float psx = fmaf(-(float)(r / 3 - 1), P.cdx[0], xi.x);
+        const float psy = fmaf(-(float)(r % 3 - 1), P.cdx[1], xi.y);
+        for (int t = R.b[r], last = R.e[r] - 1; t <= last; t += 4) {
+            float d2[4], psz[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int tc = min(t + c, last);
+                const float4 q = walk_pos(A, tc);
+                psz[c] = fmaf(-(float)(R.z0 + (tc >= R.b1[r]) + (tc >= R.b2[r]) - R.cz), P.cdx[2], xi.z);
+                d2[c] = dist2(q.x - psx, q.y - psy, q.z - psz[c]);
             }
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (N.take(A, min(t + c, last), d2[c])) {
+                    bsx = psx;
+                    bsy = psy;
+                    bsz = psz[c];
+                }
         }
     }
+    const int best_j = N.particle(A);
     float rho = P.rho0, p = 0.0f, ux = 0.0f, uy = 0.0f, uz = 0.0f;
     if (best_j >= 0) {
         const float4 q = A.fposr[best_j], u = A.fvelp[best_j];
@@ -2050,32 +2120,24 @@ __device__ __forceinline__ void solid_fluid_walk_m(const DevParams &P, const int
                                                    int cell, float4 xi, int g, F &&f,
                                                    const float4 *__restrict__ fpos_t = nullptr)
 {
-    int cx, cy, cz;
-    cell_xyz(P, cell, cx, cy, cz);
-    const float sox = xi.x - fmaf((float)cx, P.cdx[0], P.cmin[0]);
-    const float soy = xi.y - fmaf((float)cy, P.cdx[1], P.cmin[1]);
-    const float soz = xi.z - fmaf((float)cz, P.cdx[2], P.cmin[2]);
-    const int z0 = max(cz - 1, 0), z1 = min(cz + 1, P.nz - 1) + 1;
-    const float sz0 = fmaf(-(float)(z0 - cz), P.cdx[2], soz);
-    for (int ox = -1; ox <= 1; ++ox) {
-        const int x = cx + ox;
-        if (x < 0 || x >= P.nx) continue;
-        for (int oy = -1; oy <= 1; ++oy) {
-            const int y = cy + oy;
-            if (y < 0 || y >= P.ny) continue;
-            const int rb = (x * P.ny + y) * P.nz;
-            RowMixed R;
-            R.z0 = z0;
-            R.b1 = start_f[rb + min(z0 + 1, z1)];
-            R.b2 = start_f[rb + min(z0 + 2, z1)];
-            R.sx = fmaf(-(float)ox, P.cdx[0], sox);
-            R.sy = fmaf(-(float)oy, P.cdx[1], soy);
-            for (int t = start_f[rb + z0] + g, te = start_f[rb + z1]; t < te; t += G) {
-                const float4 q = fpos_t ? fpos_t[t] : fposr[ids ? ids[t] : t];
-                float dx, dy, dz;
-                fluid_rel(P, R, t, sz0, q, dx, dy, dz);
-                f(SlotId{ids, t}, dx, dy, dz);
-            }
+    const RowRanges<true> W(P, cell, start_f);
+    const float sox = xi.x - fmaf((float)W.cx, P.cdx[0], P.cmin[0]);
+    const float soy = xi.y - fmaf((float)W.cy, P.cdx[1], P.cmin[1]);
+    const float soz = xi.z - fmaf((float)W.cz, P.cdx[2], P.cmin[2]);
+    const float sz0 = fmaf(-(float)(W.z0 - W.cz), P.cdx[2], soz);
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+        RowMixed R;
+        R.z0 = W.z0;
+        R.b1 = W.b1[r];
+        R.b2 = W.b2[r];
+        R.sx = fmaf(-(float)(r / 3 - 1), P.cdx[0], sox);
+        R.sy = fmaf(-(float)(r % 3 - 1), P.cdx[1], soy);
+        for (int t = W.b[r] + g; t < W.e[r]; t += G) {
+            const float4 q = fpos_t ? fpos_t[t] : fposr[ids ? ids[t] : t];
+            float dx, dy, dz;
+            fluid_rel(P, R, t, sz0, q, dx, dy, dz);
+            f(SlotId{ids, t}, dx, dy, dz);
         }
     }
 }
@@ -2100,22 +2162,8 @@ __device__ __forceinline__ void couple_mixed_body(const DevParams &P, const Coup
                                             }
                                         },
                                         A.fpos_t);
-        Rows rows;
-        neighbor_rows(P, A.s_cell[i], rows);
-        for (int r = 0; r < rows.count; ++r) {
-            const int c0 = rows.base[r] + rows.z0, c1 = rows.base[r] + rows.z1;
-            for (int ts = A.start_s[c0] + g, te = A.start_s[c1]; ts < te; ts += kCoupleGroup) {
-                const float4 q = A.s_pos[A.ids_s ? A.ids_s[ts] : ts];
-                const float dx = q.x - xi.x, dy = q.y - xi.y, dz = q.z - xi.z;
-                const float r2 = dist2(dx, dy, dz);
-                if (r2 < P.R2) {
-                    const float w = __expf(-r2 * P.h_inv2) * P.kdiff;
-                    nx -= dx * w;
-                    ny -= dy * w;
-                    nz -= dz * w;
-                }
-            }
-        }
+        const RowRanges<> S(P, A.s_cell[i], A.start_s);
+        couple_normal(P, A, S, xi, g, nx, ny, nz);
     }
     nx = group_sum<kCoupleGroup>(nx);
     ny = group_sum<kCoupleGroup>(ny);
@@ -2197,6 +2245,8 @@ __device__ __forceinline__ float solid_pair_weight(const DevParams &P, float dx,
     return __fmul_rn(__expf(__fmul_rn(-dist2(dx, dy, dz), P.h_inv2)), P.kdiff);
 }
 
+constexpr int kSolidAhead = 5; // list entries a lane of the deformation loads ahead
+
 // solidDeformationCalculate (src/solid.cu:10-79): F and L over the
 // reference-configuration neighbours, L^-1 (identity when singular),
 // F <- F L^-1, Green strain, St-Venant-Kirchhoff 2nd Piola, P = F S.
@@ -2220,32 +2270,54 @@ __device__ __forceinline__ void solid_deform_body(const DevParams &P, const Soli
         const float4 xi = S.pos[i], ri = S.ref[i];
         const int o = S.orig[i];
         const unsigned ci = RESOLVE ? S.cxyz[i] : 0u;
-        for (int e = S.nbr_off[o] + g, ee = S.nbr_off[o + 1]; e < ee; e += kSolidGroup) {
-            int j;
-            if (RESOLVE) {
-                const int jj = S.inv[S.nbr_orig[e]];
-                FSIM_DCHECK(jj >= 0 && jj < S.n, 512u, {
-                    S.nbr_slot[e] = -1;
-                    continue;
-                });
-                j = cells_adjacent(ci, S.cxyz[jj]) ? jj : -1;
-                S.nbr_slot[e] = j;
-            } else {
-                j = S.nbr_slot[e];
+        // kSolidAhead entries' loads are in flight together (one at a time, the chain
+        // index -> positions of each of a lane's ~20 entries was the kernel's time:
+        // 12.7 us a launch at 3,680 particles); the sums take them in list order
+        for (int e0 = S.nbr_off[o] + g, ee = S.nbr_off[o + 1]; e0 < ee; e0 += kSolidAhead * kSolidGroup) {
+            int j[kSolidAhead];
+            float4 xj[kSolidAhead], rj[kSolidAhead];
+#pragma unroll
+            for (int u = 0; u < kSolidAhead; ++u) {
+                const int e = e0 + u * kSolidGroup;
+                j[u] = -1;
+                if (e < ee) j[u] = RESOLVE ? S.inv[S.nbr_orig[e]] : S.nbr_slot[e];
             }
-            if (j < 0) continue;
-            const float4 xj = S.pos[j], rj = S.ref[j];
-            const float dx[3] = {xj.x - xi.x, xj.y - xi.y, xj.z - xi.z};
-            const float dX[3] = {__fsub_rn(rj.x, ri.x), __fsub_rn(rj.y, ri.y), __fsub_rn(rj.z, ri.z)};
-            const float w = solid_pair_weight(P, dX[0], dX[1], dX[2]);
+            if (RESOLVE) {
+                unsigned cj[kSolidAhead];
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                // roundings spelled out: the instantiations compute alike
-                const float ra = __fmul_rn(dx[a], w), la = __fmul_rn(dX[a], w);
+                for (int u = 0; u < kSolidAhead; ++u) {
+                    FSIM_DCHECK(j[u] < S.n, 512u, j[u] = -1);
+                    cj[u] = j[u] < 0 ? 0u : S.cxyz[j[u]];
+                }
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    F.m[3 * a + c] = fmaf(ra, dX[c], F.m[3 * a + c]);
-                    if (FORM_L) L.m[3 * a + c] = fmaf(la, dX[c], L.m[3 * a + c]);
+                for (int u = 0; u < kSolidAhead; ++u) {
+                    if (j[u] >= 0 && !cells_adjacent(ci, cj[u])) j[u] = -1;
+                    if (e0 + u * kSolidGroup < ee) S.nbr_slot[e0 + u * kSolidGroup] = j[u];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kSolidAhead; ++u) {
+                const int k = j[u] < 0 ? i : j[u];
+                xj[u] = S.pos[k];
+                rj[u] = S.ref[k];
+            }
+#pragma unroll
+            for (int u = 0; u < kSolidAhead; ++u) {
+                const bool in = j[u] >= 0; // else the entry adds 0 x 0
+                const float dx[3] = {in ? xj[u].x - xi.x : 0.0f, in ? xj[u].y - xi.y : 0.0f,
+                                     in ? xj[u].z - xi.z : 0.0f};
+                const float dX[3] = {in ? __fsub_rn(rj[u].x, ri.x) : 0.0f, in ? __fsub_rn(rj[u].y, ri.y) : 0.0f,
+                                     in ? __fsub_rn(rj[u].z, ri.z) : 0.0f};
+                const float w = solid_pair_weight(P, dX[0], dX[1], dX[2]);
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    // roundings spelled out: the instantiations compute alike
+                    const float ra = __fmul_rn(dx[a], w), la = __fmul_rn(dX[a], w);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        F.m[3 * a + c] = fmaf(ra, dX[c], F.m[3 * a + c]);
+                        if (FORM_L) L.m[3 * a + c] = fmaf(la, dX[c], L.m[3 * a + c]);
+                    }
                 }
             }
         }
@@ -2310,9 +2382,9 @@ __device__ __forceinline__ void solid_deform_body(const DevParams &P, const Soli
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
         S.F[9 * i + k] = F.m[k];
-        S.Pk[9 * i + k] = Pk.m[k];
+        S.F[9 * (S.n + i) + k] = Pk.m[k];
         if (FORM_L) S.L[9 * i + k] = Linv.m[k];
-        S.AV[9 * i + k] = AV.m[k];
+        S.L[9 * (S.n + i) + k] = AV.m[k];
     }
     float4 *pl = reinterpret_cast<float4 *>(S.PL + kPLStride * i);
     pl[0] = make_float4(PL.m[0], PL.m[1], PL.m[2], PL.m[3]);
@@ -2323,6 +2395,29 @@ FSIM_BATCHED_KERNEL(kb_solid_deform, SolidArgs, solid_deform_body<false>, kBlock
 FSIM_BATCHED_KERNEL(kb_solid_deform_mixed, SolidArgs, solid_deform_body<true>, kBlock)
 FSIM_BATCHED_KERNEL(kb_solid_deform_resolve, SolidArgs, (solid_deform_body<false, true>), kBlock)
 FSIM_BATCHED_KERNEL(kb_solid_deform_mixed_resolve, SolidArgs, (solid_deform_body<true, true>), kBlock)
+
+// solidUpdate (src/solid.cu:209-239) of particle i with position x, velocity v
+// and acceleration a, into pos and vel.
+__device__ __forceinline__ void solid_update_particle(const DevParams &P, const SolidArgs &S, int i, float4 x, float4 v,
+                                                      float4 a, float4 *pos, float4 *vel)
+{
+    const int t = S.type[i];
+    if (t == 1) { // FIXED_SOLID
+        v = make_float4(0.0f, 0.0f, 0.0f, v.w);
+        S.dudt[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    } else if (t == 0) { // UNCONSTRAINED_SOLID
+        x.x = fminf(fmaxf(__fmaf_rn(v.x, P.dt_sub, x.x), P.dmin[0]), P.dmax[0]);
+        x.y = fminf(fmaxf(__fmaf_rn(v.y, P.dt_sub, x.y), P.dmin[1]), P.dmax[1]);
+        x.z = fminf(fmaxf(__fmaf_rn(v.z, P.dt_sub, x.z), P.dmin[2]), P.dmax[2]);
+        v.x = __fmaf_rn(__fadd_rn(a.x, P.gx), P.dt_sub, v.x);
+        v.y = __fmaf_rn(__fadd_rn(a.y, P.gy), P.dt_sub, v.y);
+        v.z = __fmaf_rn(__fadd_rn(a.z, P.gz), P.dt_sub, v.z);
+    }
+    pos[i] = x;
+    vel[i] = v;
+}
+
+constexpr int kForceAhead = 2; // list entries a lane of the force sweep loads ahead
 
 // solidForceCalculate (src/solid.cu:81-207): fluid traction over the fluid
 // neighbours (current configuration, fluid already advanced; candidates from
@@ -2340,6 +2435,9 @@ FSIM_BATCHED_KERNEL(kb_solid_deform_mixed_resolve, SolidArgs, (solid_deform_body
 // those of the full walk (FLIST 0) bit for bit; an overflowing list (count -1)
 // or a larger displacement falls back to the walk.  Every rounding of the
 // sums is spelled out so that the three instantiations compute alike.
+//
+// With pos_out the particle is also advanced, into the other of the solid's two
+// buffers (its neighbours still read this one): one launch fewer per sub-step.
 template <bool MIXED, int FLIST = 0>
 __device__ __forceinline__ void solid_force_body(const DevParams &P, const SolidArgs &S, int blk)
 {
@@ -2396,12 +2494,11 @@ __device__ __forceinline__ void solid_force_body(const DevParams &P, const Solid
             }
         }
         if (walk) {
-            Rows rows;
-            neighbor_rows(P, S.cell[i], rows);
+            const RowRanges<> W(P, S.cell[i], S.start_f);
             int nrec = 0;
-            for (int r = 0; r < rows.count; ++r) {
-                const int c0 = rows.base[r] + rows.z0, c1 = rows.base[r] + rows.z1;
-                for (int tf = S.start_f[c0] + g, te = S.start_f[c1]; tf < te; tf += kSolidGroup) {
+#pragma unroll
+            for (int r = 0; r < 9; ++r) {
+                for (int tf = W.b[r] + g; tf < W.e[r]; tf += kSolidGroup) {
                     const int j = S.ids_f ? S.ids_f[tf] : tf;
                     FSIM_DCHECK(j >= 0 && j < S.nf, 256u, continue);
                     const float4 q = S.fposr[j];
@@ -2427,37 +2524,60 @@ __device__ __forceinline__ void solid_force_body(const DevParams &P, const Solid
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
             PLi[k] = S.PL[kPLStride * i + k];
-            AVi[k] = S.AV[9 * i + k];
+            AVi[k] = S.L[9 * (S.n + i) + k];
         }
         const float4 ri = S.ref[i];
         const int o = S.orig[i];
-        for (int e = S.nbr_off[o] + g, ee = S.nbr_off[o + 1]; e < ee; e += kSolidGroup) {
-            const int j = S.nbr_slot[e];
-            if (j < 0) continue;
-            FSIM_DCHECK(j < S.n, 2048u, continue);
-            const float4 rj = S.ref[j];
-            const float dX = __fsub_rn(rj.x, ri.x), dY = __fsub_rn(rj.y, ri.y), dZ = __fsub_rn(rj.z, ri.z);
-            const float w = solid_pair_weight(P, dX, dY, dZ);
-            const float4 *plj = reinterpret_cast<const float4 *>(S.PL + kPLStride * j);
-            const float4 q0 = plj[0], q1 = plj[1], q2 = plj[2];
-            const float PLj[9] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x};
-            const float ws = __fmul_rn(w, P.rho_s_inv);
-            auto row3 = [&](float a0, float a1, float a2) {
-                return fmaf(a2, dZ, fmaf(a1, dY, __fmul_rn(a0, dX)));
-            };
-            ax = fmaf(row3(__fadd_rn(PLj[0], PLi[0]), __fadd_rn(PLj[1], PLi[1]), __fadd_rn(PLj[2], PLi[2])), ws, ax);
-            ay = fmaf(row3(__fadd_rn(PLj[3], PLi[3]), __fadd_rn(PLj[4], PLi[4]), __fadd_rn(PLj[5], PLi[5])), ws, ay);
-            az = fmaf(row3(__fadd_rn(PLj[6], PLi[6]), __fadd_rn(PLj[7], PLi[7]), __fadd_rn(PLj[8], PLi[8])), ws, az);
-            const float4 xj = S.pos[j], vj = S.vel[j];
-            const float ddx = __fsub_rn(xj.x, xi.x), ddy = __fsub_rn(xj.y, xi.y), ddz = __fsub_rn(xj.z, xi.z);
-            const float dvdx = fmaf(__fsub_rn(vj.z, vi.z), ddz,
-                                    fmaf(__fsub_rn(vj.y, vi.y), ddy, __fmul_rn(__fsub_rn(vj.x, vi.x), ddx)));
-            const float nu = __fdiv_rn(__fmul_rn(P.h, dvdx),
-                                       __fadd_rn(fmaf(ddz, ddz, fmaf(ddy, ddy, __fmul_rn(ddx, ddx))), P.eps_h2));
-            const float visc = __fmul_rn(fmaf(__fmul_rn(P.alpha, nu), P.cs_s, -__fmul_rn(__fmul_rn(P.beta, nu), nu)), w);
-            ax = fmaf(row3(AVi[0], AVi[1], AVi[2]), visc, ax);
-            ay = fmaf(row3(AVi[3], AVi[4], AVi[5]), visc, ay);
-            az = fmaf(row3(AVi[6], AVi[7], AVi[8]), visc, az);
+        // kForceAhead entries' loads in flight together, summed in list order
+        for (int e0 = S.nbr_off[o] + g, ee = S.nbr_off[o + 1]; e0 < ee; e0 += kForceAhead * kSolidGroup) {
+            int js[kForceAhead];
+            float4 rj[kForceAhead], q0[kForceAhead], q1[kForceAhead], q2[kForceAhead], xj[kForceAhead],
+                vj[kForceAhead];
+#pragma unroll
+            for (int u = 0; u < kForceAhead; ++u) {
+                const int e = e0 + u * kSolidGroup;
+                js[u] = e < ee ? S.nbr_slot[e] : -1;
+                FSIM_DCHECK(js[u] < S.n, 2048u, js[u] = -1);
+            }
+#pragma unroll
+            for (int u = 0; u < kForceAhead; ++u) {
+                const int j = js[u] < 0 ? i : js[u];
+                rj[u] = S.ref[j];
+                const float4 *plj = reinterpret_cast<const float4 *>(S.PL + kPLStride * j);
+                q0[u] = plj[0];
+                q1[u] = plj[1];
+                q2[u] = plj[2];
+                xj[u] = S.pos[j];
+                vj[u] = S.vel[j];
+            }
+#pragma unroll
+            for (int u = 0; u < kForceAhead; ++u) {
+                const bool in = js[u] >= 0;
+                const float dX = __fsub_rn(rj[u].x, ri.x), dY = __fsub_rn(rj[u].y, ri.y), dZ = __fsub_rn(rj[u].z, ri.z);
+                const float w = solid_pair_weight(P, dX, dY, dZ);
+                const float PLj[9] = {q0[u].x, q0[u].y, q0[u].z, q0[u].w, q1[u].x,
+                                      q1[u].y, q1[u].z, q1[u].w, q2[u].x};
+                const float ws = __fmul_rn(w, P.rho_s_inv);
+                auto row3 = [&](float a0, float a1, float a2) {
+                    return fmaf(a2, dZ, fmaf(a1, dY, __fmul_rn(a0, dX)));
+                };
+                float bx = fmaf(row3(__fadd_rn(PLj[0], PLi[0]), __fadd_rn(PLj[1], PLi[1]), __fadd_rn(PLj[2], PLi[2])), ws, ax);
+                float by = fmaf(row3(__fadd_rn(PLj[3], PLi[3]), __fadd_rn(PLj[4], PLi[4]), __fadd_rn(PLj[5], PLi[5])), ws, ay);
+                float bz = fmaf(row3(__fadd_rn(PLj[6], PLi[6]), __fadd_rn(PLj[7], PLi[7]), __fadd_rn(PLj[8], PLi[8])), ws, az);
+                const float ddx = __fsub_rn(xj[u].x, xi.x), ddy = __fsub_rn(xj[u].y, xi.y),
+                            ddz = __fsub_rn(xj[u].z, xi.z);
+                const float dvdx = fmaf(__fsub_rn(vj[u].z, vi.z), ddz,
+                                        fmaf(__fsub_rn(vj[u].y, vi.y), ddy, __fmul_rn(__fsub_rn(vj[u].x, vi.x), ddx)));
+                const float nu = __fdiv_rn(__fmul_rn(P.h, dvdx),
+                                           __fadd_rn(fmaf(ddz, ddz, fmaf(ddy, ddy, __fmul_rn(ddx, ddx))), P.eps_h2));
+                const float visc = __fmul_rn(fmaf(__fmul_rn(P.alpha, nu), P.cs_s, -__fmul_rn(__fmul_rn(P.beta, nu), nu)), w);
+                bx = fmaf(row3(AVi[0], AVi[1], AVi[2]), visc, bx);
+                by = fmaf(row3(AVi[3], AVi[4], AVi[5]), visc, by);
+                bz = fmaf(row3(AVi[6], AVi[7], AVi[8]), visc, bz);
+                ax = in ? bx : ax;
+                ay = in ? by : ay;
+                az = in ? bz : az;
+            }
         }
     }
     cx = group_sum(cx);
@@ -2468,33 +2588,21 @@ __device__ __forceinline__ void solid_force_body(const DevParams &P, const Solid
     az = group_sum(az);
     if (!valid || g) return;
     S.couple[i] = make_float4(cx, cy, cz, 0.0f);
-    S.dudt[i] = make_float4(__fadd_rn(ax, cx), __fadd_rn(ay, cy), __fadd_rn(az, cz), 0.0f);
+    const float4 a = make_float4(__fadd_rn(ax, cx), __fadd_rn(ay, cy), __fadd_rn(az, cz), 0.0f);
+    S.dudt[i] = a;
+    if (S.pos_out) solid_update_particle(P, S, i, S.pos[i], S.vel[i], a, S.pos_out, S.vel_out);
 }
 FSIM_BATCHED_KERNEL_P(kb_solid_force, SolidArgs, solid_force_body<false>, kBlock)
 FSIM_BATCHED_KERNEL_P(kb_solid_force_record, SolidArgs, (solid_force_body<false, 1>), kBlock)
 FSIM_BATCHED_KERNEL_P(kb_solid_force_listed, SolidArgs, (solid_force_body<false, 2>), kBlock)
 FSIM_BATCHED_KERNEL(kb_solid_force_mixed, SolidArgs, solid_force_body<true>, kBlock)
 
-// solidUpdate (src/solid.cu:209-239)
+// The update as a launch of its own, in place: the first of an odd number of
+// sub-steps, and the fused launch.
 __device__ __forceinline__ void solid_update_body(const DevParams &P, const SolidArgs &S, int blk)
 {
     const int i = blk * blockDim.x + threadIdx.x;
-    if (i >= S.n) return;
-    const int t = S.type[i];
-    if (t == 1) { // FIXED_SOLID
-        float4 v = S.vel[i];
-        S.vel[i] = make_float4(0.0f, 0.0f, 0.0f, v.w);
-        S.dudt[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    } else if (t == 0) { // UNCONSTRAINED_SOLID
-        const float4 x = S.pos[i], v = S.vel[i], a = S.dudt[i];
-        float nx = x.x + v.x * P.dt_sub, ny = x.y + v.y * P.dt_sub, nz = x.z + v.z * P.dt_sub;
-        S.vel[i] = make_float4(v.x + (a.x + P.gx) * P.dt_sub, v.y + (a.y + P.gy) * P.dt_sub,
-                               v.z + (a.z + P.gz) * P.dt_sub, v.w);
-        nx = fminf(fmaxf(nx, P.dmin[0]), P.dmax[0]);
-        ny = fminf(fmaxf(ny, P.dmin[1]), P.dmax[1]);
-        nz = fminf(fmaxf(nz, P.dmin[2]), P.dmax[2]);
-        S.pos[i] = make_float4(nx, ny, nz, x.w);
-    }
+    if (i < S.n) solid_update_particle(P, S, i, S.pos[i], S.vel[i], S.dudt[i], S.pos, S.vel);
 }
 FSIM_BATCHED_KERNEL(kb_solid_update, SolidArgs, solid_update_body, kBlock)
 

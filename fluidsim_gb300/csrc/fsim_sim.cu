@@ -76,7 +76,8 @@ struct fsim_sim {
     int *s_cell = nullptr, *s_key = nullptr, *s_slot = nullptr, *s_tmp = nullptr;
     int *s_cnt = nullptr, *s_start = nullptr;
     float4 *s_np = nullptr, *s_dudt = nullptr, *s_couple = nullptr;
-    float *s_F = nullptr, *s_P = nullptr, *s_L = nullptr, *s_PL = nullptr, *s_AV = nullptr;
+    float *s_F = nullptr, *s_L = nullptr, *s_PL = nullptr; // s_F: F, then P; s_L: L^-1, then cof(F) L^-1
+    float *s_P = nullptr;         // the second half of s_F
     int *s_inv = nullptr;         // sorted position of every input id (written by the gather)
     unsigned *s_cxyz = nullptr;   // packed cell coordinates, sorted order
     int *s_nbr_off = nullptr, *s_nbr_orig = nullptr; // static reference neighbours (CSR, input ids)
@@ -743,15 +744,14 @@ void plan_solid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, in
         SolidArgs S;
         S.pos = h->s_pos[ps];
         S.vel = h->s_vel[ps];
+        S.pos_out = S.vel_out = nullptr;
         S.ref = h->s_ref[ps];
         S.type = h->s_type[ps];
         S.cell = h->s_cell;
         S.np = h->s_np;
         S.F = h->s_F;
-        S.Pk = h->s_P;
         S.L = h->s_L;
         S.PL = h->s_PL;
-        S.AV = h->s_AV;
         S.dudt = h->s_dudt;
         S.couple = h->s_couple;
         S.fposr = h->f_posr[pf];
@@ -779,14 +779,26 @@ void plan_solid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, in
     }
     const bool mixed = !m.empty() && m[0]->mixed;
     if (m.empty() || !m[0]->cfg.solid_fused) {
-        // one batched launch per phase per sub-step; an instance takes part in
-        // the sub-steps it has
+        // two batched launches per sub-step, deformation and force with the
+        // update; an instance takes part in the sub-steps it has.  The update
+        // goes to the solid's other buffer and back (the state before the cell
+        // phase's copy, which nothing reads any more), so that it may share the
+        // force launch; of an odd number of sub-steps the first stays in place
+        // and takes an update launch, so that all end in the same buffer.
         for (int k = 0; k < max_sub; ++k) {
-            std::vector<int> wb, tb;
-            for (fsim_sim *h : m) {
-                const bool active = h->ns && k < h->cfg.solid_sub_step;
+            std::vector<int> wb, ub;
+            for (size_t q = 0; q < m.size(); ++q) {
+                fsim_sim *h = m[q];
+                const int nsub = h->cfg.solid_sub_step, odd = nsub & 1;
+                const bool active = h->ns && k < nsub, in_place = odd && k == 0;
                 wb.push_back(active ? blocks_for((long long)kSolidGroup * h->ns, kBlock) : 0);
-                tb.push_back(active ? blocks_for(h->ns, kBlock) : 0);
+                ub.push_back(active && in_place ? blocks_for(h->ns, kBlock) : 0);
+                const int from = in_place || (k - odd) % 2 == 0 ? ps : 1 - ps;
+                SolidArgs &S = it[q].A;
+                S.pos = h->s_pos[from];
+                S.vel = h->s_vel[from];
+                S.pos_out = in_place ? nullptr : h->s_pos[1 - from];
+                S.vel_out = in_place ? nullptr : h->s_vel[1 - from];
             }
             // sub-step 0 also resolves the step's list slots for the later sub-steps
             add_launch(pl, ab, mixed ? (k == 0 ? L_DEFORM_M_R : L_DEFORM_M) : (k == 0 ? L_DEFORM_R : L_DEFORM), it,
@@ -795,7 +807,7 @@ void plan_solid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, in
             const bool lists = !mixed && !m[0]->cfg.solid_full_walk;
             add_launch(pl, ab, mixed ? L_FORCE_M : !lists ? L_FORCE : k == 0 ? L_FORCE_RECORD : L_FORCE_LISTED, it,
                        wb);
-            add_launch(pl, ab, L_UPDATE, it, tb);
+            add_launch(pl, ab, L_UPDATE, it, ub);
         }
         return;
     }
@@ -1246,13 +1258,14 @@ fsim_status alloc_state(fsim_sim *h)
     if ((st = dalloc(h, &h->s_cell, ns)) || (st = dalloc(h, &h->s_key, ns)) || (st = dalloc(h, &h->s_slot, ns)) ||
         (st = dalloc(h, &h->s_tmp, ns)) || (st = dalloc(h, &h->s_cnt, nc)) || (st = dalloc(h, &h->s_start, nc + 1)) ||
         (st = dalloc(h, &h->s_np, ns)) || (st = dalloc(h, &h->s_dudt, ns)) || (st = dalloc(h, &h->s_couple, ns)) ||
-        (st = dalloc(h, &h->s_F, 9 * (size_t)ns)) || (st = dalloc(h, &h->s_P, 9 * (size_t)ns)) ||
-        (st = dalloc(h, &h->s_L, 9 * (size_t)ns)) || (st = dalloc(h, &h->s_PL, (size_t)kPLStride * ns)) ||
-        (st = dalloc(h, &h->s_AV, 9 * (size_t)ns)) || (st = dalloc(h, &h->s_inv, ns)) ||
+        (st = dalloc(h, &h->s_F, 18 * (size_t)ns)) || (st = dalloc(h, &h->s_L, 18 * (size_t)ns)) ||
+        (st = dalloc(h, &h->s_PL, (size_t)kPLStride * ns)) ||
+        (st = dalloc(h, &h->s_inv, ns)) ||
         (st = dalloc(h, &h->s_cxyz, ns)) ||
         (st = dalloc(h, &h->s_fl, (size_t)kFluidListCap * kSolidGroup * ns)) ||
         (st = dalloc(h, &h->s_fl_cnt, (size_t)kSolidGroup * ns)) || (st = dalloc(h, &h->s_fl_org, ns)))
         return st;
+    h->s_P = h->s_F + 9 * (size_t)ns;
     // virtual
     if ((st = dalloc(h, &h->v_posr, nv)) || (st = dalloc(h, &h->v_velp, nv)) || (st = dalloc(h, &h->v_normal, nv)) ||
         (st = dalloc(h, &h->v_orig, nv)) || (st = dalloc(h, &h->v_cell, nv)) ||

@@ -298,11 +298,12 @@ struct CellRefArgs {
 // solid sub-step kernels (deformation, force, update, fused)
 struct SolidArgs {
     float4 *pos, *vel;
+    float4 *pos_out, *vel_out; // where the force sweep advances the solid to (nullptr: kb_solid_update does, in place)
     const float4 *ref;
     const int *type, *cell;
     const int *ids_f;      // per-step fluid cell index of a neighbour-list instance (else nullptr)
     const float4 *np;
-    float *F, *Pk, *L, *AV; // 9 floats per particle, row-major
+    float *F, *L;           // 9 floats per particle, row-major: F then P; L^-1 then cof(F) L^-1
     float *PL;              // kPLStride floats per particle (9 used): three 16-byte loads per neighbour
     float4 *dudt, *couple;
     const float4 *fposr, *fvelp;
