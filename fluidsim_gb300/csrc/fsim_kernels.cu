@@ -143,19 +143,6 @@ struct RowRanges {
     }
 };
 
-// f(c0, c1) for the cell rows [c0, c1) within `reach` cells of cell c on each axis.
-template <class F>
-__device__ __forceinline__ void for_rows_within(const DevParams &P, int c, int reach, F &&f)
-{
-    const int row = c / P.nz, cz = c - row * P.nz, cx = row / P.ny, cy = row - cx * P.ny;
-    const int z0 = max(cz - reach, 0), z1 = min(cz + reach, P.nz - 1) + 1;
-    for (int x = max(cx - reach, 0); x <= min(cx + reach, P.nx - 1); ++x)
-        for (int y = max(cy - reach, 0); y <= min(cy + reach, P.ny - 1); ++y) {
-            const int base = (x * P.ny + y) * P.nz;
-            f(base + z0, base + z1);
-        }
-}
-
 // ------------------------------------------------------- batched launches
 // Every step kernel has a body taking (params, args, local block index) and a
 // batched wrapper: one launch serves many instances, each with its own
@@ -537,7 +524,13 @@ __device__ __forceinline__ float rcp_approx(float x)
 // The terms of one pair: drho += x w, a += f (dx, dy, dz).
 // EXACT (mixed form): every rounding spelled out (no contraction freedom left to
 // the compiler), so that every kernel inlining this rounds identically.
-template <bool LIMITER, int VISCID, bool EXACT = false>
+// SPELLED: the one contraction of the plain terms that came out differently in
+// different kernels (either product of P* may be the one left unrounded, and for a
+// solid neighbour, whose density is the particle's own, both are alike to the
+// compiler): fixed for the one-instance list sweep.  The batched forms keep their
+// own, so a batch member that touches a solid can differ from its standalone run
+// in the last bit.
+template <bool LIMITER, int VISCID, bool EXACT = false, bool SPELLED = false>
 __device__ __forceinline__ void riemann_terms(const DevParams &P, float dx, float dy, float dz, float r2, float uix,
                                               float uiy, float uiz, float rhoi, float pi, float ujx, float ujy,
                                               float ujz, float rhoj, float pj, bool clamp_ps, float &x, float &w,
@@ -567,7 +560,7 @@ __device__ __forceinline__ void riemann_terms(const DevParams &P, float dx, floa
     const float a = (uix - ujx) * dx + (uiy - ujy) * dy + (uiz - ujz) * dz;
     const float du = fmaxf(a * inv_r, 0.0f); // only du >= 0 adds dissipation
     const float lim = LIMITER ? fminf(3.0f * du, P.c0) : P.c0;
-    float ps = (rhoi * pj + rhoj * pi) * rs_inv;
+    float ps = (SPELLED ? __fmaf_rn(rhoj, pi, __fmul_rn(rhoi, pj)) : rhoi * pj + rhoj * pi) * rs_inv;
     ps = fmaf(rhoi * rhoj * rs_inv * du, lim, ps);
     if (clamp_ps) ps = fmaxf(ps, 0.0f);
     const float r = r2 * inv_r;
@@ -914,16 +907,20 @@ __global__ void __launch_bounds__(kBlock) kb_nl_decide(const Item<NlDecideArgs> 
     }
 }
 
-// The list build, one lane per particle: the list grid's cells are a fraction
-// 1 / reach of the list radius, so the candidates of a particle are the cells
-// within `reach` of its own -- (2 reach + 1)^2 rows (x, y), each one z-contiguous
-// index range.  Particles are sorted on that grid, so a column of cells holds
-// its particles in z order and a warp's lanes are (nearly) consecutive in it:
-// their candidate loads are shifted copies of one another and coalesce.  Hits
-// (r^2 < Rs^2) collect in a two-group ring per lane in shared memory and leave
-// in whole groups.  Per particle: its fluid, then wall, then solid candidates,
-// in row order.
-constexpr int kNlBuildWarps = kNlBuildThreads / 32, kNlBuildRing = 2 * kNlGroup;
+// The list build, one lane per particle: the candidates of its 27 cells of the
+// list grid, a chunk at a time -- all loads first, then one bit per hit
+// (r^2 < Rs^2), then the hits in candidate order into a ring per lane in shared
+// memory, which leaves in whole groups.  Bound by issue: about 730 candidates a
+// particle for ~93 entries, so a candidate costs its test (8 instructions) and a
+// predicated OR, and only the hits the append.  (The lanes of a warp mostly
+// share a cell, so a candidate load is a broadcast.)  Per particle: its fluid,
+// then wall, then solid candidates, in row order -- the order in which the
+// stream sweep sums them -- each species from a whole group on.  Measured, a step
+// with a build above one without: 4.7 ms with the warp-uniform stream of the cell
+// walk (32 instructions a candidate), 3.6 ms so, at 4.2 M particles; 1.1 and 0.88
+// at 1 M.  Cells of a third of the radius test 310 candidates but reorder the
+// particles, which gained the plain sweep 4 % and cost the mixed one 11 %.
+constexpr int kNlBuildWarps = kNlBuildThreads / 32, kNlBuildRing = 4 * kNlGroup;
 
 // Store group `grp` of the lane's list from the ring (entries past `tot` as -1):
 // two 16-byte stores, a full sector.
@@ -941,45 +938,54 @@ __device__ __forceinline__ void nl_store_group(const NlBuildArgs &A, int (*ring)
     __stcs(dst + 1, make_int4(v[4], v[5], v[6], v[7]));
 }
 
+// Test candidates j .. j + C of a row ending at je (C at most 16; the position
+// arrays are kNlReadAhead entries longer than their counts) and append the hits.
+template <int C>
+__device__ __forceinline__ void nl_chunk(const NlBuildArgs &A, const float4 *__restrict__ pos, int (*ring)[32], int lane,
+                                         int i, int &tot, int j, int je, float4 pr)
+{
+    static_assert(C <= kNlReadAhead && C + kNlGroup <= kNlBuildRing, "chunk");
+    unsigned bits = 0;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        const float4 q = pos[j + c];
+        if (dist2(q.x - pr.x, q.y - pr.y, q.z - pr.z) < A.R2s) bits |= 1u << c;
+    }
+    if (je - j < C) bits &= (1u << (je - j)) - 1u;
+    const int grp = tot / kNlGroup;
+    while (bits) {
+        const int c = __ffs(bits) - 1;
+        bits &= bits - 1;
+        ring[tot++ & (kNlBuildRing - 1)][lane] = j + c;
+    }
+    for (int g = grp; g < tot / kNlGroup; ++g) nl_store_group(A, ring, lane, i, g, tot);
+}
+
 template <int SP>
 __device__ __forceinline__ void nl_gather(const DevParams &P, const NlBuildArgs &A, int (*ring)[32], int lane, int i,
                                           bool valid, int &tot, int cx, int cy, int cz, float4 pr)
 {
     const int *__restrict__ start = SP == 0 ? A.start_f : SP == 1 ? A.start_v : A.start_s;
     const float4 *__restrict__ pos = SP == 0 ? A.posr : SP == 1 ? A.v_posr : A.s_pos;
-    const int K = A.reach;
-#pragma unroll 1
-    for (int ox = -K; ox <= K; ++ox) {
-        const int x = cx + ox, mx = max(abs(ox) - 1, 0);
-        const bool inx = valid && x >= 0 && x < P.nx;
-#pragma unroll 1
-        for (int oy = -K; oy <= K; ++oy) {
-            const int y = cy + oy, my = max(abs(oy) - 1, 0);
-            int zr = K; // cells of this row that can hold a point within reach
-            while ((zr - 1) * (zr - 1) + mx * mx + my * my >= K * K) --zr;
-            int j = 0, je = 0;
-            if (inx && y >= 0 && y < P.ny) {
-                const int base = (x * P.ny + y) * P.nz;
-                j = start[base + max(cz - zr, 0)];
-                je = start[base + min(cz + zr, P.nz - 1) + 1];
-            }
-            for (; j < je; j += kNlGroup) {
-                const int grp = tot / kNlGroup;
-#pragma unroll
-                for (int c = 0; c < kNlGroup; ++c) {
-                    if (j + c < je) {
-                        FSIM_DCHECK(j + c < (SP == 0 ? A.n : SP == 1 ? A.nv : A.ns), 2u, continue);
-                        const float4 q = pos[j + c];
-                        const float r2 = dist2(q.x - pr.x, q.y - pr.y, q.z - pr.z);
-                        if (r2 < A.R2s) {
-                            ring[tot & (kNlBuildRing - 1)][lane] = j + c;
-                            ++tot;
-                        }
-                    }
-                }
-                if (tot / kNlGroup != grp) nl_store_group(A, ring, lane, i, grp, tot);
-            }
+    const int z0 = max(cz - 1, 0), z1 = min(cz + 1, P.nz - 1) + 1;
+    // row r's range, read one row ahead
+    auto range = [&](int r, int &b, int &e) {
+        const int x = cx + r / 3 - 1, y = cy + r % 3 - 1;
+        b = e = 0;
+        if (valid && r < 9 && x >= 0 && x < P.nx && y >= 0 && y < P.ny) {
+            b = start[(x * P.ny + y) * P.nz + z0];
+            e = start[(x * P.ny + y) * P.nz + z1];
         }
+    };
+    int b, e;
+    range(0, b, e);
+#pragma unroll 1
+    for (int r = 0; r < 9; ++r) {
+        int j = b;
+        const int je = e;
+        range(r + 1, b, e);
+        for (; je - j > 8; j += 16) nl_chunk<16>(A, pos, ring, lane, i, tot, j, je, pr);
+        if (j < je) nl_chunk<8>(A, pos, ring, lane, i, tot, j, je, pr);
     }
 }
 
@@ -1028,11 +1034,12 @@ FSIM_REBUILD_KERNEL(kg_nl_build, NlBuildArgs, nl_build_body, kNlBuildWarps * 32,
 // entries, as the stream sweep sums them), r^2 < R^2, the Riemann pair terms, then
 // fluidUpdate (src/fluid.cu:234-269) as in the stream sweep; the particle's
 // squared displacement since the build goes into the instance's running maximum.
-// With one lane per particle it is bound by the L1's wavefronts (a scattered
-// 32-byte record per entry: 21 wavefronts per warp and entry of a possible 8)
-// and by issue.  Measured, 4.2 M / 1 M / 32 k particles: 1.16 / 0.31 / 0.060 ms
-// with a test and branch per entry, 1.05 / 0.27 / 0.029 ms branch-free with the
-// next group prefetched and (above 262,144 particles) lists of the fine grid.
+// With one lane per particle the plain form is bound by the L1's wavefronts (a
+// scattered 32-byte record per entry, 21-28 wavefronts per warp and entry of a
+// possible 8) and the mixed form by issue (110 instructions an entry).  Measured,
+// 4.2 M / 1 M / 32 k particles: plain 1.16 / 0.31 / 0.060 ms with a test and branch
+// per entry, 1.08 / 0.28 / 0.028 ms branch-free with the next group prefetched;
+// mixed 1.59 -> 1.38 ms at 4.2 M.
 // One 32-byte (position, velocity) record with a single 256-bit load through
 // the read-only path (32-byte aligned: records start on 256-byte allocations).
 __device__ __forceinline__ void load_record(const float4 *p, float4 &a, float4 &b)
@@ -1081,20 +1088,21 @@ struct ListSum {
                     : "r"((int)p.in), "f"(p.x), "f"(p.w));
             return;
         }
-        // a term out of range is stored as 0 x 0
+        // a term out of range is stored as 0 x 0 (its weight as -1 where the
+        // compensated sum must pass over it: adding 0 would fold in the compensation)
         __syncwarp();
         sh[0][lane] = p.in ? p.f : 0.0f;
         sh[1][lane] = p.in ? p.x : 0.0f;
         sh[2][lane] = p.in ? p.dx : 0.0f;
         sh[3][lane] = p.in ? p.dy : 0.0f;
         sh[4][lane] = p.in ? p.dz : 0.0f;
-        sh[5][lane] = p.in ? p.w : 0.0f;
+        sh[5][lane] = p.in ? p.w : KAHAN ? -1.0f : 0.0f;
         __syncwarp();
         if (g < 4) {
             const float *l = &sh[g == 3 ? 1 : 0][lane - g], *r = &sh[2 + g][lane - g];
 #pragma unroll 4
             for (int k = 0; k < G; ++k) {
-                if (KAHAN && g == 3) kahan_add(l[k], r[k], true, acc.ax, acc.drho_c);
+                if (KAHAN && g == 3) kahan_add(l[k], r[k], r[k] >= 0.0f, acc.ax, acc.drho_c);
                 else acc.ax = __fmaf_rn(l[k], r[k], acc.ax);
             }
         }
@@ -1145,7 +1153,9 @@ __device__ __forceinline__ void walk_list(const FluidSweepArgs &A, int i, bool v
 #pragma unroll
             for (int q = 0; q < kNlGroup; ++q) {
                 FSIM_DCHECK(e[q] >= 0 && e[q] < A.n, 1u, continue);
-                sum.add(fluid(e[q]));
+                ListPair p = fluid(e[q]);
+                if (KAHAN) p.in = p.in && k * kNlGroup + q < cnt.x; // not the last group's filling
+                sum.add(p);
             }
         }
         for (int k = 0; k < nv; ++k) {
@@ -1176,7 +1186,7 @@ __device__ __forceinline__ void walk_list(const FluidSweepArgs &A, int i, bool v
 }
 
 // Particle i's pairs in the plain form.
-template <int VISCID, bool CHECK, bool LANES>
+template <int VISCID, bool CHECK, bool LANES, bool ONE>
 __device__ __forceinline__ void fluid_sweep_nl_pairs(const DevParams &P, const FluidSweepArgs &A, int i, bool valid,
                                                      float4 pr, float4 vp, ListSum<LANES, false> &sum)
 {
@@ -1214,8 +1224,9 @@ __device__ __forceinline__ void fluid_sweep_nl_pairs(const DevParams &P, const F
             const float r2 = rel(q, p);
             p.in = r2 < P.R2 && (!CHECK || cells_adjacent(ci, A.nl_cxyz_s[j]));
             const float k2 = 2.0f * ((vp.x - sv.x) * np.x + (vp.y - sv.y) * np.y + (vp.z - sv.z) * np.z);
-            riemann_terms<false, VISCID>(P, p.dx, p.dy, p.dz, r2, vp.x, vp.y, vp.z, pr.w, vp.w, vp.x - k2 * np.x,
-                                         vp.y - k2 * np.y, vp.z - k2 * np.z, pr.w, np.w, false, p.x, p.w, p.f);
+            riemann_terms<false, VISCID, false, ONE>(P, p.dx, p.dy, p.dz, r2, vp.x, vp.y, vp.z, pr.w, vp.w, vp.x - k2 * np.x,
+                                                     vp.y - k2 * np.y, vp.z - k2 * np.z, pr.w, np.w, false, p.x, p.w,
+                                                     p.f);
             return p;
         });
 }
@@ -1227,7 +1238,7 @@ __device__ __forceinline__ float (*lane_terms())[32]
     return sweep_terms + kSweepTermRows * (threadIdx.x >> 5);
 }
 
-template <int VISCID, bool LANES>
+template <int VISCID, bool LANES, bool ONE>
 __device__ __forceinline__ void fluid_sweep_nl_lanes(const DevParams &P, const FluidSweepArgs &A, int blk)
 {
     const int t = blk * blockDim.x + threadIdx.x, sh = LANES ? A.lane_shift : 0, i = t >> sh;
@@ -1243,8 +1254,8 @@ __device__ __forceinline__ void fluid_sweep_nl_lanes(const DevParams &P, const F
         pr = A.posr[i];
         vp = A.velp[i];
     }
-    if (A.nl_cxyz_f) fluid_sweep_nl_pairs<VISCID, true, LANES>(P, A, i, valid, pr, vp, sum);
-    else fluid_sweep_nl_pairs<VISCID, false, LANES>(P, A, i, valid, pr, vp, sum);
+    if (A.nl_cxyz_f) fluid_sweep_nl_pairs<VISCID, true, LANES, ONE>(P, A, i, valid, pr, vp, sum);
+    else fluid_sweep_nl_pairs<VISCID, false, LANES, ONE>(P, A, i, valid, pr, vp, sum);
     const PairAcc acc = sum.total();
     unsigned d2bits = 0u;
     if (valid && sum.g == 0) {
@@ -1255,11 +1266,11 @@ __device__ __forceinline__ void fluid_sweep_nl_lanes(const DevParams &P, const F
     const unsigned wmax = __reduce_max_sync(kFull, d2bits);
     if ((threadIdx.x & 31) == 0 && wmax) atomicMax(&A.nl->maxd2, wmax);
 }
-template <int VISCID>
+template <int VISCID, bool ONE = false>
 __device__ __forceinline__ void fluid_sweep_nl_body(const DevParams &P, const FluidSweepArgs &A, int blk)
 {
-    if (A.lane_shift) fluid_sweep_nl_lanes<VISCID, true>(P, A, blk); // uniform over the launch
-    else fluid_sweep_nl_lanes<VISCID, false>(P, A, blk);
+    if (A.lane_shift) fluid_sweep_nl_lanes<VISCID, true, ONE>(P, A, blk); // uniform over the launch
+    else fluid_sweep_nl_lanes<VISCID, false, ONE>(P, A, blk);
 }
 
 // launch shapes of the list sweep: threads per block, minimum blocks per SM
@@ -1278,7 +1289,7 @@ template <int VISCID, class SH>
 __global__ void __launch_bounds__(SH::threads, SH::min_blocks) kb_fluid_sweep_nl_1(const DevParams P,
                                                                                    const FluidSweepArgs A)
 {
-    fluid_sweep_nl_body<VISCID>(P, A, (int)blockIdx.x);
+    fluid_sweep_nl_body<VISCID, true>(P, A, (int)blockIdx.x);
 }
 template <int VISCID, class SH>
 __global__ void __launch_bounds__(SH::threads, SH::min_blocks)
@@ -1374,14 +1385,16 @@ FSIM_BATCHED_KERNEL(kb_virt, VirtArgs, virt_body, kBlock)
 // gradient sum over the other virtual particles, normalised, zero when its
 // squared length is below EPS_FOR_SUM.  Walls never move: computed once.
 __global__ void k_virt_normal(const DevParams P, const float4 *__restrict__ v_posr, const int *__restrict__ v_cell,
-                              const int *__restrict__ start_v, float4 *__restrict__ v_normal, int n, int reach)
+                              const int *__restrict__ start_v, float4 *__restrict__ v_normal, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 xi = v_posr[i];
+    Rows rows;
+    neighbor_rows(P, v_cell[i], rows);
     float nx = 0.0f, ny = 0.0f, nz = 0.0f;
-    for_rows_within(P, v_cell[i], reach, [&](int c0, int c1) {
-        for (int j = start_v[c0], je = start_v[c1]; j < je; ++j) {
+    for (int r = 0; r < rows.count; ++r) {
+        for (int j = start_v[rows.base[r] + rows.z0], je = start_v[rows.base[r] + rows.z1]; j < je; ++j) {
             if (j == i) continue;
             const float4 q = v_posr[j];
             const float dx = q.x - xi.x, dy = q.y - xi.y, dz = q.z - xi.z;
@@ -1393,7 +1406,7 @@ __global__ void k_virt_normal(const DevParams P, const float4 *__restrict__ v_po
                 nz -= dz * w;
             }
         }
-    });
+    }
     const float l2 = nx * nx + ny * ny + nz * nz;
     if (l2 < FSIM_EPS_FOR_SUM) {
         nx = ny = nz = 0.0f;
@@ -2092,13 +2105,14 @@ struct RowMixed {
     int b1, b2, z0;  // start of the row's 2nd and 3rd cell, first cell
     float sx, sy;    // solid offset minus the row's x/y cell shift
 };
-__device__ __forceinline__ void fluid_rel(const DevParams &P, const RowMixed &R, int t, float sz0, float4 q, float &dx,
-                                          float &dy, float &dz)
+__device__ __forceinline__ int fluid_rel(const DevParams &P, const RowMixed &R, int t, float sz0, float4 q, float &dx,
+                                         float &dy, float &dz)
 {
     const int k = (t >= R.b1) + (t >= R.b2);
     dx = q.x - R.sx;
     dy = q.y - R.sy;
     dz = q.z - fmaf(-(float)k, P.cdx[2], sz0);
+    return k;
 }
 
 // A candidate's particle id, read from the cell index only when asked for (a
@@ -2106,6 +2120,7 @@ __device__ __forceinline__ void fluid_rel(const DevParams &P, const RowMixed &R,
 struct SlotId {
     const int *ids;
     int t;
+    unsigned code; // the candidate's row and z cell: x + 1 | (y + 1) << 2 | cell of the row << 4
     __device__ __forceinline__ operator int() const { return ids ? ids[t] : t; }
 };
 
@@ -2136,8 +2151,8 @@ __device__ __forceinline__ void solid_fluid_walk_m(const DevParams &P, const int
         for (int t = W.b[r] + g; t < W.e[r]; t += G) {
             const float4 q = fpos_t ? fpos_t[t] : fposr[ids ? ids[t] : t];
             float dx, dy, dz;
-            fluid_rel(P, R, t, sz0, q, dx, dy, dz);
-            f(SlotId{ids, t}, dx, dy, dz);
+            const int k = fluid_rel(P, R, t, sz0, q, dx, dy, dz);
+            f(SlotId{ids, t, (unsigned)(r / 3 | (r % 3) << 2 | k << 4)}, dx, dy, dz);
         }
     }
 }
@@ -2425,7 +2440,7 @@ constexpr int kForceAhead = 2; // list entries a lane of the force sweep loads a
 // viscosity over the reference-configuration solid neighbours.
 // MIXED: fluid positions are cell offsets, fluid (rho, p) come from delta.
 //
-// Fluid lists (plain form, FLIST): the fluid does not move during a step's
+// Fluid lists (FLIST): the fluid does not move during a step's
 // sub-steps and the candidates come from the step's cells, so sub-step 0
 // (FLIST 1) walks the 27 cells and records, per lane, the candidates within
 // (R + d)(1 + 1e-5) of the particle; later sub-steps (FLIST 2) walk only that
@@ -2462,10 +2477,61 @@ __device__ __forceinline__ void solid_force_body(const DevParams &P, const Solid
             cy = fmaf(f, dy, cy);
             cz = fmaf(f, dz, cz);
         };
-        if (MIXED) {
+        const int T = kSolidGroup * S.n; // stride of the entry-major lane lists
+        bool walk = true;
+        if (FLIST == 2) {
+            const float4 o = S.fl_org[i];
+            const int c = S.fl_cnt[t];
+            if (c >= 0 && dist2(xi.x - o.x, xi.y - o.y, xi.z - o.z) < P.fl_move2) {
+                walk = false;
+                if (MIXED) {
+                    // a candidate's relative position from its code, as the walk forms it
+                    int cx_, cy_, cz_;
+                    cell_xyz(P, S.cell[i], cx_, cy_, cz_);
+                    const float sox = xi.x - fmaf((float)cx_, P.cdx[0], P.cmin[0]);
+                    const float soy = xi.y - fmaf((float)cy_, P.cdx[1], P.cmin[1]);
+                    const float soz = xi.z - fmaf((float)cz_, P.cdx[2], P.cmin[2]);
+                    const float sz0 = fmaf(-(float)(max(cz_ - 1, 0) - cz_), P.cdx[2], soz);
+                    for (int e = 0; e < c; ++e) {
+                        const unsigned v = (unsigned)S.fl[(size_t)e * T + t];
+                        const int j = (int)(v & kIndexMask), code = (int)(v >> kCodeShift);
+                        FSIM_DCHECK(j < S.nf, 1024u, continue);
+                        const float4 q = S.fposr[j];
+                        const float dx = q.x - fmaf(-(float)((code & 3) - 1), P.cdx[0], sox);
+                        const float dy = q.y - fmaf(-(float)((code >> 2 & 3) - 1), P.cdx[1], soy);
+                        const float dz = q.z - fmaf(-(float)(code >> 4), P.cdx[2], sz0);
+                        const float r2 = dist2(dx, dy, dz);
+                        if (r2 < P.R2) {
+                            const float4 u = S.fvelp[j];
+                            traction(dx, dy, dz, r2, u, fmaf(P.rho0, u.w, P.rho0), eos_delta(P, u.w));
+                        }
+                    }
+                } else {
+                    for (int e = 0; e < c; ++e) {
+                        const int j = S.fl[(size_t)e * T + t];
+                        FSIM_DCHECK(j >= 0 && j < S.nf, 1024u, continue);
+                        const float4 q = S.fposr[j];
+                        const float dx = q.x - xi.x, dy = q.y - xi.y, dz = q.z - xi.z;
+                        const float r2 = dist2(dx, dy, dz);
+                        if (r2 < P.R2) {
+                            const float4 u = S.fvelp[j];
+                            traction(dx, dy, dz, r2, u, q.w, u.w);
+                        }
+                    }
+                }
+            }
+        }
+        int nrec = 0;
+        if (MIXED && walk) {
             solid_fluid_walk_m<kSolidGroup>(P, S.start_f, S.ids_f, S.fposr, S.cell[i], xi, g,
                                             [&](SlotId s, float dx, float dy, float dz) {
                                                 const float r2 = dist2(dx, dy, dz);
+                                                if (FLIST == 1 && r2 < P.fl_build2) {
+                                                    if (nrec < kFluidListCap)
+                                                        S.fl[(size_t)nrec * T + t] = (int)((unsigned)(int)s |
+                                                                                           s.code << kCodeShift);
+                                                    ++nrec;
+                                                }
                                                 if (r2 < P.R2) {
                                                     const float4 u = S.fvelp[(int)s];
                                                     traction(dx, dy, dz, r2, u, fmaf(P.rho0, u.w, P.rho0),
@@ -2473,29 +2539,8 @@ __device__ __forceinline__ void solid_force_body(const DevParams &P, const Solid
                                                 }
                                             });
         }
-        bool walk = !MIXED;
-        const int T = kSolidGroup * S.n; // stride of the entry-major lane lists
-        if (!MIXED && FLIST == 2) {
-            const float4 o = S.fl_org[i];
-            const int c = S.fl_cnt[t];
-            if (c >= 0 && dist2(xi.x - o.x, xi.y - o.y, xi.z - o.z) < P.fl_move2) {
-                walk = false;
-                for (int e = 0; e < c; ++e) {
-                    const int j = S.fl[(size_t)e * T + t];
-                    FSIM_DCHECK(j >= 0 && j < S.nf, 1024u, continue);
-                    const float4 q = S.fposr[j];
-                    const float dx = q.x - xi.x, dy = q.y - xi.y, dz = q.z - xi.z;
-                    const float r2 = dist2(dx, dy, dz);
-                    if (r2 < P.R2) {
-                        const float4 u = S.fvelp[j];
-                        traction(dx, dy, dz, r2, u, q.w, u.w);
-                    }
-                }
-            }
-        }
-        if (walk) {
+        if (!MIXED && walk) {
             const RowRanges<> W(P, S.cell[i], S.start_f);
-            int nrec = 0;
 #pragma unroll
             for (int r = 0; r < 9; ++r) {
                 for (int tf = W.b[r] + g; tf < W.e[r]; tf += kSolidGroup) {
@@ -2514,10 +2559,10 @@ __device__ __forceinline__ void solid_force_body(const DevParams &P, const Solid
                     }
                 }
             }
-            if (FLIST == 1) {
-                S.fl_cnt[t] = nrec <= kFluidListCap ? nrec : -1;
-                if (g == 0) S.fl_org[i] = xi;
-            }
+        }
+        if (FLIST == 1) {
+            S.fl_cnt[t] = nrec <= kFluidListCap ? nrec : -1;
+            if (g == 0) S.fl_org[i] = xi;
         }
         // solidSolidForce (src/solid.cu:119-157)
         float PLi[9], AVi[9];
@@ -2596,6 +2641,8 @@ FSIM_BATCHED_KERNEL_P(kb_solid_force, SolidArgs, solid_force_body<false>, kBlock
 FSIM_BATCHED_KERNEL_P(kb_solid_force_record, SolidArgs, (solid_force_body<false, 1>), kBlock)
 FSIM_BATCHED_KERNEL_P(kb_solid_force_listed, SolidArgs, (solid_force_body<false, 2>), kBlock)
 FSIM_BATCHED_KERNEL(kb_solid_force_mixed, SolidArgs, solid_force_body<true>, kBlock)
+FSIM_BATCHED_KERNEL(kb_solid_force_mixed_record, SolidArgs, (solid_force_body<true, 1>), kBlock)
+FSIM_BATCHED_KERNEL(kb_solid_force_mixed_listed, SolidArgs, (solid_force_body<true, 2>), kBlock)
 
 // The update as a launch of its own, in place: the first of an odd number of
 // sub-steps, and the fused launch.
@@ -2860,7 +2907,7 @@ __global__ void k_neighbor_counts(const DevParams P, const DevParams Pv, const f
                                   const int *__restrict__ cell_f, const int *__restrict__ start_f,
                                   const int *__restrict__ ids_f, const float4 *__restrict__ s_pos,
                                   const int *__restrict__ start_s, const int *__restrict__ ids_s,
-                                  const float4 *__restrict__ v_posr, const int *__restrict__ start_v, int reach_v,
+                                  const float4 *__restrict__ v_posr, const int *__restrict__ start_v,
                                   int *__restrict__ out, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2880,12 +2927,15 @@ __global__ void k_neighbor_counts(const DevParams P, const DevParams Pv, const f
             cs += dist2(q.x - p.x, q.y - p.y, q.z - p.z) < P.R2;
         }
     }
-    for_rows_within(Pv, ids_f ? cell_index(Pv, p.x, p.y, p.z, nullptr) : cell_f[i], reach_v, [&](int c0, int c1) {
+    Rows vrows;
+    neighbor_rows(Pv, ids_f ? cell_index(Pv, p.x, p.y, p.z, nullptr) : cell_f[i], vrows);
+    for (int r = 0; r < vrows.count; ++r) {
+        const int c0 = vrows.base[r] + vrows.z0, c1 = vrows.base[r] + vrows.z1;
         for (int j = start_v[c0]; j < start_v[c1]; ++j) {
             const float4 q = v_posr[j];
             cv += dist2(q.x - p.x, q.y - p.y, q.z - p.z) < P.R2;
         }
-    });
+    }
     out[3 * i] = cf;
     out[3 * i + 1] = cs;
     out[3 * i + 2] = cv;
@@ -2934,8 +2984,7 @@ __global__ void k_neighbor_counts_mixed(const DevParams P, const DevParams Pv, c
                                         const int *__restrict__ ids_f, const float4 *__restrict__ s_pos,
                                         const int *__restrict__ start_s, const int *__restrict__ ids_s,
                                         const float4 *__restrict__ v_posr, const int *__restrict__ start_v,
-                                        const unsigned *__restrict__ v_cxyz, int reach_v, int *__restrict__ out,
-                                        int n)
+                                        const unsigned *__restrict__ v_cxyz, int *__restrict__ out, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -2968,7 +3017,10 @@ __global__ void k_neighbor_counts_mixed(const DevParams P, const DevParams Pv, c
                     }
             }
     if (v_cxyz) {
-        for_rows_within(Pv, cell_index(Pv, pa.x, pa.y, pa.z, nullptr), reach_v, [&](int c0, int c1) {
+        Rows vrows;
+        neighbor_rows(Pv, cell_index(Pv, pa.x, pa.y, pa.z, nullptr), vrows);
+        for (int r = 0; r < vrows.count; ++r) {
+            const int c0 = vrows.base[r] + vrows.z0, c1 = vrows.base[r] + vrows.z1;
             for (int j = start_v[c0]; j < start_v[c1]; ++j) {
                 int jx, jy, jz;
                 unpack_cell(v_cxyz[j], jx, jy, jz);
@@ -2978,7 +3030,7 @@ __global__ void k_neighbor_counts_mixed(const DevParams P, const DevParams Pv, c
                 cv += dist2(q.x - shifted(obx, ox, P.cdx[0]), q.y - shifted(oby, oy, P.cdx[1]),
                             q.z - shifted(obz, oz, P.cdx[2])) < P.R2;
             }
-        });
+        }
     }
     out[3 * i] = cf;
     out[3 * i + 1] = cs;
@@ -3476,6 +3528,8 @@ fsim_status enqueue_plan(const Plan &pl, cudaStream_t st, int shape_arg, cudaEve
         case L_VIRT_M: FSIM_LAUNCH(kb_virt_mixed, VirtArgs, kBlock); break;
         case L_DEFORM_M: FSIM_LAUNCH(kb_solid_deform_mixed, SolidArgs, kBlock); break;
         case L_FORCE_M: FSIM_LAUNCH(kb_solid_force_mixed, SolidArgs, kBlock); break;
+        case L_FORCE_M_RECORD: FSIM_LAUNCH(kb_solid_force_mixed_record, SolidArgs, kBlock); break;
+        case L_FORCE_M_LISTED: FSIM_LAUNCH(kb_solid_force_mixed_listed, SolidArgs, kBlock); break;
         case L_SOLID_FUSED: {
             SolidFusedArgs F;
             F.bstart_w = tb;
@@ -3517,6 +3571,7 @@ int launch_phase(int kind)
     case L_SWEEP: return FSIM_PHASE_FLUID;
     case L_DEFORM: case L_FORCE: case L_UPDATE: case L_DEFORM_M: case L_FORCE_M: case L_SOLID_FUSED:
     case L_SOLID_SLOTS: case L_FORCE_RECORD: case L_FORCE_LISTED: case L_DEFORM_R: case L_DEFORM_M_R:
+    case L_FORCE_M_RECORD: case L_FORCE_M_LISTED:
         return FSIM_PHASE_SOLID;
     default: return FSIM_PHASE_CELL;
     }
@@ -3547,9 +3602,9 @@ void launch_k_iota(int grid, cudaStream_t st, int *a, int n)
     k_iota<<<grid, kBlock, 0, st>>>(a, n);
 }
 
-void launch_k_virt_normal(int grid, cudaStream_t st, const DevParams P, const float4 *v_posr, const int *v_cell, const int *start_v, float4 *v_normal, int n, int reach)
+void launch_k_virt_normal(int grid, cudaStream_t st, const DevParams P, const float4 *v_posr, const int *v_cell, const int *start_v, float4 *v_normal, int n)
 {
-    k_virt_normal<<<grid, kBlock, 0, st>>>(P, v_posr, v_cell, start_v, v_normal, n, reach);
+    k_virt_normal<<<grid, kBlock, 0, st>>>(P, v_posr, v_cell, start_v, v_normal, n);
 }
 
 void launch_k_fluid_to_mixed(int grid, cudaStream_t st, const DevParams P, float4 *posr, float4 *velp, int *cell, int n, unsigned *flags)
@@ -3592,9 +3647,9 @@ void launch_k_probe(int grid, cudaStream_t st, const DevParams P, const ProbeArg
     k_probe<<<grid, kBlock, 0, st>>>(P, A);
 }
 
-void launch_k_neighbor_counts(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, int reach_v, int *out, int n)
+void launch_k_neighbor_counts(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, int *out, int n)
 {
-    k_neighbor_counts<<<grid, kBlock, 0, st>>>(P, Pv, fposr, cell_f, start_f, ids_f, s_pos, start_s, ids_s, v_posr, start_v, reach_v, out, n);
+    k_neighbor_counts<<<grid, kBlock, 0, st>>>(P, Pv, fposr, cell_f, start_f, ids_f, s_pos, start_s, ids_s, v_posr, start_v, out, n);
 }
 
 void launch_k_neighbor_counts_nl(int grid, cudaStream_t st, const DevParams P, const float4 *fposr, const int *list, const int2 *cnt, const float4 *s_pos, const float4 *v_posr, int *out, int n)
@@ -3602,9 +3657,9 @@ void launch_k_neighbor_counts_nl(int grid, cudaStream_t st, const DevParams P, c
     k_neighbor_counts_nl<<<grid, kBlock, 0, st>>>(P, fposr, list, cnt, s_pos, v_posr, out, n);
 }
 
-void launch_k_neighbor_counts_mixed(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, const unsigned *v_cxyz, int reach_v, int *out, int n)
+void launch_k_neighbor_counts_mixed(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, const unsigned *v_cxyz, int *out, int n)
 {
-    k_neighbor_counts_mixed<<<grid, kBlock, 0, st>>>(P, Pv, fposr, cell_f, start_f, ids_f, s_pos, start_s, ids_s, v_posr, start_v, v_cxyz, reach_v, out, n);
+    k_neighbor_counts_mixed<<<grid, kBlock, 0, st>>>(P, Pv, fposr, cell_f, start_f, ids_f, s_pos, start_s, ids_s, v_posr, start_v, v_cxyz, out, n);
 }
 
 void launch_k_neighbor_counts_nlm(int grid, cudaStream_t st, const DevParams P, const float4 *fposr, const int *cell_f, const unsigned *cxyz_f, const int *list, const int2 *cnt, const float4 *s_pos, const unsigned *cxyz_s, const float4 *v_posr, const unsigned *cxyz_v, int *out, int n)

@@ -102,7 +102,7 @@ struct fsim_sim {
     bool nl_check = false;        // pairs also need neighbouring impact-grid cells (f_cxyz, v_icxyz, s_cxyz)
     unsigned *f_cxyz = nullptr, *v_icxyz = nullptr;
     DevParams Pl;                 // the list grid's parameters (else unused)
-    int ncell_l = 0, nl_cap = 0, nl_reach = 1;
+    int ncell_l = 0, nl_cap = 0;
     float nl_R2s = 0.0f, nl_move2 = 0.0f;
     int *nl_list = nullptr;
     int2 *nl_cnt = nullptr;
@@ -540,7 +540,7 @@ void plan_cell_nl(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, 
         const NlBuildArgs ba{h->f_x0,   h->f_lcell,  h->f_lstart, mixed ? h->v_abs : h->v_posr, h->v_start,
                              h->s_x0,   h->s_lstart, h->nf,       h->nl_cap,  h->nl_list,
                              h->nl_cnt, h->nl_state, h->d_flags,  h->nl_R2s,  h->nv,
-                             h->ns,     h->nl_reach};
+                             h->ns};
         const Item<NlBuildArgs> bt{h->Pl, ba};
         bi.push_back(bt);
         bb.push_back(blocks_for(h->nf, kNlBuildThreads));
@@ -803,10 +803,11 @@ void plan_solid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, in
             // sub-step 0 also resolves the step's list slots for the later sub-steps
             add_launch(pl, ab, mixed ? (k == 0 ? L_DEFORM_M_R : L_DEFORM_M) : (k == 0 ? L_DEFORM_R : L_DEFORM), it,
                        wb);
-            // plain form: sub-step 0 records each lane's fluid list, later sub-steps walk it
-            const bool lists = !mixed && !m[0]->cfg.solid_full_walk;
-            add_launch(pl, ab, mixed ? L_FORCE_M : !lists ? L_FORCE : k == 0 ? L_FORCE_RECORD : L_FORCE_LISTED, it,
-                       wb);
+            // sub-step 0 records each lane's fluid list, later sub-steps walk it
+            const bool lists = !m[0]->cfg.solid_full_walk;
+            const int plain = !lists ? L_FORCE : k == 0 ? L_FORCE_RECORD : L_FORCE_LISTED;
+            const int mix = !lists ? L_FORCE_M : k == 0 ? L_FORCE_M_RECORD : L_FORCE_M_LISTED;
+            add_launch(pl, ab, mixed ? mix : plain, it, wb);
             add_launch(pl, ab, L_UPDATE, it, ub);
         }
         return;
@@ -1120,8 +1121,7 @@ fsim_status sort_virtual(fsim_sim *h, const float *vpos_host, float4 *vpos_dev =
     if (e == cudaSuccess && (st = enqueue_plan(pl, h->stream, 0)) == FSIM_OK) {
         e = cudaMemsetAsync(h->v_velp, 0, sizeof(float4) * n, h->stream);
         // the normal sums the walls within R: any grid of cells >= R finds them
-        launch_k_virt_normal(blocks_for(n, kBlock), h->stream, G, h->v_posr, h->v_cell, h->v_start, h->v_normal, n,
-                             h->nl ? h->nl_reach : 1);
+        launch_k_virt_normal(blocks_for(n, kBlock), h->stream, G, h->v_posr, h->v_cell, h->v_start, h->v_normal, n);
         if (h->nl) launch_k_cells_of(blocks_for(n, kBlock), h->stream, h->P, h->v_posr, n, h->v_icell, h->v_icxyz);
         if (e == cudaSuccess) e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
@@ -1267,15 +1267,16 @@ fsim_status alloc_state(fsim_sim *h)
         return st;
     h->s_P = h->s_F + 9 * (size_t)ns;
     // virtual
-    if ((st = dalloc(h, &h->v_posr, nv)) || (st = dalloc(h, &h->v_velp, nv)) || (st = dalloc(h, &h->v_normal, nv)) ||
+    if ((st = dalloc(h, &h->v_posr, nv + kNlReadAhead)) || (st = dalloc(h, &h->v_velp, nv)) || (st = dalloc(h, &h->v_normal, nv)) ||
         (st = dalloc(h, &h->v_orig, nv)) || (st = dalloc(h, &h->v_cell, nv)) ||
-        (st = dalloc(h, &h->v_start, (h->nl ? h->ncell_l : nc) + 1)))
+        (st = dalloc(h, &h->v_start, nc + 1)))
         return st;
     // fluid neighbour lists
     if (h->nl) {
         const int ncl = h->ncell_l;
         if ((st = dalloc(h, &h->nl_list, (size_t)h->nl_cap * nf)) || (st = dalloc(h, &h->nl_cnt, nf)) ||
-            (st = dalloc(h, &h->nl_state, 1)) || (st = dalloc(h, &h->f_x0, nf)) || (st = dalloc(h, &h->s_x0, ns)) ||
+            (st = dalloc(h, &h->nl_state, 1)) || (st = dalloc(h, &h->f_x0, nf + kNlReadAhead)) ||
+            (st = dalloc(h, &h->s_x0, ns + kNlReadAhead)) ||
             (st = dalloc(h, &h->f_ids, nf)) || (st = dalloc(h, &h->f_lcell, nf)) ||
             (st = dalloc(h, &h->f_lcnt, ncl)) || (st = dalloc(h, &h->f_lstart, ncl + 1)) ||
             (st = dalloc(h, &h->s_ids, ns)) || (st = dalloc(h, &h->s_lcell, ns)) ||
@@ -1284,7 +1285,7 @@ fsim_status alloc_state(fsim_sim *h)
             (st = dalloc(h, &h->f_spos, nf)))
             return st;
         if (h->nl_check && ((st = dalloc(h, &h->f_cxyz, nf)) || (st = dalloc(h, &h->v_icxyz, nv)))) return st;
-        if (h->mixed && ((st = dalloc(h, &h->f_cell2, nf)) || (st = dalloc(h, &h->v_abs, nv)))) return st;
+        if (h->mixed && ((st = dalloc(h, &h->f_cell2, nf)) || (st = dalloc(h, &h->v_abs, nv + kNlReadAhead)))) return st;
         NlState init{};
         init.force = 1; // the first step builds
         CK(cudaMemcpyAsync(h->nl_state, &init, sizeof init, cudaMemcpyHostToDevice, h->stream));
@@ -1312,7 +1313,7 @@ fsim_status alloc_state(fsim_sim *h)
     CK(cudaMemsetAsync(h->f_cell, 0, sizeof(int) * (nf ? nf : 1), h->stream));
     CK(cudaMemsetAsync(h->f_start, 0, sizeof(int) * (nc + 1), h->stream));
     CK(cudaMemsetAsync(h->s_start, 0, sizeof(int) * (nc + 1), h->stream));
-    CK(cudaMemsetAsync(h->v_start, 0, sizeof(int) * ((h->nl ? h->ncell_l : nc) + 1), h->stream));
+    CK(cudaMemsetAsync(h->v_start, 0, sizeof(int) * (nc + 1), h->stream));
     CK(cudaMemsetAsync(h->s_np, 0, sizeof(float4) * (ns ? ns : 1), h->stream));
     return FSIM_OK;
 }
@@ -1385,30 +1386,6 @@ namespace {
 // on all three axes) that is the set {r < R}, else (nl_check) the list sweep
 // also compares the pair's packed cell coordinates.  The list grid has cells
 // of at least Rs (1 + 1e-3) on the reference grid's origin.
-// The list grid's cells per axis (at least Rs (1 + 1e-3) / reach wide) and its
-// reach, the finest of 3, 2, 1 whose cells stay few enough.  The finer the
-// cells, the fewer candidates a build tests (about 310 against 730 per
-// particle) and the more a warp's lanes walk alike.  Instances of up to 262,144
-// fluid particles keep reach 1: there the sweep is bound by latency and not by
-// the L1, so the order gains it nothing.
-int list_grid(const fsim_derived &d, double Rs, size_t nf, size_t ns, size_t nv, int n[3])
-{
-    for (int reach = nf > 262144 ? 3 : 1;; --reach) {
-        double cells = 1.0;
-        bool fits = true;
-        for (int a = 0; a < 3; ++a) {
-            const double L = (double)d.cell_max[a] - (double)d.cell_min[a];
-            const double c = std::max(1.0, std::floor(reach * L / (Rs * (1.0 + 1e-3))));
-            n[a] = (int)std::min(c, 1e9);
-            cells *= c;
-            // FP32 rounding of the cell coordinate against the 1e-3 margin
-            fits = fits && 8e-7 * c < 0.5e-3 * reach;
-        }
-        const double most = std::min((double)kMaxScanTiles * kScanTile, 64.0 * ((double)nf + ns + nv) + 65536.0);
-        if (reach == 1 || (fits && cells <= most)) return reach;
-    }
-}
-
 void setup_lists(fsim_sim *h)
 {
     h->nl = false;
@@ -1435,15 +1412,14 @@ void setup_lists(fsim_sim *h)
     if (!(move > 0.0)) return;
     DevParams Pl = h->P;
     int n[3];
-    const int reach = list_grid(h->der, Rs, h->nf, h->ns, h->nv, n);
     for (int a = 0; a < 3; ++a) {
         const double L = (double)h->der.cell_max[a] - (double)h->der.cell_min[a];
+        n[a] = std::max(1, (int)std::floor(L / (Rs * (1.0 + 1e-3))));
         Pl.cinv[a] = (float)(n[a] / L);
         Pl.cdx[a] = (float)(L / n[a]);
         // the cells must still hold Rs with the FP32 inverse the kernels use
-        if (!(reach / (double)Pl.cinv[a] >= Rs * (1.0 + 5e-4))) return;
+        if (!(1.0 / (double)Pl.cinv[a] >= Rs * (1.0 + 5e-4))) return;
     }
-    h->nl_reach = reach;
     Pl.nx = n[0];
     Pl.ny = n[1];
     Pl.nz = n[2];
@@ -2017,11 +1993,11 @@ extern "C" fsim_status fsim_neighbor_counts(fsim_handle h, int *out, size_t byte
         launch_k_neighbor_counts_mixed(g, h->stream, h->P, h->nl ? h->Pl : h->P, h->f_posr[h->f_cur], h->f_cell,
                                        h->f_start, h->nl ? h->f_ids : nullptr, h->s_pos[h->s_cur], h->s_start,
                                        h->nl ? h->s_ids : nullptr, h->v_posr, h->v_start,
-                                       h->nl ? h->v_icxyz : nullptr, h->nl_reach, d_counts, h->nf);
+                                       h->nl ? h->v_icxyz : nullptr, d_counts, h->nf);
     else
         launch_k_neighbor_counts(g, h->stream, h->P, h->nl ? h->Pl : h->P, h->f_posr[h->f_cur], h->f_cell,
                                  h->f_start, h->nl ? h->f_ids : nullptr, h->s_pos[h->s_cur], h->s_start,
-                                 h->nl ? h->s_ids : nullptr, h->v_posr, h->v_start, h->nl_reach, d_counts, h->nf);
+                                 h->nl ? h->s_ids : nullptr, h->v_posr, h->v_start, d_counts, h->nf);
     CK_LAUNCH();
     // reorder to input order in place is not possible; copy sorted and unpermute on the host
     std::vector<int> sorted(3 * (size_t)h->nf), orig(h->nf);
@@ -2380,7 +2356,6 @@ struct SnapHeader {
     fsim_config cfg;
 };
 constexpr char kSnapMagic[8] = {'F', 'S', 'I', 'M', 'S', 'N', 'P', '1'};
-constexpr uint32_t kSnapVersion = 3;     // version 2 loads too (snap_arrays_v2)
 constexpr size_t kSnapHeaderBytes = 512; // header padded; arrays start 16-byte aligned
 static_assert(sizeof(SnapHeader) <= kSnapHeaderBytes, "snapshot header");
 
@@ -2388,9 +2363,6 @@ struct SnapArray {
     void *dev;
     size_t bytes;
 };
-// places of some arrays in snap_arrays
-enum { kSnapWallPos = 9, kSnapWallVel = 10, kSnapWallOrig = 12, kSnapWallStart = 14, kSnapFluidListStart = 17,
-       kSnapSolidListStart = 20, kSnapListState = 22, kSnapWallAbs = 23 };
 // A neighbour-list instance also saves what its lists were built from (the
 // positions and list-grid cells of the last build, the particles' order then)
 // and its list state; loading rebuilds the same lists from them.
@@ -2401,7 +2373,7 @@ std::vector<SnapArray> snap_arrays(fsim_sim *h, int pf, int ps)
         {h->f_posr[pf], 16 * nf}, {h->f_velp[pf], 16 * nf}, {h->f_orig[pf], 4 * nf},   {h->f_cell, 4 * nf},
         {h->s_pos[ps], 16 * ns},  {h->s_vel[ps], 16 * ns},  {h->s_ref[ps], 16 * ns},   {h->s_type[ps], 4 * ns},
         {h->s_orig[ps], 4 * ns},  {h->v_posr, 16 * nv},     {h->v_velp, 16 * nv},      {h->v_normal, 16 * nv},
-        {h->v_orig, 4 * nv},      {h->v_cell, 4 * nv},      {h->v_start, 4 * ((h->nl ? h->ncell_l : nc) + 1)}};
+        {h->v_orig, 4 * nv},      {h->v_cell, 4 * nv},      {h->v_start, 4 * (nc + 1)}};
     if (h->nl) {
         const size_t ncl = h->ncell_l;
         const std::vector<SnapArray> b = {{h->f_x0, 16 * nf},           {h->f_lcell, 4 * nf},
@@ -2412,89 +2384,6 @@ std::vector<SnapArray> snap_arrays(fsim_sim *h, int pf, int ps)
         if (h->mixed) a.push_back({h->v_abs, 16 * nv});
     }
     return a;
-}
-
-// Version 2 of the format, of a neighbour-list instance: the same arrays, but
-// the particles and walls were sorted on a list grid of cells as wide as the
-// list radius.  What describes that order comes back as {nullptr, bytes}.
-std::vector<SnapArray> snap_arrays_v2(fsim_sim *h)
-{
-    std::vector<SnapArray> a = snap_arrays(h, 0, 0);
-    if (!h->nl) return a;
-    const double R = std::sqrt((double)h->der.impact_distance_square), Rs = R * (1.0 + h->cfg.neighbor_skin);
-    size_t ncl = 1;
-    for (int k = 0; k < 3; ++k) {
-        const double L = (double)h->der.cell_max[k] - (double)h->der.cell_min[k];
-        ncl *= (size_t)std::max(1, (int)std::floor(L / (Rs * (1.0 + 1e-3))));
-    }
-    a[kSnapWallStart].bytes = 4 * ((size_t)h->ncell + 1);
-    a[kSnapFluidListStart].bytes = a[kSnapSolidListStart].bytes = 4 * (ncl + 1);
-    for (size_t k = kSnapWallPos; k < a.size(); ++k) a[k].dev = nullptr;
-    return a;
-}
-
-size_t snap_payload(const std::vector<SnapArray> &arrays)
-{
-    size_t b = 0;
-    for (const SnapArray &a : arrays) b += (a.bytes + 15) & ~size_t(15);
-    return b;
-}
-
-// The walls and list state of a version-2 snapshot of a neighbour-list
-// instance: the walls sorted anew with their densities, velocities and
-// pressures, and a list build forced at the next step.
-fsim_status restore_v2_lists(fsim_sim *h, const char *in)
-{
-    const std::vector<SnapArray> arrays = snap_arrays_v2(h);
-    std::vector<const char *> at;
-    for (const SnapArray &a : arrays) {
-        at.push_back(in);
-        in += (a.bytes + 15) & ~size_t(15);
-    }
-    const char *posr = at[kSnapWallPos], *velp = at[kSnapWallVel], *orig = at[kSnapWallOrig],
-               *abs = h->mixed ? at[kSnapWallAbs] : posr;
-    const size_t nv = h->nv;
-    std::vector<float> xyz(3 * nv);
-    std::vector<float4> u(nv), by_input(nv), sorted(nv);
-    std::vector<float> rho(nv);
-    for (size_t k = 0; k < nv; ++k) {
-        int o;
-        float4 x, r, v;
-        std::memcpy(&o, orig + 4 * k, 4);
-        std::memcpy(&r, posr + 16 * k, 16);
-        std::memcpy(&x, abs + 16 * k, 16);
-        std::memcpy(&v, velp + 16 * k, 16);
-        if (o < 0 || o >= h->nv) {
-            fsim_set_error("corrupt snapshot (wall ids)");
-            return FSIM_EIO;
-        }
-        xyz[3 * (size_t)o] = x.x;
-        xyz[3 * (size_t)o + 1] = x.y;
-        xyz[3 * (size_t)o + 2] = x.z;
-        rho[o] = r.w;
-        by_input[o] = v;
-    }
-    fsim_status st;
-    if (nv) {
-        if ((st = sort_virtual(h, xyz.data()))) return st;
-        if (h->mixed && (st = walls_to_mixed(h))) return st;
-        std::vector<int> order(nv);
-        CK(cudaStreamSynchronize(h->stream));
-        CK(cudaMemcpy(order.data(), h->v_orig, sizeof(int) * nv, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(sorted.data(), h->v_posr, sizeof(float4) * nv, cudaMemcpyDeviceToHost));
-        for (size_t k = 0; k < nv; ++k) {
-            sorted[k].w = rho[order[k]];
-            u[k] = by_input[order[k]];
-        }
-        CK(cudaMemcpy(h->v_posr, sorted.data(), sizeof(float4) * nv, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(h->v_velp, u.data(), sizeof(float4) * nv, cudaMemcpyHostToDevice));
-    }
-    NlState saved, fresh{};
-    std::memcpy(&saved, at[kSnapListState], sizeof saved);
-    fresh.builds = saved.builds;
-    fresh.force = 1;
-    CK(cudaMemcpy(h->nl_state, &fresh, sizeof fresh, cudaMemcpyHostToDevice));
-    return FSIM_OK;
 }
 
 // Build the lists from the saved build state (positions and cells of the last
@@ -2519,7 +2408,7 @@ fsim_status nl_restore(fsim_sim *h)
                std::vector<Item<NlBuildArgs>>{{h->Pl, NlBuildArgs{h->f_x0, h->f_lcell, h->f_lstart, vpos,
                                                                   h->v_start, h->s_x0, h->s_lstart, h->nf, h->nl_cap,
                                                                   h->nl_list, h->nl_cnt, h->nl_state, h->d_flags,
-                                                                  h->nl_R2s, h->nv, h->ns, h->nl_reach}}},
+                                                                  h->nl_R2s, h->nv, h->ns}}},
                {blocks_for(h->nf, kNlBuildThreads)}, kRebuildBuildGrid, 1);
     pl.host = ab.bytes;
     cudaError_t e = cudaMalloc((void **)&pl.arena, std::max<size_t>(ab.bytes.size(), 1));
@@ -2540,12 +2429,18 @@ fsim_status nl_restore(fsim_sim *h)
     CK(cudaMemcpy(h->nl_state, &saved, sizeof saved, cudaMemcpyHostToDevice));
     return FSIM_OK;
 }
+size_t snap_payload(fsim_sim *h)
+{
+    size_t b = 0;
+    for (const SnapArray &a : snap_arrays(h, 0, 0)) b += (a.bytes + 15) & ~size_t(15);
+    return b;
+}
 } // namespace
 
 extern "C" fsim_status fsim_snapshot_bytes(fsim_handle h, size_t *bytes)
 {
     if (!h || !bytes) return FSIM_EINVAL;
-    *bytes = kSnapHeaderBytes + snap_payload(snap_arrays(h, 0, 0));
+    *bytes = kSnapHeaderBytes + snap_payload(h);
     return FSIM_OK;
 }
 
@@ -2554,7 +2449,7 @@ extern "C" fsim_status fsim_snapshot_save(fsim_handle h, long long step, void *b
     NvtxRange nvtx_("fsim_snapshot_save");
     if (!h || !buf) return FSIM_EINVAL;
     if (h->batch) batch_wait(h);
-    const size_t need = kSnapHeaderBytes + snap_payload(snap_arrays(h, 0, 0));
+    const size_t need = kSnapHeaderBytes + snap_payload(h);
     if (bytes != need) {
         fsim_set_error("a snapshot of this instance takes %zu bytes, got %zu", need, bytes);
         return FSIM_EINVAL;
@@ -2563,7 +2458,7 @@ extern "C" fsim_status fsim_snapshot_save(fsim_handle h, long long step, void *b
     SnapHeader hd;
     std::memset(&hd, 0, sizeof hd);
     std::memcpy(hd.magic, kSnapMagic, 8);
-    hd.version = kSnapVersion;
+    hd.version = 2;
     hd.config_bytes = sizeof(fsim_config);
     hd.step = step;
     hd.n_fluid = h->nf;
@@ -2598,17 +2493,15 @@ extern "C" fsim_status fsim_snapshot_load(const void *buf, size_t bytes, int dev
         return FSIM_EIO;
     }
     std::memcpy(&hd, buf, sizeof hd);
-    if (std::memcmp(hd.magic, kSnapMagic, 8) || (hd.version != 2 && hd.version != kSnapVersion) || hd.config_bytes != sizeof(fsim_config) ||
+    if (std::memcmp(hd.magic, kSnapMagic, 8) || hd.version != 2 || hd.config_bytes != sizeof(fsim_config) ||
         hd.n_fluid < 0 || hd.n_solid < 0 || hd.n_virt < 0) {
-        fsim_set_error("not a version-2 or version-3 fluidsim snapshot");
+        fsim_set_error("not a version-2 fluidsim snapshot");
         return FSIM_EIO;
     }
     fsim_sim *h = nullptr;
     fsim_status st = new_handle(&hd.cfg, hd.n_fluid, hd.n_solid, hd.n_virt, device, &h);
     if (st) return st;
-    // (no array is allocated yet: only the sizes count here)
-    const bool v2 = hd.version == 2;
-    if (h->ncell != hd.ncell || bytes != kSnapHeaderBytes + snap_payload(v2 ? snap_arrays_v2(h) : snap_arrays(h, 0, 0)) ||
+    if (h->ncell != hd.ncell || bytes != kSnapHeaderBytes + snap_payload(h) ||
         hd.payload_bytes != bytes - kSnapHeaderBytes) {
         fsim_set_error("snapshot size does not match its header");
         delete h;
@@ -2626,8 +2519,8 @@ extern "C" fsim_status fsim_snapshot_load(const void *buf, size_t bytes, int dev
     std::vector<float> ref(3 * (size_t)ns);
     const char *ref_src = nullptr, *orig_src = nullptr;
     cudaError_t e = cudaSuccess;
-    for (const SnapArray &a : v2 ? snap_arrays_v2(h) : snap_arrays(h, 0, 0)) {
-        if (a.dev && a.bytes && e == cudaSuccess) e = cudaMemcpy(a.dev, in + off, a.bytes, cudaMemcpyHostToDevice);
+    for (const SnapArray &a : snap_arrays(h, 0, 0)) {
+        if (a.bytes && e == cudaSuccess) e = cudaMemcpy(a.dev, in + off, a.bytes, cudaMemcpyHostToDevice);
         if (a.dev == h->s_ref[0]) ref_src = in + off;
         if (a.dev == h->s_orig[0]) orig_src = in + off;
         off += (a.bytes + 15) & ~size_t(15);
@@ -2668,7 +2561,7 @@ extern "C" fsim_status fsim_snapshot_load(const void *buf, size_t bytes, int dev
             return st ? st : FSIM_ECUDA;
         }
     }
-    if (h->nl && (st = v2 ? restore_v2_lists(h, in + kSnapHeaderBytes) : nl_restore(h))) {
+    if (h->nl && (st = nl_restore(h))) {
         free_all(h);
         delete h;
         return st;
@@ -3246,7 +3139,7 @@ extern "C" fsim_status fsim_estimate_bytes(const fsim_config *cfg, int n_fluid, 
     if (cfg->precision == FSIM_PRECISION_MIXED) b += nc * sizeof(float2); // per-cell references
     if (cfg->neighbor_skin > 0.0f) {
         // fluid neighbour lists (as setup_lists sizes them) and the list-grid
-        // sort, build state and per-step index:
+        // sort, build state and per-step index (at most as many cells as nc):
         // lists, list counts, ids, list cells, packed cells; x0, the 32-byte
         // records and the positions in the index's order; the mixed form's
         // carried cells and absolute wall positions
@@ -3256,12 +3149,7 @@ extern "C" fsim_status fsim_estimate_bytes(const fsim_config *cfg, int n_fluid, 
         b += nf * (cap + 5) * sizeof(int) + nf * 4 * sizeof(float4);
         b += ns * (sizeof(float4) + 2 * sizeof(int)) + nv * 2 * sizeof(int);
         if (cfg->precision == FSIM_PRECISION_MIXED) b += nf * sizeof(int) + nv * sizeof(float4);
-        int n[3];
-        const double skin = cfg->neighbor_skin;
-        list_grid(d, std::sqrt((double)d.impact_distance_square) * (1.0 + skin), nf, ns, nv, n);
-        const size_t ncl = (size_t)n[0] * n[1] * n[2];
-        b += (ncl * 2 + (ncl + 1) * 2) * sizeof(int) + sizeof(NlState);
-        if (ncl > nc) b += (ncl - nc) * sizeof(int); // the walls' starts
+        b += nc * sizeof(int) * 2 + (nc + 1) * sizeof(int) * 2 + sizeof(NlState);
     }
     b += 2 * kMaxScanTiles * sizeof(int) + sizeof(unsigned);
     size_t words = 3 * nf;

@@ -199,9 +199,9 @@ struct NlBuildArgs {
     unsigned *flags;
     float R2s; // list radius^2
     int nv, ns;
-    int reach; // cells of the list grid that cover the list radius
 };
 constexpr int kNlGroup = 8;                // list entries per 32-byte group (the capacity is a multiple)
+constexpr int kNlReadAhead = 16;           // entries past its count that the build may read of a position array
 constexpr int kNlPad = 2 * kNlGroup;       // capacity set aside for the species' group boundaries
 constexpr int kNlIndexMax = (1 << 30) - 1; // particles of a species
 constexpr int kNlCapMax = 32768;           // entries of a species fit 16 bits
@@ -312,8 +312,8 @@ struct SolidArgs {
     // static reference-configuration neighbours (CSR over input ids)
     const int *orig, *inv, *nbr_off, *nbr_orig;
     const int *nbr_owner;  // input id of each entry's particle
-    // fluid candidates of each solid lane within the recording radius (plain
-    // form, entry-major: entry e of lane t at e * (kSolidGroup * n) + t), their
+    // fluid candidates of each solid lane within the recording radius (with the
+    // mixed form's 6-bit cell code above kCodeShift; entry-major: entry e of lane t at e * (kSolidGroup * n) + t), their
     // counts (-1: overflow) and where each particle was when they were recorded
     int *fl, *fl_cnt;
     float4 *fl_org;
@@ -484,7 +484,7 @@ enum LaunchKind {
     L_ZERO, L_HASH, L_SCAN_REDUCE, L_SCAN_PARTIALS, L_SCAN_APPLY, L_SCATTER, L_GATHER_F, L_GATHER_S,
     L_COUPLE, L_VIRT, L_SWEEP, L_DEFORM, L_FORCE, L_UPDATE,
     L_HASH_M, L_CELLREF, L_COUPLE_M, L_VIRT_M, L_DEFORM_M, L_FORCE_M, L_SOLID_FUSED, L_SOLID_SLOTS,
-    L_FORCE_RECORD, L_FORCE_LISTED, L_DEFORM_R, L_DEFORM_M_R,
+    L_FORCE_RECORD, L_FORCE_LISTED, L_FORCE_M_RECORD, L_FORCE_M_LISTED, L_DEFORM_R, L_DEFORM_M_R,
     L_NL_DECIDE, L_NL_BUILD, L_RANK_F, L_RANK_S, L_MIXED_ABS, L_MIXED_REC
 };
 
@@ -573,7 +573,7 @@ int fused_grid(bool mixed, int want);
 // One launch of a utility kernel (kBlock threads per block) on `st`.
 void launch_k_pack_f4(int grid, cudaStream_t st, const float *xyz, const float *w, int n, float wconst, float4 *out);
 void launch_k_iota(int grid, cudaStream_t st, int *a, int n);
-void launch_k_virt_normal(int grid, cudaStream_t st, const DevParams P, const float4 *v_posr, const int *v_cell, const int *start_v, float4 *v_normal, int n, int reach);
+void launch_k_virt_normal(int grid, cudaStream_t st, const DevParams P, const float4 *v_posr, const int *v_cell, const int *start_v, float4 *v_normal, int n);
 void launch_k_fluid_to_mixed(int grid, cudaStream_t st, const DevParams P, float4 *posr, float4 *velp, int *cell, int n, unsigned *flags);
 void launch_k_offsets_in_cells(int grid, cudaStream_t st, const DevParams P, float4 *pos, const int *cell, int n);
 void launch_k_unpermute_mixed(int grid, cudaStream_t st, const DevParams P, const float4 *pos, const float4 *velp, const int *cell, const int *orig, int n, int what, float *out);
@@ -582,9 +582,9 @@ void launch_k_unpermute_words(int grid, cudaStream_t st, const int *src, const i
 void launch_k_permute_in_mixed(int grid, cudaStream_t st, const DevParams P, float4 *pos, float4 *velp, const int *cell, const int *orig, int n, int what, const float *in);
 void launch_k_permute_in_f4(int grid, cudaStream_t st, float4 *dst, const int *orig, int n, int comp, int width, const float *in);
 void launch_k_probe(int grid, cudaStream_t st, const DevParams P, const ProbeArgs A);
-void launch_k_neighbor_counts(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, int reach_v, int *out, int n);
+void launch_k_neighbor_counts(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, int *out, int n);
 void launch_k_neighbor_counts_nl(int grid, cudaStream_t st, const DevParams P, const float4 *fposr, const int *list, const int2 *cnt, const float4 *s_pos, const float4 *v_posr, int *out, int n);
-void launch_k_neighbor_counts_mixed(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, const unsigned *v_cxyz, int reach_v, int *out, int n);
+void launch_k_neighbor_counts_mixed(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, const unsigned *v_cxyz, int *out, int n);
 void launch_k_neighbor_counts_nlm(int grid, cudaStream_t st, const DevParams P, const float4 *fposr, const int *cell_f, const unsigned *cxyz_f, const int *list, const int2 *cnt, const float4 *s_pos, const unsigned *cxyz_s, const float4 *v_posr, const unsigned *cxyz_v, int *out, int n);
 void launch_k_gather_f4(int grid, cudaStream_t st, const int *ids, const float4 *src, int n, float4 *dst);
 void launch_k_pack_records(int grid, cudaStream_t st, const float4 *posr, const float4 *velp, const unsigned *cxyz, int n, float4 *rec);

@@ -433,9 +433,8 @@ fsim_status fsim_probe(fsim_handle h, const float *points, int n, float *out);
  * current cell-sorted order, so that an instance restored from it continues
  * bit for bit like the original.  Per-step products (cell starts, solid
  * stress, derivatives) are recomputed by the next step.  The format is this
- * library's own: fixed header ("FSIMSNP1", version 3, counts, fsim_config),
- * then raw device arrays, native byte order.  Version-2 snapshots load too; an
- * instance with neighbour lists then rebuilds them at its next step. */
+ * library's own: fixed header ("FSIMSNP1", version 1, counts, fsim_config),
+ * then raw device arrays, native byte order. */
 fsim_status fsim_snapshot_bytes(fsim_handle h, size_t *bytes);
 fsim_status fsim_snapshot_save(fsim_handle h, long long step, void *buf, size_t bytes);
 fsim_status fsim_snapshot_load(const void *buf, size_t bytes, int device, fsim_handle *out, long long *step);

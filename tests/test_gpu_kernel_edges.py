@@ -1,0 +1,147 @@
+"""The list build, the list sweep's lanes and the solid sub-steps at their edges.
+
+Sizes around the ends of warps, blocks, the build's chunks and of the rule for
+the lanes that share a particle (8,192 and 16,384 fluid particles); batches of
+which only one member rebuilds; the mixed form's solid-fluid lists; odd and even
+numbers of solid sub-steps.
+
+The rates are held to the bound of the other per-phase tests: at most twice
+the FP32 oracle's own error against FP64, plus 5e-5 of the largest value; the
+mixed form's to 2e-4 of the cell walk's, the bound of tests/test_gpu_lists.py.
+Everything else is compared exactly.
+"""
+import numpy as np
+import pytest
+
+from conftest import nerr
+from fluidsim_gb300 import api, cases
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def _box(fluid, tank=None, layers=3, solid=True, precision=api.PRECISION_FP32, seed=3, gap=1):
+    tank = tank or (fluid[0] + 13, fluid[1] + 6, fluid[2] + 1)
+    cfg = cases._config(0.01, tank, keep=True, precision=precision)
+    block = (2, min(6, tank[1]), min(6, tank[2])) if solid else (0, 0, 0)
+    case = cases._case(0.01, tank, fluid, (fluid[0] + gap, 0, 0), block, 2 if solid else 0, virt_layers=layers,
+                       jitter=0.01, seed=seed)
+    cfg, pa = cases.make((cfg, case))
+    rng = np.random.default_rng(seed)
+    vel = rng.uniform(-0.3, 0.3, pa.fluid_vel.shape).astype(np.float32)
+    return cfg, api.ParticleArrays(pa.fluid_pos, vel, pa.fluid_rho, pa.fluid_p, pa.solid_pos, pa.solid_vel,
+                                   pa.solid_ref_pos, pa.solid_type, pa.virt_pos)
+
+
+SIZES = [(1, 1, 1), (1, 1, 31), (3, 11, 1), (1, 127, 1), (3, 43, 1), (16, 16, 32), (17, 16, 32), (25, 26, 25),
+         (26, 26, 25)]
+
+
+@pytest.mark.parametrize("fluid", SIZES)
+def test_plain_rates_and_pairs(fluid):
+    cfg, pa = _box(fluid)
+    r64, r32 = orc.OracleSim(cfg, pa, "f64"), orc.OracleSim(cfg, pa, "f32")
+    with api.Simulation(cfg, pa, device=0) as sim:
+        for ph in (api.PHASE_CELL, api.PHASE_COUPLE, api.PHASE_VIRT):
+            sim.phase(ph)
+            r64.phase(ph)
+            r32.phase(ph)
+        assert np.array_equal(sim.list_counts(), sim.neighbor_counts())
+        assert np.array_equal(sim.neighbor_counts(), r64.neighbor_counts())
+        sim.phase(api.PHASE_FLUID)
+        r64.phase(api.PHASE_FLUID)
+        r32.phase(api.PHASE_FLUID)
+        sim.sync()
+        for f in ("fluid_drho_dt", "fluid_du_dt"):
+            want = r64.get(f)
+            assert nerr(sim.get(f), want) <= 2.0 * nerr(r32.get(f), want) + 5e-5, f
+
+
+@pytest.mark.parametrize("fluid", [(1, 1, 1), (3, 11, 1), (16, 16, 32), (17, 16, 32), (25, 26, 25), (26, 26, 25)])
+def test_mixed_rates_and_pairs(fluid):
+    cfg, pa = _box(fluid, precision=api.PRECISION_MIXED)
+    walk = api.Config.from_buffer_copy(cfg)
+    walk.neighbor_skin = 0.0
+    with api.Simulation(cfg, pa, device=0) as a, api.Simulation(walk, pa, device=0) as b:
+        for ph in range(4):
+            a.phase(ph)
+            b.phase(ph)
+            if ph == api.PHASE_CELL:
+                assert np.array_equal(a.list_counts(), a.neighbor_counts())
+                assert np.array_equal(a.neighbor_counts(), b.neighbor_counts())
+        for f in ("fluid_drho_dt", "fluid_du_dt"):
+            assert nerr(a.get(f), b.get(f).astype(np.float64)) <= 2e-4, f
+
+
+def test_one_member_of_a_batch_rebuilds():
+    # solids out of the fluid's reach: where they touch, the launch forms of the plain
+    # form round the fluid-solid terms differently in the last bit
+    specs = [_box((9, 8, 7), seed=1, gap=5), _box((20, 18, 19), seed=2, gap=5),
+             _box((11, 10, 13), solid=False, seed=4)]
+    fast = specs[1][1]
+    fast.fluid_vel[:, 0] += 3.0
+    alone, members = [], []
+    for cfg, pa in specs:
+        s = api.Simulation(cfg, pa, device=0)
+        s.step(14)
+        s.sync()
+        alone.append({f: s.get(f) for f in ("fluid_pos", "fluid_vel", "fluid_p")})
+        alone[-1]["builds"] = s.list_stats()["builds"]
+        s.close()
+        members.append(api.Simulation(cfg, pa, device=0))
+    with api.Batch(members) as b:
+        b.step(14)
+        b.sync()
+        for s, want in zip(members, alone):
+            assert s.list_stats()["builds"] == want.pop("builds")
+            for f, w in want.items():
+                assert np.array_equal(s.get(f), w), f
+    assert members[1].list_stats()["builds"] > members[0].list_stats()["builds"]
+    for s in members:
+        s.close()
+
+
+@pytest.mark.parametrize("speed_share", [0.0, 0.75])
+def test_mixed_solid_fluid_lists_equal_full_walk(speed_share):
+    """The mixed form's solid sub-steps after the first walk recorded lists of
+    (particle, cell code) as the plain form's do: bit for bit the full walk of every
+    sub-step, at rest and with the plate at 0.75 of the allowed displacement (0.1 R)
+    per sub-step, where later sub-steps fall back to the walk."""
+    cfg, pa = cases.make(cases.tiny_box(precision=api.PRECISION_MIXED))
+    R = float(np.sqrt(api.derive(cfg).impact_distance_square))
+    shift = pa.solid_pos[:, 0].min() - pa.fluid_pos[:, 0].max() - cfg.particle_diameter
+    sp, sr, sv = pa.solid_pos.copy(), pa.solid_ref_pos.copy(), np.zeros_like(pa.solid_vel)
+    sp[:, 0] -= shift
+    sr[:, 0] -= shift
+    sv[pa.solid_type == 0, 0] = -speed_share * 0.1 * R / (cfg.dt / cfg.solid_sub_step)
+    pa = api.ParticleArrays(pa.fluid_pos, pa.fluid_vel, pa.fluid_rho, pa.fluid_p, sp, sv, sr, pa.solid_type,
+                            pa.virt_pos)
+    out = []
+    for full in (0, 1):
+        c = api.Config.from_buffer_copy(cfg)
+        c.solid_full_walk = full
+        with api.Simulation(c, pa, device=0) as s:
+            s.step(6 if speed_share == 0.0 else 1)
+            s.sync()
+            out.append({f: s.get(f) for f in ("solid_pos", "solid_vel", "solid_couple_dudt", "fluid_pos")})
+    assert np.any(out[0]["solid_couple_dudt"] != 0.0)
+    for f in out[0]:
+        assert np.array_equal(out[0][f], out[1][f]), f
+
+
+@pytest.mark.parametrize("sub_steps", [1, 2, 3])
+def test_odd_and_even_sub_steps_equal_the_fused_launch(sub_steps):
+    """The force launches advance the solid from buffer to buffer; the fused launch
+    (which walks the fluid in every sub-step) updates it in place."""
+    cfg, pa = cases.make(cases.tiny_box(jitter=0.01, seed=5))
+    cfg.solid_sub_step = sub_steps
+    out = []
+    for fused in (0, 1):
+        c = api.Config.from_buffer_copy(cfg)
+        c.solid_fused = fused
+        with api.Simulation(c, pa, device=0) as s:
+            s.step(3)
+            s.sync()
+            out.append({f: s.get(f) for f in ("solid_pos", "solid_vel", "solid_F", "solid_PK1", "fluid_pos")})
+    for f in out[0]:
+        assert np.array_equal(out[0][f], out[1][f]), f
