@@ -358,6 +358,37 @@ void add_sweep_launch(Plan &pl, ArenaBuilder &ab, const std::vector<Item<FluidSw
     pl.launches.push_back(L);
 }
 
+// The scans of the items' cell counts (blocks per item of the tile passes in sb,
+// of the partials pass in sp; 0: not scanned): one cluster per item, or three
+// passes where an item has too many cells for that.
+void add_scan(Plan &pl, ArenaBuilder &ab, const std::vector<Item<ScanArgs>> &items, const std::vector<int> &sb,
+              const std::vector<int> &sp)
+{
+    std::vector<Item<ScanArgs>> scanned;
+    int most = 0;
+    for (size_t k = 0; k < items.size(); ++k)
+        if (sp[k]) {
+            scanned.push_back(items[k]);
+            most = std::max(most, items[k].A.n);
+        }
+    if (most <= kClusterScanMax) {
+        add_launch(pl, ab, L_SCAN, scanned, std::vector<int>(scanned.size(), 1));
+        return;
+    }
+    add_launch(pl, ab, L_SCAN_REDUCE, items, sb);
+    add_launch(pl, ab, L_SCAN_PARTIALS, items, sp);
+    add_launch(pl, ab, L_SCAN_APPLY, items, sb);
+}
+
+// Put the launches added since `first` on a branch of the step's graph, and have
+// the first of them wait for the branches in `join`.
+void set_branch(Plan &pl, size_t first, int branch, unsigned join = 0)
+{
+    for (size_t k = first; k < pl.launches.size(); ++k) pl.launches[k].branch = branch;
+    if (first < pl.launches.size()) pl.launches[first].join |= join;
+}
+constexpr unsigned branch_bit(int branch) { return 1u << (branch - 1); }
+
 // The cell phase of neighbour-list instances (parity pf -> 1-pf, ps -> 1-ps):
 // the list decision; on a rebuild, the counting sort of fluid and solid on the
 // list grid, else an unpermuted copy; the per-step impact-grid index; on a
@@ -462,6 +493,21 @@ void plan_cell_nl(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, 
     }
     add_launch(pl, ab, L_GATHER_F, gf, gfb);
     add_launch(pl, ab, L_GATHER_S, gs, gsb);
+    // the list build (runs only on a rebuild), beside the index
+    const size_t first_build = pl.launches.size();
+    std::vector<Item<NlBuildArgs>> bi;
+    std::vector<int> bb;
+    for (fsim_sim *h : m) {
+        const NlBuildArgs ba{h->f_x0,   h->f_lcell,  h->f_lstart, mixed ? h->v_abs : h->v_posr, h->v_start,
+                             h->s_x0,   h->s_lstart, h->nf,       h->nl_cap,  h->nl_list,
+                             h->nl_cnt, h->nl_state, h->d_flags,  h->nl_R2s,  h->nv,
+                             h->ns};
+        const Item<NlBuildArgs> bt{h->Pl, ba};
+        bi.push_back(bt);
+        bb.push_back(blocks_for(h->nf, kNlBuildThreads));
+    }
+    add_rebuild_launch(pl, ab, L_NL_BUILD, bi, bb, kRebuildBuildGrid, 1);
+    set_branch(pl, first_build, kBranchBuild);
     // the per-step impact-grid index of the particles as they now lie
     hi.clear();
     si.clear();
@@ -512,9 +558,7 @@ void plan_cell_nl(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, 
     }
     add_launch(pl, ab, L_HASH, hi, hb);
     add_launch(pl, ab, L_HASH_M, hmi, hmb);
-    add_launch(pl, ab, L_SCAN_REDUCE, si, sb);
-    add_launch(pl, ab, L_SCAN_PARTIALS, si, sp);
-    add_launch(pl, ab, L_SCAN_APPLY, si, sb);
+    add_scan(pl, ab, si, sb, sp);
     add_launch(pl, ab, L_SCATTER, ci, cb);
     add_launch(pl, ab, L_RANK_F, ri, rb);
     if (mixed) {
@@ -533,19 +577,6 @@ void plan_cell_nl(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, 
         add_launch(pl, ab, L_CELLREF, cr, crb);
         add_launch(pl, ab, L_MIXED_REC, cr, rcb);
     }
-    // the list build (runs only on a rebuild)
-    std::vector<Item<NlBuildArgs>> bi;
-    std::vector<int> bb;
-    for (fsim_sim *h : m) {
-        const NlBuildArgs ba{h->f_x0,   h->f_lcell,  h->f_lstart, mixed ? h->v_abs : h->v_posr, h->v_start,
-                             h->s_x0,   h->s_lstart, h->nf,       h->nl_cap,  h->nl_list,
-                             h->nl_cnt, h->nl_state, h->d_flags,  h->nl_R2s,  h->nv,
-                             h->ns};
-        const Item<NlBuildArgs> bt{h->Pl, ba};
-        bi.push_back(bt);
-        bb.push_back(blocks_for(h->nf, kNlBuildThreads));
-    }
-    add_rebuild_launch(pl, ab, L_NL_BUILD, bi, bb, kRebuildBuildGrid, 1);
 }
 
 // The cell phase: counting sort of fluid and solid (parity pf -> 1-pf, ps -> 1-ps).
@@ -592,9 +623,7 @@ void plan_cell(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, int
     add_launch(pl, ab, L_ZERO, zi, zb);
     add_launch(pl, ab, L_HASH, hi, hb);
     add_launch(pl, ab, L_HASH_M, hmi, hmb);
-    add_launch(pl, ab, L_SCAN_REDUCE, si, sb);
-    add_launch(pl, ab, L_SCAN_PARTIALS, si, sp);
-    add_launch(pl, ab, L_SCAN_APPLY, si, sb);
+    add_scan(pl, ab, si, sb, sp);
     add_launch(pl, ab, L_SCATTER, ci, cb);
     std::vector<Item<GatherFluidArgs>> gf;
     std::vector<Item<GatherSolidArgs>> gs;
@@ -634,7 +663,9 @@ void plan_couple(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, i
         it.push_back(ci);
         nb.push_back(h->nf && h->ns ? blocks_for((long long)kCoupleGroup * h->ns, kBlock) : 0);
     }
+    const size_t first = pl.launches.size();
     add_launch(pl, ab, m.empty() || !m[0]->mixed ? L_COUPLE : L_COUPLE_M, it, nb);
+    set_branch(pl, first, kBranchCouple);
 }
 
 void plan_virt(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, int pf)
@@ -649,7 +680,10 @@ void plan_virt(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, int
         it.push_back(vi);
         nb.push_back(blocks_for(h->nv, kBlock));
     }
+    // (the build reads the wall positions that the search rewrites)
+    const size_t first = pl.launches.size();
     add_launch(pl, ab, m.empty() || !m[0]->mixed ? L_VIRT : L_VIRT_M, it, nb);
+    set_branch(pl, first, 0, branch_bit(kBranchBuild));
 }
 
 // Lanes that share a particle of the list sweep (log2), by the fluid particles
@@ -724,6 +758,7 @@ void plan_fluid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, in
     if (pl.launches.size() > before) {
         pl.sweep_index = (int)before;
         pl.launches.back().lane_shift = lane_shift;
+        pl.launches.back().join = branch_bit(kBranchBuild) | branch_bit(kBranchCouple);
     }
 }
 
@@ -731,7 +766,9 @@ void plan_fluid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, in
 // per-phase batched launches, or (solid_fused) one persistent cooperative
 // launch for all sub-steps of all instances
 
-void plan_solid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, int pf, int ps)
+// parts: the first deformation (which needs the cell phase only), the rest
+enum { kSolidFirst = 1, kSolidRest = 2 };
+void plan_solid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, int pf, int ps, int parts)
 {
     int max_sub = 0;
     for (fsim_sim *h : m)
@@ -801,17 +838,25 @@ void plan_solid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, in
                 S.vel_out = in_place ? nullptr : h->s_vel[1 - from];
             }
             // sub-step 0 also resolves the step's list slots for the later sub-steps
-            add_launch(pl, ab, mixed ? (k == 0 ? L_DEFORM_M_R : L_DEFORM_M) : (k == 0 ? L_DEFORM_R : L_DEFORM), it,
-                       wb);
+            if (parts & (k == 0 ? kSolidFirst : kSolidRest)) {
+                const size_t first = pl.launches.size();
+                add_launch(pl, ab, mixed ? (k == 0 ? L_DEFORM_M_R : L_DEFORM_M) : (k == 0 ? L_DEFORM_R : L_DEFORM), it,
+                           wb);
+                if (k == 0) set_branch(pl, first, kBranchDeform);
+            }
+            if (!(parts & kSolidRest)) break;
             // sub-step 0 records each lane's fluid list, later sub-steps walk it
             const bool lists = !m[0]->cfg.solid_full_walk;
             const int plain = !lists ? L_FORCE : k == 0 ? L_FORCE_RECORD : L_FORCE_LISTED;
             const int mix = !lists ? L_FORCE_M : k == 0 ? L_FORCE_M_RECORD : L_FORCE_M_LISTED;
+            const size_t force = pl.launches.size();
             add_launch(pl, ab, mixed ? mix : plain, it, wb);
+            if (k == 0) set_branch(pl, force, 0, branch_bit(kBranchDeform) | branch_bit(kBranchCouple));
             add_launch(pl, ab, L_UPDATE, it, ub);
         }
         return;
     }
+    if (!(parts & kSolidRest)) return;
     {
         std::vector<int> eb;
         for (fsim_sim *h : m) eb.push_back(h->ns ? blocks_for(h->s_ne, kBlock) : 0);
@@ -840,6 +885,8 @@ void plan_solid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, in
     pl.launches.push_back(L);
 }
 
+constexpr unsigned kAllPhases = 0x1fu;
+
 // phases: bit k = FSIM_PHASE k
 fsim_status build_plan(const std::vector<fsim_sim *> &m, unsigned phases, int pf, int ps, Plan **out)
 {
@@ -866,13 +913,16 @@ fsim_status build_plan(const std::vector<fsim_sim *> &m, unsigned phases, int pf
         pf ^= 1;
         ps ^= 1;
     }
+    // a whole step: the solid's first deformation does not wait for the fluid
+    const bool ahead = phases == kAllPhases;
+    if (ahead) plan_solid(*pl, ab, m, pf, ps, kSolidFirst);
     if (phases & (1u << FSIM_PHASE_COUPLE)) plan_couple(*pl, ab, m, pf, ps);
     if (phases & (1u << FSIM_PHASE_VIRT)) plan_virt(*pl, ab, m, pf);
     if (phases & (1u << FSIM_PHASE_FLUID)) {
         plan_fluid(*pl, ab, m, pf, ps);
         pf ^= 1;
     }
-    if (phases & (1u << FSIM_PHASE_SOLID)) plan_solid(*pl, ab, m, pf, ps);
+    if (phases & (1u << FSIM_PHASE_SOLID)) plan_solid(*pl, ab, m, pf, ps, ahead ? kSolidRest : kSolidFirst | kSolidRest);
     pl->pf_after = pf;
     pl->ps_after = ps;
     pl->host = ab.bytes;
@@ -890,11 +940,23 @@ fsim_status build_plan(const std::vector<fsim_sim *> &m, unsigned phases, int pf
     return FSIM_OK;
 }
 
+fsim_status open_side_streams(SideStreams &side)
+{
+    for (int b = 0; b < kBranches; ++b) {
+        CK(cudaStreamCreateWithFlags(&side.st[b], cudaStreamNonBlocking));
+        CK(cudaEventCreateWithFlags(&side.fork[b], cudaEventDisableTiming));
+        CK(cudaEventCreateWithFlags(&side.join[b], cudaEventDisableTiming));
+    }
+    return FSIM_OK;
+}
+
 fsim_status capture_plan(Plan &pl, cudaStream_t st, int shape)
 {
     cudaGraph_t graph = nullptr;
+    SideStreams side;
+    if (fsim_status r = open_side_streams(side)) return r;
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    fsim_status s = enqueue_plan(pl, st, shape);
+    fsim_status s = enqueue_plan(pl, st, shape, nullptr, nullptr, nullptr, cudaEventRecordDefault, nullptr, 0, &side);
     cudaError_t e = cudaStreamEndCapture(st, &graph);
     if (s) {
         if (graph) cudaGraphDestroy(graph);
@@ -919,8 +981,11 @@ fsim_status capture_timed_plan(Plan &pl, cudaStream_t st, int shape)
 {
     for (int k = 0; k < 2; ++k)
         if (!pl.tev[k]) CK(cudaEventCreate(&pl.tev[k]));
+    SideStreams side;
+    if (fsim_status r = open_side_streams(side)) return r;
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    fsim_status s = enqueue_plan(pl, st, shape, pl.tev[0], pl.tev[1], nullptr, cudaEventRecordExternal);
+    fsim_status s = enqueue_plan(pl, st, shape, pl.tev[0], pl.tev[1], nullptr, cudaEventRecordExternal,
+                                 nullptr, 0, &side);
     cudaError_t e = cudaStreamEndCapture(st, &pl.tgraph);
     if (s) return s;
     if (e != cudaSuccess) {
@@ -963,8 +1028,6 @@ void after_plan(fsim_sim *h, unsigned phases, const Plan &pl)
     if (phases & (1u << FSIM_PHASE_FLUID)) h->rec_live = false;
     if ((phases & (1u << FSIM_PHASE_SOLID)) && h->ns) h->s_mech_ok = true;
 }
-
-constexpr unsigned kAllPhases = 0x1fu;
 
 fsim_status handle_step_plan(fsim_sim *h, Plan **out)
 {

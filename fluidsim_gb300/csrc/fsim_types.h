@@ -61,6 +61,8 @@ constexpr int kBlock = 256;         // threads per block of the element-wise and
 constexpr int kScanThreads = 1024;  // cell-count scan: threads per block
 constexpr int kScanItems = 4;       //   and counts per thread
 constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr int kScanCluster = 8;     // blocks of a cluster that scans an item's counts alone
+constexpr int kClusterScanChunk = kScanCluster * kScanThreads * 16, kClusterScanMax = 4 * kClusterScanChunk;
 constexpr int kMaxScanTiles = 16384; // cell grids up to 67M cells
 constexpr int kFluidListCap = 48;   // fluid list entries per solid lane
 constexpr int kPLStride = 12;       // floats per particle of the solid's P L^-1 array (16-byte rows)
@@ -481,7 +483,7 @@ constexpr int kNlBuildThreads = 128;
 // instances by one step (or one phase), with every launch's {params, args}
 // items and block prefix tables in one device arena.
 enum LaunchKind {
-    L_ZERO, L_HASH, L_SCAN_REDUCE, L_SCAN_PARTIALS, L_SCAN_APPLY, L_SCATTER, L_GATHER_F, L_GATHER_S,
+    L_ZERO, L_HASH, L_SCAN, L_SCAN_REDUCE, L_SCAN_PARTIALS, L_SCAN_APPLY, L_SCATTER, L_GATHER_F, L_GATHER_S,
     L_COUPLE, L_VIRT, L_SWEEP, L_DEFORM, L_FORCE, L_UPDATE,
     L_HASH_M, L_CELLREF, L_COUPLE_M, L_VIRT_M, L_DEFORM_M, L_FORCE_M, L_SOLID_FUSED, L_SOLID_SLOTS,
     L_FORCE_RECORD, L_FORCE_LISTED, L_FORCE_M_RECORD, L_FORCE_M_LISTED, L_DEFORM_R, L_DEFORM_M_R,
@@ -500,6 +502,8 @@ struct Launch {
     unsigned polls;                       // L_SOLID_FUSED: barrier wait limit, 0 = the default
     const int *act = nullptr;             // launches of the list rebuild: the plan's rebuilding instances
     int per = 1;                          //   and the items each instance has
+    int branch = 0;                       // in a captured step: 0 the main stream, k side stream k - 1
+    unsigned join = 0;                    // side streams (bits) this launch waits for
 };
 
 struct Plan {
@@ -554,6 +558,25 @@ const Item<Args> &host_item(const Plan &pl, const Launch &L)
         }                                                                                                      \
     } while (0)
 
+// Side streams of a step's capture: launches that do not depend on one another
+// become parallel branches of its graph (the list build beside the cell index, the
+// coupling beside the wall search, the solid's first deformation beside all of the
+// fluid).  Outside a capture a plan runs launch by launch on one stream.
+constexpr int kBranches = 3;
+enum { kBranchBuild = 1, kBranchCouple = 2, kBranchDeform = 3 };
+struct SideStreams {
+    cudaStream_t st[kBranches] = {};
+    cudaEvent_t fork[kBranches] = {}, join[kBranches] = {};
+    ~SideStreams()
+    {
+        for (int b = 0; b < kBranches; ++b) {
+            if (st[b]) cudaStreamDestroy(st[b]);
+            if (fork[b]) cudaEventDestroy(fork[b]);
+            if (join[b]) cudaEventDestroy(join[b]);
+        }
+    }
+};
+
 // ---------------------------------------------- entry points of the kernels
 // Enqueue a plan's launches on `st`, the fluid sweep with launch shape
 // `shape`; optional events around the sweep (recorded with sweep_flags:
@@ -561,11 +584,12 @@ const Item<Args> &host_item(const Plan &pl, const Launch &L)
 // per_launch: 2 events per launch, recorded before and after it.
 // tune_ev (the autotuner): instead of one sweep, tune_rounds rounds of one
 // sweep per launch shape, round r shape s between tune_ev[2 (r S + s)] and
-// tune_ev[2 (r S + s) + 1] (S = kSweepShapes).
+// tune_ev[2 (r S + s) + 1] (S = kSweepShapes).  side (a capture): the launches'
+// branches go to these streams.
 fsim_status enqueue_plan(const Plan &pl, cudaStream_t st, int shape, cudaEvent_t sweep0 = nullptr,
                          cudaEvent_t sweep1 = nullptr, const cudaEvent_t *per_launch = nullptr,
                          unsigned sweep_flags = cudaEventRecordDefault, const cudaEvent_t *tune_ev = nullptr,
-                         int tune_rounds = 0);
+                         int tune_rounds = 0, const SideStreams *side = nullptr);
 // the FSIM_PHASE_* a launch kind belongs to
 int launch_phase(int kind);
 // CTAs of the fused solid kernel that fit on the current device at once (<= want)

@@ -145,3 +145,22 @@ def test_odd_and_even_sub_steps_equal_the_fused_launch(sub_steps):
             out.append({f: s.get(f) for f in ("solid_pos", "solid_vel", "solid_F", "solid_PK1", "fluid_pos")})
     for f in out[0]:
         assert np.array_equal(out[0][f], out[1][f]), f
+
+
+@pytest.mark.parametrize("tank", [(30, 20, 20), (300, 100, 100), (600, 150, 150)])
+@pytest.mark.parametrize("skin", [0.15, 0.0])
+def test_cell_starts_of_every_scan(tank, skin):
+    """Cell grids of one and two chunks of the cluster scan (131,072 counts each) and
+    beyond its limit (524,288): neighbour counts by the cell walk equal the oracle's."""
+    cfg, pa = _box((9, 8, 7), tank=tank, layers=0)
+    cfg.neighbor_skin = skin
+    # particles in the last cells too: the carry across chunks counts
+    pos = pa.fluid_pos.copy()
+    pos[::2] += np.float32(0.01) * (np.array(tank, np.float32) - np.array([9, 8, 7], np.float32))
+    pa = api.ParticleArrays(pos, pa.fluid_vel, pa.fluid_rho, pa.fluid_p, pa.solid_pos, pa.solid_vel,
+                            pa.solid_ref_pos, pa.solid_type, pa.virt_pos)
+    ref = orc.OracleSim(cfg, pa, "f64")
+    ref.phase(api.PHASE_CELL)
+    with api.Simulation(cfg, pa, device=0) as sim:
+        sim.phase(api.PHASE_CELL)
+        assert np.array_equal(sim.neighbor_counts(), ref.neighbor_counts())
