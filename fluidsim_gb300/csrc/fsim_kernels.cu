@@ -1052,7 +1052,17 @@ __device__ __forceinline__ void nl_gather(const DevParams &P, const NlBuildArgs 
     }
 }
 
-__device__ __forceinline__ void nl_build_body(const DevParams &P, const NlBuildArgs &A, int blk)
+// Particle i's entry counts (v0, s0: where its wall and solid entries begin).
+__device__ __forceinline__ void nl_store_counts(const NlBuildArgs &A, int i, int nf, int v0, int nv, int s0, int ns)
+{
+    A.cnt[i] = make_int2(min(nf, A.cap), max(min(nv, A.cap - v0), 0) | max(min(ns, A.cap - s0), 0) << 16);
+    if (nf + nv + ns > A.cap - kNlPad) {
+        atomicAdd(&A.nl->overflow, 1);
+        atomicOr(A.flags, FLAG_LIST_OVERFLOW);
+    }
+}
+
+__device__ __forceinline__ void nl_build_lanes(const DevParams &P, const NlBuildArgs &A, int blk)
 {
     __shared__ int rings[kNlBuildWarps][kNlBuildRing][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1084,14 +1094,67 @@ __device__ __forceinline__ void nl_build_body(const DevParams &P, const NlBuildA
     const int ns = tot - s0;
     if (tot % kNlGroup) nl_store_group(A, ring, lane, i, tot / kNlGroup, tot);
     if (!valid) return;
-    A.cnt[i] = make_int2(min(nf, A.cap), max(min(nv, A.cap - v0), 0) | max(min(ns, A.cap - s0), 0) << 16);
-    if (nf + nv + ns > A.cap - kNlPad) {
-        atomicAdd(&A.nl->overflow, 1);
-        atomicOr(A.flags, FLAG_LIST_OVERFLOW);
-    }
+    nl_store_counts(A, i, nf, v0, nv, s0, ns);
 }
 
-FSIM_REBUILD_KERNEL(kg_nl_build, NlBuildArgs, nl_build_body, kNlBuildWarps * 32, blocks_for(A.n, kNlBuildThreads))
+// The same list built by a warp per particle: lanes 0..26 read the three
+// species' row ranges, then the lanes test 32 candidates of a row at once and
+// the hits of a ballot are stored in candidate order.  For instances too small to
+// fill the GPU with a lane per particle, where the build is the latency of one
+// lane's 730 candidates.
+__device__ __forceinline__ void nl_build_warp(const DevParams &P, const NlBuildArgs &A, int blk)
+{
+    const int lane = threadIdx.x & 31, i = blk * kNlBuildWarps + (int)(threadIdx.x >> 5);
+    if (i >= A.n) return; // whole warp
+    const float4 pr = A.posr[i];
+    const int cell = A.cell_f[i];
+    const int row = cell / P.nz, cz = cell - row * P.nz, cx = row / P.ny, cy = row - cx * P.ny;
+    int b = 0, e = 0;
+    if (lane < 27) {
+        const int *__restrict__ start = lane < 9 ? A.start_f : lane < 18 ? A.start_v : A.start_s;
+        const int x = cx + lane % 9 / 3 - 1, y = cy + lane % 3 - 1;
+        if (x >= 0 && x < P.nx && y >= 0 && y < P.ny) {
+            const int base = (x * P.ny + y) * P.nz;
+            b = start[base + max(cz - 1, 0)];
+            e = start[base + min(cz + 1, P.nz - 1) + 1];
+        }
+    }
+    int tot = 0, begin[3], count[3];
+#pragma unroll
+    for (int sp = 0; sp < 3; ++sp) {
+        const float4 *__restrict__ pos = sp == 0 ? A.posr : sp == 1 ? A.v_posr : A.s_pos;
+        begin[sp] = tot;
+        for (int r = 0; r < 9; ++r) {
+            const int je = __shfl_sync(kFull, e, 9 * sp + r);
+            for (int j0 = __shfl_sync(kFull, b, 9 * sp + r); j0 < je; j0 += 32) {
+                const int j = j0 + lane;
+                const float4 q = pos[min(j, je - 1)];
+                const bool hit = j < je && dist2(q.x - pr.x, q.y - pr.y, q.z - pr.z) < A.R2s;
+                const unsigned hits = __ballot_sync(kFull, hit);
+                const int k = tot + __popc(hits & ((1u << lane) - 1u));
+                if (hit && k < A.cap) A.list[((size_t)(k / kNlGroup) * A.n + i) * kNlGroup + k % kNlGroup] = j;
+                tot += __popc(hits);
+            }
+        }
+        count[sp] = tot - begin[sp];
+        const int end = (tot + kNlGroup - 1) / kNlGroup * kNlGroup;
+        if (sp == 0 && tot + lane < end && tot + lane < A.cap) // the last fluid group filled up with the particle
+            A.list[((size_t)((tot + lane) / kNlGroup) * A.n + i) * kNlGroup + (tot + lane) % kNlGroup] = i;
+        tot = end;
+    }
+    if (lane == 0) nl_store_counts(A, i, count[0], begin[1], count[1], begin[2], count[2]);
+}
+
+__device__ __forceinline__ int nl_build_blocks(int n)
+{
+    return n <= kNlWarpBuildMax ? blocks_for(n, kNlBuildWarps) : blocks_for(n, kNlBuildThreads);
+}
+__device__ __forceinline__ void nl_build_body(const DevParams &P, const NlBuildArgs &A, int blk)
+{
+    if (A.n <= kNlWarpBuildMax) nl_build_warp(P, A, blk);
+    else nl_build_lanes(P, A, blk);
+}
+FSIM_REBUILD_KERNEL(kg_nl_build, NlBuildArgs, nl_build_body, kNlBuildWarps * 32, nl_build_blocks(A.n))
 
 // The list sweep: every particle's list in order (fluid, then wall, then solid
 // entries, as the stream sweep sums them), r^2 < R^2, the Riemann pair terms, then

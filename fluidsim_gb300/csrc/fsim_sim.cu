@@ -504,7 +504,7 @@ void plan_cell_nl(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, 
                              h->ns};
         const Item<NlBuildArgs> bt{h->Pl, ba};
         bi.push_back(bt);
-        bb.push_back(blocks_for(h->nf, kNlBuildThreads));
+        bb.push_back(blocks_for(h->nf, h->nf <= kNlWarpBuildMax ? kNlBuildThreads / 32 : kNlBuildThreads));
     }
     add_rebuild_launch(pl, ab, L_NL_BUILD, bi, bb, kRebuildBuildGrid, 1);
     set_branch(pl, first_build, kBranchBuild);
@@ -2472,7 +2472,7 @@ fsim_status nl_restore(fsim_sim *h)
                                                                   h->v_start, h->s_x0, h->s_lstart, h->nf, h->nl_cap,
                                                                   h->nl_list, h->nl_cnt, h->nl_state, h->d_flags,
                                                                   h->nl_R2s, h->nv, h->ns}}},
-               {blocks_for(h->nf, kNlBuildThreads)}, kRebuildBuildGrid, 1);
+               {blocks_for(h->nf, h->nf <= kNlWarpBuildMax ? kNlBuildThreads / 32 : kNlBuildThreads)}, kRebuildBuildGrid, 1);
     pl.host = ab.bytes;
     cudaError_t e = cudaMalloc((void **)&pl.arena, std::max<size_t>(ab.bytes.size(), 1));
     if (e == cudaSuccess) e = cudaMemcpy(pl.act, only, sizeof only, cudaMemcpyHostToDevice);
