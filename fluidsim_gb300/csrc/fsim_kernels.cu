@@ -3347,6 +3347,40 @@ __global__ void k_offsets_in_cells(const DevParams P, float4 *__restrict__ pos, 
     p.z = (float)((double)p.z - cell_corner(P, 2, cz));
     pos[s] = p;
 }
+// absolute position, density and pressure of a mixed-form particle, and back
+__device__ __forceinline__ float4 mixed_position(const DevParams &P, float4 off, int cell)
+{
+    int cx, cy, cz;
+    cell_xyz(P, cell, cx, cy, cz);
+    return make_float4((float)(cell_corner(P, 0, cx) + (double)off.x), (float)(cell_corner(P, 1, cy) + (double)off.y),
+                       (float)(cell_corner(P, 2, cz) + (double)off.z), 0.0f);
+}
+__device__ __forceinline__ float mixed_density(const DevParams &P, float delta)
+{
+    return (float)((double)P.rho0 * (1.0 + (double)delta));
+}
+__device__ __forceinline__ float mixed_pressure(const DevParams &P, float delta)
+{
+    const double pr = (double)P.rho2p * expm1((double)P.gamma * log1p((double)delta));
+    return (float)fmax(pr, (double)P.min_p);
+}
+__device__ __forceinline__ float4 mixed_offset(const DevParams &P, float x, float y, float z, float w, int cell)
+{
+    int cx, cy, cz;
+    cell_xyz(P, cell, cx, cy, cz);
+    return make_float4((float)((double)x - cell_corner(P, 0, cx)), (float)((double)y - cell_corner(P, 1, cy)),
+                       (float)((double)z - cell_corner(P, 2, cz)), w);
+}
+__device__ __forceinline__ float mixed_delta(const DevParams &P, float rho)
+{
+    return (float)((double)rho / (double)P.rho0 - 1.0);
+}
+__device__ __forceinline__ void store3(float *out, size_t i, float4 v)
+{
+    out[3 * i] = v.x;
+    out[3 * i + 1] = v.y;
+    out[3 * i + 2] = v.z;
+}
 // out[orig[s]] = absolute position / density / pressure of a mixed-form particle
 __global__ void k_unpermute_mixed(const DevParams P, const float4 *__restrict__ pos, const float4 *__restrict__ velp,
                                   const int *__restrict__ cell, const int *__restrict__ orig, int n, int what,
@@ -3355,22 +3389,8 @@ __global__ void k_unpermute_mixed(const DevParams P, const float4 *__restrict__ 
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const int o = orig[s];
-    if (what == MF_POS) {
-        const float4 p = pos[s];
-        int cx, cy, cz;
-        cell_xyz(P, cell[s], cx, cy, cz);
-        out[3 * o] = (float)(cell_corner(P, 0, cx) + (double)p.x);
-        out[3 * o + 1] = (float)(cell_corner(P, 1, cy) + (double)p.y);
-        out[3 * o + 2] = (float)(cell_corner(P, 2, cz) + (double)p.z);
-    } else {
-        const double d = (double)velp[s].w;
-        if (what == MF_RHO) {
-            out[o] = (float)((double)P.rho0 * (1.0 + d));
-        } else {
-            const double pr = (double)P.rho2p * expm1((double)P.gamma * log1p(d));
-            out[o] = (float)fmax(pr, (double)P.min_p);
-        }
-    }
+    if (what == MF_POS) store3(out, o, mixed_position(P, pos[s], cell[s]));
+    else out[o] = what == MF_RHO ? mixed_density(P, velp[s].w) : mixed_pressure(P, velp[s].w);
 }
 // set a mixed-form position (offset from the particle's current cell) or density
 __global__ void k_permute_in_mixed(const DevParams P, float4 *__restrict__ pos, float4 *__restrict__ velp,
@@ -3380,17 +3400,85 @@ __global__ void k_permute_in_mixed(const DevParams P, float4 *__restrict__ pos, 
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const int o = orig[s];
-    if (what == MF_POS) {
-        float4 p = pos[s];
-        int cx, cy, cz;
-        cell_xyz(P, cell[s], cx, cy, cz);
-        p.x = (float)((double)in[3 * o] - cell_corner(P, 0, cx));
-        p.y = (float)((double)in[3 * o + 1] - cell_corner(P, 1, cy));
-        p.z = (float)((double)in[3 * o + 2] - cell_corner(P, 2, cz));
-        pos[s] = p;
-    } else {
-        velp[s].w = (float)((double)in[o] / (double)P.rho0 - 1.0);
+    if (what == MF_POS) pos[s] = mixed_offset(P, in[3 * o], in[3 * o + 1], in[3 * o + 2], pos[s].w, cell[s]);
+    else velp[s].w = mixed_delta(P, in[o]);
+}
+
+// The whole state at once, in input order, for callers that move several fields
+// (the pointers of the others are nullptr): one pass over each species instead
+// of one launch and pass per field.
+__global__ void k_state_out(const DevParams P, const StateArgs A)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int s = t - A.fluid_threads;
+    if (t < A.nf) {
+        const size_t o = A.forig[t];
+        const float4 q = A.fpos[t], u = A.fvel[t];
+        if (A.field[SF_POS]) store3(A.field[SF_POS], o, P.mixed ? mixed_position(P, q, A.fcell[t]) : q);
+        if (A.field[SF_VEL]) store3(A.field[SF_VEL], o, u);
+        if (A.field[SF_RHO]) A.field[SF_RHO][o] = P.mixed ? mixed_density(P, u.w) : q.w;
+        if (A.field[SF_P]) A.field[SF_P][o] = P.mixed ? mixed_pressure(P, u.w) : u.w;
+    } else if (s >= 0 && s < A.ns) {
+        const size_t o = A.sorig[s];
+        if (A.field[SF_SOLID_POS]) store3(A.field[SF_SOLID_POS], o, A.spos[s]);
+        if (A.field[SF_SOLID_VEL]) store3(A.field[SF_SOLID_VEL], o, A.svel[s]);
     }
+}
+// Words copied between several pairs of buffers in one launch (one of each pair
+// in mapped host memory): blockIdx.y is the pair.  A cudaMemcpyAsync per field
+// costs its engine's start-up and 2-4 us of host time each.
+__global__ void k_copy_fields(const CopyArgs A)
+{
+    const CopyArgs::Pair &p = A.pair[blockIdx.y];
+    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x, n = gridDim.x * (size_t)blockDim.x;
+    if (p.wide) {
+        for (size_t k = i; k < p.words / 4; k += n)
+            reinterpret_cast<uint4 *>(p.dst)[k] = reinterpret_cast<const uint4 *>(p.src)[k];
+        if (i < p.words % 4) p.dst[p.words / 4 * 4 + i] = p.src[p.words / 4 * 4 + i];
+    } else {
+        for (size_t k = i; k < p.words; k += n) p.dst[k] = p.src[k];
+    }
+}
+// The same into the state; new fluid positions fold their squared displacement
+// since the last list build into the instance's maximum (nl, as k_nl_displacement).
+__global__ void k_state_in(const DevParams P, const StateArgs A)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int s = t - A.fluid_threads;
+    unsigned d2 = 0u;
+    if (t < A.nf) {
+        const size_t o = A.forig[t];
+        float4 q = A.fpos[t], u = A.fvel[t];
+        if (const float *x = A.field[SF_POS])
+            q = P.mixed ? mixed_offset(P, x[3 * o], x[3 * o + 1], x[3 * o + 2], q.w, A.fcell[t])
+                        : make_float4(x[3 * o], x[3 * o + 1], x[3 * o + 2], q.w);
+        if (const float *x = A.field[SF_VEL]) u = make_float4(x[3 * o], x[3 * o + 1], x[3 * o + 2], u.w);
+        if (A.field[SF_RHO]) {
+            if (P.mixed) u.w = mixed_delta(P, A.field[SF_RHO][o]);
+            else q.w = A.field[SF_RHO][o];
+        }
+        if (A.field[SF_P]) u.w = A.field[SF_P][o]; // plain form only
+        A.fpos[t] = q;
+        A.fvel[t] = u;
+        if (A.nl && A.field[SF_POS]) {
+            float4 p = q;
+            if (P.mixed) {
+                int cx, cy, cz;
+                cell_xyz(P, A.fcell[t], cx, cy, cz);
+                p = mixed_abs(P, p, cx, cy, cz, 0.0f);
+            }
+            const float4 x0 = A.x0[t];
+            d2 = __float_as_uint(dist2(p.x - x0.x, p.y - x0.y, p.z - x0.z));
+        }
+    } else if (s >= 0 && s < A.ns) {
+        const size_t o = A.sorig[s];
+        if (const float *x = A.field[SF_SOLID_POS])
+            A.spos[s] = make_float4(x[3 * o], x[3 * o + 1], x[3 * o + 2], A.spos[s].w);
+        if (const float *x = A.field[SF_SOLID_VEL])
+            A.svel[s] = make_float4(x[3 * o], x[3 * o + 1], x[3 * o + 2], A.svel[s].w);
+    }
+    d2 = __reduce_max_sync(kFull, d2);
+    if ((threadIdx.x & 31) == 0 && d2) atomicMax(&A.nl->maxd2, d2);
 }
 
 // ------------------------------------------------- conservation (FP64)
@@ -3790,6 +3878,19 @@ void launch_k_permute_in_mixed(int grid, cudaStream_t st, const DevParams P, flo
 void launch_k_permute_in_f4(int grid, cudaStream_t st, float4 *dst, const int *orig, int n, int comp, int width, const float *in)
 {
     k_permute_in_f4<<<grid, kBlock, 0, st>>>(dst, orig, n, comp, width, in);
+}
+
+void launch_k_state(cudaStream_t st, const DevParams P, const StateArgs A, bool in)
+{
+    const int grid = (A.fluid_threads + A.ns + kBlock - 1) / kBlock;
+    if (in) k_state_in<<<grid, kBlock, 0, st>>>(P, A);
+    else k_state_out<<<grid, kBlock, 0, st>>>(P, A);
+}
+
+void launch_k_copy_fields(cudaStream_t st, const CopyArgs A, int pairs, size_t most_words)
+{
+    const size_t blocks = (most_words / 4 + kBlock) / kBlock;
+    k_copy_fields<<<dim3((unsigned)std::min<size_t>(blocks, 304), pairs), kBlock, 0, st>>>(A);
 }
 
 void launch_k_probe(int grid, cudaStream_t st, const DevParams P, const ProbeArgs A)

@@ -1840,6 +1840,22 @@ fsim_status set_target(fsim_sim *h, int field, float4 **dst, const int **orig, i
     return FSIM_OK;
 }
 
+// After state fields were set: what is kept beside the fluid state follows it.
+fsim_status refresh_copies(fsim_sim *h, bool fluid_pos, bool fluid)
+{
+    const int n = h->nf;
+    if (h->nl && fluid_pos && h->f_sorted) { // the index's position copy
+        launch_k_gather_f4(blocks_for(n, kBlock), h->stream, h->f_ids, h->f_posr[h->f_cur], n, h->f_spos);
+        CK_LAUNCH();
+    }
+    if (h->nl && fluid && h->rec_live) { // between the cell and fluid phases: the records
+        launch_k_pack_records(blocks_for(n, kBlock), h->stream, h->f_posr[h->f_cur], h->f_velp[h->f_cur],
+                              h->mixed ? h->f_cxyz : nullptr, n, h->f_rec);
+        CK_LAUNCH();
+    }
+    return FSIM_OK;
+}
+
 // Enqueue on the handle's stream the kernel that scatters `field` (input
 // order, device memory `stg`) into the state (n > 0).  New fluid positions of
 // a neighbour-list instance count as displacement since the last list build
@@ -1865,16 +1881,7 @@ fsim_status enqueue_permute_in(fsim_sim *h, int field, int n, const float *stg)
                                  n, h->nl_state);
         CK_LAUNCH();
     }
-    if (h->nl && field == FSIM_FLUID_POS && h->f_sorted) { // the index's position copy follows the state
-        launch_k_gather_f4(blocks_for(n, kBlock), h->stream, h->f_ids, h->f_posr[h->f_cur], n, h->f_spos);
-        CK_LAUNCH();
-    }
-    if (h->nl && field < 10 && h->rec_live) { // between the cell and fluid phases: records follow the state
-        launch_k_pack_records(blocks_for(n, kBlock), h->stream, h->f_posr[h->f_cur], h->f_velp[h->f_cur],
-                              h->mixed ? h->f_cxyz : nullptr, n, h->f_rec);
-        CK_LAUNCH();
-    }
-    return FSIM_OK;
+    return refresh_copies(h, field == FSIM_FLUID_POS, field < 10);
 }
 } // namespace
 
@@ -1924,6 +1931,103 @@ fsim_status bulk_reserve(fsim_sim *h, size_t bytes, int nev)
 }
 } // namespace
 
+namespace {
+// Up to this many bytes the fields of a call move through one kernel over the
+// state and, to or from page-locked host memory, one that copies them all: with a
+// launch, an event, a stream switch and a copy per field they were host and launch
+// latency (42 us to read and 51 us to write the six fields of 32,000 particles).
+// Above, the copies of the first fields overlap the kernels of the later ones.
+constexpr size_t kStateBytes = 4u << 20;
+
+// Enqueue the copies of a call's fields between the bulk buffer and host memory:
+// one kernel if all host buffers are page-locked and mapped (so the device can
+// address them) and word-aligned, else one copy per field.
+fsim_status copy_fields(fsim_sim *h, int nfields, void *const *host, const size_t *bytes, bool to_host)
+{
+    CopyArgs C{};
+    int pairs = 0;
+    size_t off = 0, most = 0;
+    bool direct = true;
+    for (int k = 0; k < nfields && direct; ++k) {
+        if (!bytes[k]) continue;
+        cudaPointerAttributes at{};
+        direct = reinterpret_cast<uintptr_t>(host[k]) % 4 == 0 &&
+                 cudaPointerGetAttributes(&at, host[k]) == cudaSuccess && at.type == cudaMemoryTypeHost &&
+                 at.devicePointer;
+        // the whole buffer must lie in page-locked memory: its last word too
+        cudaPointerAttributes end{};
+        const char *last = static_cast<const char *>(host[k]) + bytes[k] - 4;
+        direct = direct && cudaPointerGetAttributes(&end, last) == cudaSuccess && end.type == cudaMemoryTypeHost &&
+                 static_cast<const char *>(end.devicePointer) - static_cast<const char *>(at.devicePointer) ==
+                     (ptrdiff_t)(bytes[k] - 4);
+        if (!direct) break;
+        unsigned *dev = reinterpret_cast<unsigned *>(static_cast<char *>(h->bulk) + off);
+        unsigned *mapped = static_cast<unsigned *>(at.devicePointer);
+        CopyArgs::Pair &p = C.pair[pairs++];
+        p.dst = to_host ? mapped : dev;
+        p.src = to_host ? dev : mapped;
+        p.words = bytes[k] / 4;
+        p.wide = reinterpret_cast<uintptr_t>(mapped) % 16 == 0;
+        most = std::max(most, p.words);
+        off += (bytes[k] + 255) & ~size_t(255);
+    }
+    if (direct) {
+        launch_k_copy_fields(h->stream, C, pairs, most);
+        CK_LAUNCH();
+        return FSIM_OK;
+    }
+    cudaGetLastError(); // a pageable buffer's query may have failed
+    off = 0;
+    for (int k = 0; k < nfields; ++k) {
+        if (!bytes[k]) continue;
+        char *dev = static_cast<char *>(h->bulk) + off;
+        if (to_host) CK(cudaMemcpyAsync(host[k], dev, bytes[k], cudaMemcpyDeviceToHost, h->stream));
+        else CK(cudaMemcpyAsync(dev, host[k], bytes[k], cudaMemcpyHostToDevice, h->stream));
+        off += (bytes[k] + 255) & ~size_t(255);
+    }
+    return FSIM_OK;
+}
+
+// The StateArgs of a call that moves distinct state fields, their buffers in
+// `bulk`; false when some field is of another kind or asked for twice.
+bool state_args(fsim_sim *h, int nfields, const int *fields, const size_t *bytes, StateArgs &A)
+{
+    A = StateArgs{};
+    size_t off = 0;
+    for (int k = 0; k < nfields; ++k) {
+        int f;
+        switch (fields[k]) {
+        case FSIM_FLUID_POS: f = SF_POS; break;
+        case FSIM_FLUID_VEL: f = SF_VEL; break;
+        case FSIM_FLUID_RHO: f = SF_RHO; break;
+        case FSIM_FLUID_P: f = SF_P; break;
+        case FSIM_SOLID_POS: f = SF_SOLID_POS; break;
+        case FSIM_SOLID_VEL: f = SF_SOLID_VEL; break;
+        default: return false;
+        }
+        if (A.field[f]) return false;
+        if (!bytes[k]) continue;
+        A.field[f] = reinterpret_cast<float *>(static_cast<char *>(h->bulk) + off);
+        off += (bytes[k] + 255) & ~size_t(255);
+    }
+    const bool fluid = A.field[SF_POS] || A.field[SF_VEL] || A.field[SF_RHO] || A.field[SF_P];
+    const bool solid = A.field[SF_SOLID_POS] || A.field[SF_SOLID_VEL];
+    A.fpos = h->f_posr[h->f_cur];
+    A.fvel = h->f_velp[h->f_cur];
+    A.forig = h->f_orig[h->f_cur];
+    A.fcell = h->f_cell;
+    A.spos = h->s_pos[h->s_cur];
+    A.svel = h->s_vel[h->s_cur];
+    A.sorig = h->s_orig[h->s_cur];
+    A.x0 = h->f_x0;
+    A.nl = h->nl ? h->nl_state : nullptr;
+    A.nf = fluid ? h->nf : 0;
+    A.ns = solid ? h->ns : 0;
+    A.fluid_threads = blocks_for(A.nf, kBlock) * kBlock;
+    return off > 0;
+}
+} // namespace
+
 extern "C" fsim_status fsim_get_fields(fsim_handle h, int nfields, const int *fields, void *const *dst,
                                        const size_t *bytes)
 {
@@ -1942,6 +2046,14 @@ extern "C" fsim_status fsim_get_fields(fsim_handle h, int nfields, const int *fi
     fsim_status st = bulk_reserve(h, total, nfields);
     if (st) return st;
     size_t off = 0;
+    StateArgs A;
+    if (total <= kStateBytes && state_args(h, nfields, fields, bytes, A)) {
+        launch_k_state(h->stream, h->P, A, false);
+        CK_LAUNCH();
+        if ((st = copy_fields(h, nfields, dst, bytes, true))) return st;
+        CK(cudaStreamSynchronize(h->stream));
+        return FSIM_OK;
+    }
     for (int k = 0; k < nfields; ++k) {
         if (!counts[k]) continue;
         float *stg = reinterpret_cast<float *>(static_cast<char *>(h->bulk) + off);
@@ -1976,6 +2088,17 @@ extern "C" fsim_status fsim_set_fields(fsim_handle h, int nfields, const int *fi
     DeviceGuard guard(h->device);
     fsim_status st = bulk_reserve(h, total, nfields);
     if (st) return st;
+    StateArgs A;
+    if (total <= kStateBytes && state_args(h, nfields, fields, bytes, A)) {
+        if ((st = copy_fields(h, nfields, const_cast<void *const *>(src), bytes, false))) return st;
+        CK(cudaEventRecord(h->xfer_events[0], h->stream));
+        launch_k_state(h->stream, h->P, A, true);
+        CK_LAUNCH();
+        if ((st = refresh_copies(h, A.field[SF_POS], A.nf > 0))) return st;
+        CK(cudaEventSynchronize(h->xfer_events[0])); // the host buffers may be reused on return
+        if (h->batch) CK(cudaStreamSynchronize(h->stream));
+        return FSIM_OK;
+    }
     // the copies start after the handle's queued work (they overwrite the bulk buffer)
     CK(cudaEventRecord(h->ev1, h->stream));
     CK(cudaStreamWaitEvent(h->copy_stream, h->ev1, 0));

@@ -449,6 +449,28 @@ struct GridBarrier {
     unsigned count, gen;
 };
 
+// Several state fields at once (k_state_out / k_state_in): device buffers in
+// input order per StateField (nullptr: not moved), and the state they belong to.
+enum StateField { SF_POS, SF_VEL, SF_RHO, SF_P, SF_SOLID_POS, SF_SOLID_VEL, SF_COUNT };
+struct StateArgs {
+    float *field[SF_COUNT];
+    float4 *fpos, *fvel, *spos, *svel;
+    const int *forig, *fcell, *sorig;
+    const float4 *x0; // list instances: positions at the last build
+    NlState *nl;
+    int nf, ns, fluid_threads; // threads of the fluid (whole blocks) before the solid's
+};
+
+// buffer pairs of k_copy_fields; wide: both sides 16-byte aligned
+struct CopyArgs {
+    struct Pair {
+        unsigned *dst;
+        const unsigned *src;
+        size_t words;
+        int wide;
+    } pair[SF_COUNT];
+};
+
 // what the mixed-form field (un)permutes move
 enum MixedField { MF_POS = 0, MF_RHO = 1, MF_P = 2 };
 
@@ -608,6 +630,8 @@ void launch_k_unpermute_f4(int grid, cudaStream_t st, const float4 *src, const i
 void launch_k_unpermute_words(int grid, cudaStream_t st, const int *src, const int *orig, int n, int width, int *out);
 void launch_k_permute_in_mixed(int grid, cudaStream_t st, const DevParams P, float4 *pos, float4 *velp, const int *cell, const int *orig, int n, int what, const float *in);
 void launch_k_permute_in_f4(int grid, cudaStream_t st, float4 *dst, const int *orig, int n, int comp, int width, const float *in);
+void launch_k_state(cudaStream_t st, const DevParams P, const StateArgs A, bool in);
+void launch_k_copy_fields(cudaStream_t st, const CopyArgs A, int pairs, size_t most_words);
 void launch_k_probe(int grid, cudaStream_t st, const DevParams P, const ProbeArgs A);
 void launch_k_neighbor_counts(int grid, cudaStream_t st, const DevParams P, const DevParams Pv, const float4 *fposr, const int *cell_f, const int *start_f, const int *ids_f, const float4 *s_pos, const int *start_s, const int *ids_s, const float4 *v_posr, const int *start_v, int *out, int n);
 void launch_k_neighbor_counts_nl(int grid, cudaStream_t st, const DevParams P, const float4 *fposr, const int *list, const int2 *cnt, const float4 *s_pos, const float4 *v_posr, int *out, int n);

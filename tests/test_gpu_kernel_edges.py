@@ -164,3 +164,48 @@ def test_cell_starts_of_every_scan(tank, skin):
     with api.Simulation(cfg, pa, device=0) as sim:
         sim.phase(api.PHASE_CELL)
         assert np.array_equal(sim.neighbor_counts(), ref.neighbor_counts())
+
+
+def _host_views(sim, names, pinned, shift):
+    """A float32 view per field in one host buffer, each `shift` bytes past a 16-byte boundary."""
+    sizes = [int(np.prod(sim.get(k).shape)) for k in names]
+    total = sum(4 * n + 32 for n in sizes)
+    owner = api.PinnedBuffer((total,), np.uint8) if pinned else np.zeros(total + 64, np.uint8)
+    raw = owner.array if pinned else owner
+    at = -raw.ctypes.data % 16
+    views = []
+    for n in sizes:
+        views.append(raw[at + shift:at + shift + 4 * n])
+        at += (4 * n + shift + 15) // 16 * 16
+    return owner, views
+
+
+@pytest.mark.parametrize("precision", [api.PRECISION_FP32, api.PRECISION_MIXED])
+@pytest.mark.parametrize("pinned,shift", [(True, 0), (True, 4), (True, 2), (False, 0), (False, 2)])
+def test_fields_together_equal_fields_one_by_one(precision, pinned, shift):
+    """Page-locked buffers move through one copy kernel (16-byte or 4-byte words), other
+    buffers and odd alignments through one copy per field: the same bytes either way."""
+    cfg, pa = _box((9, 7, 5), precision=precision)
+    names = ("solid_vel", "fluid_p", "fluid_pos", "fluid_rho", "solid_pos", "fluid_vel")
+    with api.Simulation(cfg, pa, device=0) as a, api.Simulation(cfg, pa, device=0) as b:
+        for s in (a, b):
+            s.step(3)
+        owner, views = _host_views(a, names, pinned, shift)
+        ptrs, sizes = [v.ctypes.data for v in views], [v.nbytes for v in views]
+        a.get_many_ptr(names, ptrs, sizes)
+        for k, v in zip(names, views):
+            assert v.tobytes() == a.get(k).tobytes(), k
+        # write back a moved state, together into a and one by one into b
+        take = [k for k in range(len(names)) if precision == api.PRECISION_FP32 or names[k] != "fluid_p"]
+        for k in take:
+            if names[k] == "fluid_vel":
+                views[k][:] = np.frombuffer((np.frombuffer(views[k].tobytes(), np.float32) * 2).tobytes(), np.uint8)
+        a.set_many_ptr([names[k] for k in take], [ptrs[k] for k in take], [sizes[k] for k in take])
+        for k in take:
+            b.set(names[k], np.frombuffer(views[k].tobytes(), np.float32))
+        for s in (a, b):
+            s.step(2)
+            s.sync()
+        for k in names:
+            assert np.array_equal(a.get(k), b.get(k)), k
+        del views, owner
