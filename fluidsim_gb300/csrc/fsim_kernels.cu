@@ -2407,8 +2407,11 @@ __device__ __forceinline__ void solid_deform_body(const DevParams &P, const Soli
     M3 F, L;
 #pragma unroll
     for (int k = 0; k < 9; ++k) F.m[k] = L.m[k] = 0.0f;
+    float4 xi, ri, vi;
     if (valid) {
-        const float4 xi = S.pos[i], ri = S.ref[i];
+        xi = S.pos[i];
+        ri = S.ref[i];
+        vi = S.vel[i];
         const int o = S.orig[i];
         const unsigned ci = RESOLVE ? S.cxyz[i] : 0u;
         // kSolidAhead entries' loads are in flight together (one at a time, the chain
@@ -2530,12 +2533,14 @@ __device__ __forceinline__ void solid_deform_body(const DevParams &P, const Soli
     float4 *pl = reinterpret_cast<float4 *>(S.PL + kPLStride * i);
     pl[0] = make_float4(PL.m[0], PL.m[1], PL.m[2], PL.m[3]);
     pl[1] = make_float4(PL.m[4], PL.m[5], PL.m[6], PL.m[7]);
-    pl[2] = make_float4(PL.m[8], 0.0f, 0.0f, 0.0f);
+    pl[2] = make_float4(PL.m[8], ri.x, ri.y, ri.z);
+    pl[3] = make_float4(xi.x, xi.y, xi.z, vi.x);
+    pl[4] = make_float4(vi.y, vi.z, 0.0f, 0.0f);
 }
-FSIM_BATCHED_KERNEL(kb_solid_deform, SolidArgs, solid_deform_body<false>, kBlock)
-FSIM_BATCHED_KERNEL(kb_solid_deform_mixed, SolidArgs, solid_deform_body<true>, kBlock)
-FSIM_BATCHED_KERNEL(kb_solid_deform_resolve, SolidArgs, (solid_deform_body<false, true>), kBlock)
-FSIM_BATCHED_KERNEL(kb_solid_deform_mixed_resolve, SolidArgs, (solid_deform_body<true, true>), kBlock)
+FSIM_BATCHED_KERNEL(kb_solid_deform, SolidArgs, solid_deform_body<false>, kSolidBlock)
+FSIM_BATCHED_KERNEL(kb_solid_deform_mixed, SolidArgs, solid_deform_body<true>, kSolidBlock)
+FSIM_BATCHED_KERNEL(kb_solid_deform_resolve, SolidArgs, (solid_deform_body<false, true>), kSolidBlock)
+FSIM_BATCHED_KERNEL(kb_solid_deform_mixed_resolve, SolidArgs, (solid_deform_body<true, true>), kSolidBlock)
 
 // solidUpdate (src/solid.cu:209-239) of particle i with position x, velocity v
 // and acceleration a, into pos and vel.
@@ -2556,6 +2561,15 @@ __device__ __forceinline__ void solid_update_particle(const DevParams &P, const 
     }
     pos[i] = x;
     vel[i] = v;
+}
+
+// 32 bytes of a solid record with one load (an ordinary one: in the fused launch
+// the same kernel wrote them).
+__device__ __forceinline__ void load_solid_record(const float *p, float4 &a, float4 &b)
+{
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p));
 }
 
 constexpr int kForceAhead = 2; // list entries a lane of the force sweep loads ahead
@@ -2702,8 +2716,8 @@ __device__ __forceinline__ void solid_force_body(const DevParams &P, const Solid
         // kForceAhead entries' loads in flight together, summed in list order
         for (int e0 = S.nbr_off[o] + g, ee = S.nbr_off[o + 1]; e0 < ee; e0 += kForceAhead * kSolidGroup) {
             int js[kForceAhead];
-            float4 rj[kForceAhead], q0[kForceAhead], q1[kForceAhead], q2[kForceAhead], xj[kForceAhead],
-                vj[kForceAhead];
+            float4 q0[kForceAhead], q1[kForceAhead], q2[kForceAhead], q3[kForceAhead];
+            float2 q4[kForceAhead];
 #pragma unroll
             for (int u = 0; u < kForceAhead; ++u) {
                 const int e = e0 + u * kSolidGroup;
@@ -2713,18 +2727,16 @@ __device__ __forceinline__ void solid_force_body(const DevParams &P, const Solid
 #pragma unroll
             for (int u = 0; u < kForceAhead; ++u) {
                 const int j = js[u] < 0 ? i : js[u];
-                rj[u] = S.ref[j];
-                const float4 *plj = reinterpret_cast<const float4 *>(S.PL + kPLStride * j);
-                q0[u] = plj[0];
-                q1[u] = plj[1];
-                q2[u] = plj[2];
-                xj[u] = S.pos[j];
-                vj[u] = S.vel[j];
+                const float *rec = S.PL + kPLStride * j;
+                load_solid_record(rec, q0[u], q1[u]);
+                load_solid_record(rec + 8, q2[u], q3[u]);
+                q4[u] = *reinterpret_cast<const float2 *>(rec + 16);
             }
 #pragma unroll
             for (int u = 0; u < kForceAhead; ++u) {
                 const bool in = js[u] >= 0;
-                const float dX = __fsub_rn(rj[u].x, ri.x), dY = __fsub_rn(rj[u].y, ri.y), dZ = __fsub_rn(rj[u].z, ri.z);
+                const float4 xj = q3[u]; // position; velocity x
+                const float dX = __fsub_rn(q2[u].y, ri.x), dY = __fsub_rn(q2[u].z, ri.y), dZ = __fsub_rn(q2[u].w, ri.z);
                 const float w = solid_pair_weight(P, dX, dY, dZ);
                 const float PLj[9] = {q0[u].x, q0[u].y, q0[u].z, q0[u].w, q1[u].x,
                                       q1[u].y, q1[u].z, q1[u].w, q2[u].x};
@@ -2735,10 +2747,9 @@ __device__ __forceinline__ void solid_force_body(const DevParams &P, const Solid
                 float bx = fmaf(row3(__fadd_rn(PLj[0], PLi[0]), __fadd_rn(PLj[1], PLi[1]), __fadd_rn(PLj[2], PLi[2])), ws, ax);
                 float by = fmaf(row3(__fadd_rn(PLj[3], PLi[3]), __fadd_rn(PLj[4], PLi[4]), __fadd_rn(PLj[5], PLi[5])), ws, ay);
                 float bz = fmaf(row3(__fadd_rn(PLj[6], PLi[6]), __fadd_rn(PLj[7], PLi[7]), __fadd_rn(PLj[8], PLi[8])), ws, az);
-                const float ddx = __fsub_rn(xj[u].x, xi.x), ddy = __fsub_rn(xj[u].y, xi.y),
-                            ddz = __fsub_rn(xj[u].z, xi.z);
-                const float dvdx = fmaf(__fsub_rn(vj[u].z, vi.z), ddz,
-                                        fmaf(__fsub_rn(vj[u].y, vi.y), ddy, __fmul_rn(__fsub_rn(vj[u].x, vi.x), ddx)));
+                const float ddx = __fsub_rn(xj.x, xi.x), ddy = __fsub_rn(xj.y, xi.y), ddz = __fsub_rn(xj.z, xi.z);
+                const float dvdx = fmaf(__fsub_rn(q4[u].y, vi.z), ddz,
+                                        fmaf(__fsub_rn(q4[u].x, vi.y), ddy, __fmul_rn(__fsub_rn(xj.w, vi.x), ddx)));
                 const float nu = __fdiv_rn(__fmul_rn(P.h, dvdx),
                                            __fadd_rn(fmaf(ddz, ddz, fmaf(ddy, ddy, __fmul_rn(ddx, ddx))), P.eps_h2));
                 const float visc = __fmul_rn(fmaf(__fmul_rn(P.alpha, nu), P.cs_s, -__fmul_rn(__fmul_rn(P.beta, nu), nu)), w);
@@ -2763,12 +2774,12 @@ __device__ __forceinline__ void solid_force_body(const DevParams &P, const Solid
     S.dudt[i] = a;
     if (S.pos_out) solid_update_particle(P, S, i, S.pos[i], S.vel[i], a, S.pos_out, S.vel_out);
 }
-FSIM_BATCHED_KERNEL_P(kb_solid_force, SolidArgs, solid_force_body<false>, kBlock)
-FSIM_BATCHED_KERNEL_P(kb_solid_force_record, SolidArgs, (solid_force_body<false, 1>), kBlock)
-FSIM_BATCHED_KERNEL_P(kb_solid_force_listed, SolidArgs, (solid_force_body<false, 2>), kBlock)
-FSIM_BATCHED_KERNEL(kb_solid_force_mixed, SolidArgs, solid_force_body<true>, kBlock)
-FSIM_BATCHED_KERNEL(kb_solid_force_mixed_record, SolidArgs, (solid_force_body<true, 1>), kBlock)
-FSIM_BATCHED_KERNEL(kb_solid_force_mixed_listed, SolidArgs, (solid_force_body<true, 2>), kBlock)
+FSIM_BATCHED_KERNEL_P(kb_solid_force, SolidArgs, solid_force_body<false>, kSolidBlock)
+FSIM_BATCHED_KERNEL_P(kb_solid_force_record, SolidArgs, (solid_force_body<false, 1>), kSolidBlock)
+FSIM_BATCHED_KERNEL_P(kb_solid_force_listed, SolidArgs, (solid_force_body<false, 2>), kSolidBlock)
+FSIM_BATCHED_KERNEL(kb_solid_force_mixed, SolidArgs, solid_force_body<true>, kSolidBlock)
+FSIM_BATCHED_KERNEL(kb_solid_force_mixed_record, SolidArgs, (solid_force_body<true, 1>), kSolidBlock)
+FSIM_BATCHED_KERNEL(kb_solid_force_mixed_listed, SolidArgs, (solid_force_body<true, 2>), kSolidBlock)
 
 // The update as a launch of its own, in place: the first of an odd number of
 // sub-steps, and the fused launch.
@@ -3752,22 +3763,22 @@ fsim_status enqueue_plan(const Plan &pl, cudaStream_t main_st, int shape_arg, cu
             }
             if (sweep1) CK(cudaEventRecordWithFlags(sweep1, st, sweep_flags));
             break;
-        case L_DEFORM: FSIM_LAUNCH(kb_solid_deform, SolidArgs, kBlock); break;
-        case L_FORCE: { FSIM_LAUNCH_P(kb_solid_force, SolidArgs, kBlock); } break;
-        case L_FORCE_RECORD: { FSIM_LAUNCH_P(kb_solid_force_record, SolidArgs, kBlock); } break;
-        case L_FORCE_LISTED: { FSIM_LAUNCH_P(kb_solid_force_listed, SolidArgs, kBlock); } break;
+        case L_DEFORM: FSIM_LAUNCH(kb_solid_deform, SolidArgs, kSolidBlock); break;
+        case L_FORCE: { FSIM_LAUNCH_P(kb_solid_force, SolidArgs, kSolidBlock); } break;
+        case L_FORCE_RECORD: { FSIM_LAUNCH_P(kb_solid_force_record, SolidArgs, kSolidBlock); } break;
+        case L_FORCE_LISTED: { FSIM_LAUNCH_P(kb_solid_force_listed, SolidArgs, kSolidBlock); } break;
         case L_UPDATE: FSIM_LAUNCH(kb_solid_update, SolidArgs, kBlock); break;
         case L_SOLID_SLOTS: FSIM_LAUNCH(kb_solid_slots, SolidArgs, kBlock); break;
-        case L_DEFORM_R: FSIM_LAUNCH(kb_solid_deform_resolve, SolidArgs, kBlock); break;
-        case L_DEFORM_M_R: FSIM_LAUNCH(kb_solid_deform_mixed_resolve, SolidArgs, kBlock); break;
+        case L_DEFORM_R: FSIM_LAUNCH(kb_solid_deform_resolve, SolidArgs, kSolidBlock); break;
+        case L_DEFORM_M_R: FSIM_LAUNCH(kb_solid_deform_mixed_resolve, SolidArgs, kSolidBlock); break;
         case L_HASH_M: FSIM_LAUNCH(kb_hash_mixed, HashMixedArgs, kBlock); break;
         case L_CELLREF: FSIM_LAUNCH(kb_cell_ref, CellRefArgs, kBlock); break;
         case L_COUPLE_M: FSIM_LAUNCH(kb_couple_mixed, CoupleArgs, kBlock); break;
         case L_VIRT_M: FSIM_LAUNCH(kb_virt_mixed, VirtArgs, kBlock); break;
-        case L_DEFORM_M: FSIM_LAUNCH(kb_solid_deform_mixed, SolidArgs, kBlock); break;
-        case L_FORCE_M: FSIM_LAUNCH(kb_solid_force_mixed, SolidArgs, kBlock); break;
-        case L_FORCE_M_RECORD: FSIM_LAUNCH(kb_solid_force_mixed_record, SolidArgs, kBlock); break;
-        case L_FORCE_M_LISTED: FSIM_LAUNCH(kb_solid_force_mixed_listed, SolidArgs, kBlock); break;
+        case L_DEFORM_M: FSIM_LAUNCH(kb_solid_deform_mixed, SolidArgs, kSolidBlock); break;
+        case L_FORCE_M: FSIM_LAUNCH(kb_solid_force_mixed, SolidArgs, kSolidBlock); break;
+        case L_FORCE_M_RECORD: FSIM_LAUNCH(kb_solid_force_mixed_record, SolidArgs, kSolidBlock); break;
+        case L_FORCE_M_LISTED: FSIM_LAUNCH(kb_solid_force_mixed_listed, SolidArgs, kSolidBlock); break;
         case L_SOLID_FUSED: {
             SolidFusedArgs F;
             F.bstart_w = tb;

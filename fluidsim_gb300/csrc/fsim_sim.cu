@@ -828,7 +828,7 @@ void plan_solid(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, in
                 fsim_sim *h = m[q];
                 const int nsub = h->cfg.solid_sub_step, odd = nsub & 1;
                 const bool active = h->ns && k < nsub, in_place = odd && k == 0;
-                wb.push_back(active ? blocks_for((long long)kSolidGroup * h->ns, kBlock) : 0);
+                wb.push_back(active ? blocks_for((long long)kSolidGroup * h->ns, kSolidBlock) : 0);
                 ub.push_back(active && in_place ? blocks_for(h->ns, kBlock) : 0);
                 const int from = in_place || (k - odd) % 2 == 0 ? ps : 1 - ps;
                 SolidArgs &S = it[q].A;

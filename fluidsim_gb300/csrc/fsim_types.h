@@ -57,7 +57,8 @@ enum : unsigned { FLAG_OUT_OF_GRID = 1u, FLAG_BARRIER_TIMEOUT = 2u, FLAG_CELL_OV
 // scan's cost grows with the square of the count) and raise FLAG_CELL_OVERFULL.
 constexpr int kStableRankMax = 1024;
 
-constexpr int kBlock = 256;         // threads per block of the element-wise and solid kernels
+constexpr int kBlock = 256;         // threads per block of the element-wise kernels
+constexpr int kSolidBlock = 128;    // and of the solid sweeps (60-100 registers: finer blocks fill an SM better)
 constexpr int kScanThreads = 1024;  // cell-count scan: threads per block
 constexpr int kScanItems = 4;       //   and counts per thread
 constexpr int kScanTile = kScanThreads * kScanItems;
@@ -65,7 +66,7 @@ constexpr int kScanCluster = 8;     // blocks of a cluster that scans an item's 
 constexpr int kClusterScanChunk = kScanCluster * kScanThreads * 16, kClusterScanMax = 4 * kClusterScanChunk;
 constexpr int kMaxScanTiles = 16384; // cell grids up to 67M cells
 constexpr int kFluidListCap = 48;   // fluid list entries per solid lane
-constexpr int kPLStride = 12;       // floats per particle of the solid's P L^-1 array (16-byte rows)
+constexpr int kPLStride = 24;       // floats per particle of the solid's force records (32-byte aligned)
 constexpr int kCellRefLanes = 8;    // lanes per cell of the mixed form's per-cell references (a power of two)
 
 __host__ __device__ inline int blocks_for(long long n, int b) { return (int)((n + b - 1) / b); }
@@ -306,7 +307,10 @@ struct SolidArgs {
     const int *ids_f;      // per-step fluid cell index of a neighbour-list instance (else nullptr)
     const float4 *np;
     float *F, *L;           // 9 floats per particle, row-major: F then P; L^-1 then cof(F) L^-1
-    float *PL;              // kPLStride floats per particle (9 used): three 16-byte loads per neighbour
+    // force records, written by the deformation: what a force entry reads of its
+    // neighbour (P L^-1, reference position, position, velocity: 18 floats) in
+    // two 32-byte loads and one of 8, instead of six of 16 from four arrays
+    float *PL;
     float4 *dudt, *couple;
     const float4 *fposr, *fvelp;
     const int *start_f;
