@@ -3,7 +3,7 @@
 Sizes around the ends of warps, blocks, the build's chunks and of the rule for
 the lanes that share a particle (8,192 and 16,384 fluid particles); batches of
 which only one member rebuilds; the mixed form's solid-fluid lists; odd and even
-numbers of solid sub-steps.
+numbers of solid sub-steps; the conversions that read the mixed form.
 
 The rates are held to the bound of the other per-phase tests: at most twice
 the FP32 oracle's own error against FP64, plus 5e-5 of the largest value; the
@@ -209,3 +209,35 @@ def test_fields_together_equal_fields_one_by_one(precision, pinned, shift):
         for k in names:
             assert np.array_equal(a.get(k), b.get(k)), k
         del views, owner
+
+
+@pytest.mark.parametrize("gamma", [1.0, 7.0, 16.0, 17.0, 1.4])
+def test_mixed_state_reads_round_once(gamma):
+    """Densities and pressures read from the mixed form are the 64-bit values of the
+    held deviation rounded once: within one last place (half of it, and 2^-44 relative
+    from either side's arithmetic), over the fast range and what takes the other path.
+    A position read back is what was set within one last place of it and of its offset
+    (below 2^-4)."""
+    cfg, pa = _box((25, 26, 25), precision=api.PRECISION_MIXED)
+    cfg.gamma = gamma
+    rng = np.random.default_rng(5)
+    n = len(pa.fluid_rho)
+    rho0 = np.float64(cfg.fluid_density)
+    rho = (rho0 * (1.0 + rng.uniform(-1, 1, n) * 10.0 ** rng.uniform(-6, 0, n))).astype(np.float32)
+    rho[:6] = [rho0, 0.0, 2.0 * rho0, 3.5 * rho0, np.nextafter(np.float32(rho0), np.float32(0)), np.inf]
+    pos = pa.fluid_pos + rng.uniform(-1e-4, 1e-4, pa.fluid_pos.shape).astype(np.float32)
+    delta = (rho.astype(np.float64) / rho0 - 1.0).astype(np.float32).astype(np.float64)
+    with api.Simulation(cfg, pa, device=0) as sim:
+        sim.set("fluid_rho", rho)
+        sim.set("fluid_pos", pos)
+        d = sim.derived()
+        with np.errstate(divide="ignore"):
+            p = np.maximum(np.float64(d.coefficient_rho2p) * np.expm1(np.float64(np.float32(gamma)) * np.log1p(delta)),
+                           np.float64(cfg.min_pressure))
+        assert (np.abs(sim.get("fluid_pos").astype(np.float64) - pos) <= np.spacing(np.abs(pos)) + 2.0 ** -28).all()
+        for name, want in (("fluid_rho", rho0 * (1.0 + delta)), ("fluid_p", p)):
+            want = want.astype(np.float32)
+            got = sim.get(name)
+            near = (got == want) | (got == np.nextafter(want, np.float32(np.inf))) \
+                | (got == np.nextafter(want, np.float32(-np.inf)))
+            assert near.all(), (name, got[~near][:4], want[~near][:4])
