@@ -33,6 +33,7 @@
 #include <cstdio>
 #include <cstring>
 #include <new>
+#include <utility>
 #include <vector>
 
 using namespace fsim_rt;
@@ -351,6 +352,11 @@ __global__ void __cluster_dims__(kScanCluster, 1, 1) __launch_bounds__(kScanThre
     __shared__ int totals[2][kScanCluster]; // every block's copy of the cluster's totals, by chunk parity
     const ScanArgs &J = items[blockIdx.x / kScanCluster].A;
     const int rank = (int)cluster.block_rank(), n = J.n;
+    if (n <= 0) return; // the whole cluster
+    // a block's shared memory may be written only once that block is known to run:
+    // every block arrives here and waits before its first remote store, with the
+    // first chunk's loads and block scan in between
+    auto started = cluster.barrier_arrive();
     constexpr int kPer = kClusterScanChunk / (kScanCluster * kScanThreads); // counts per thread
     int carry = 0;
     for (int base = 0, par = 0; base < n; base += kClusterScanChunk, par ^= 1) { // n is the same for the cluster
@@ -369,6 +375,7 @@ __global__ void __cluster_dims__(kScanCluster, 1, 1) __launch_bounds__(kScanThre
         for (int k = 0; k < kPer; ++k) sum += v[k];
         int total;
         int run = carry + block_exclusive_scan(sum, &total);
+        if (base == 0) cluster.barrier_wait(std::move(started));
         if (threadIdx.x < kScanCluster) *cluster.map_shared_rank(&totals[par][rank], threadIdx.x) = total;
         cluster.sync();
         int all = 0;
@@ -395,7 +402,7 @@ __global__ void __cluster_dims__(kScanCluster, 1, 1) __launch_bounds__(kScanThre
                 if (i0 + k < n) J.out[i0 + k] = o[k];
         }
     }
-    if (n > 0 && rank == 0 && threadIdx.x == 0) J.out[n] = carry;
+    if (rank == 0 && threadIdx.x == 0) J.out[n] = carry;
     cluster.sync(); // no block leaves while another may still write its totals
 }
 
