@@ -143,6 +143,15 @@ struct fsim_sim {
 
 namespace {
 
+// Host memory to the device, there when the call returns.  (cudaMemcpy from
+// pageable memory may return once the data is staged, and the kernels that read it
+// run on non-blocking streams, which do not wait for the legacy stream's copies.)
+cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t st)
+{
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
 template <typename T>
 fsim_status dalloc(fsim_sim *h, T **p, size_t count)
 {
@@ -898,9 +907,9 @@ fsim_status build_plan(const std::vector<fsim_sim *> &m, unsigned phases, int pf
     pl->ps = ps;
     ArenaBuilder ab;
     if ((phases & (1u << FSIM_PHASE_CELL)) && !m.empty() && m[0]->nl) {
-        cudaError_t e = cudaMalloc((void **)&pl->act, sizeof(int) * (2 + m.size()));
-        if (e == cudaSuccess) e = cudaMemset(pl->act, 0, sizeof(int) * (2 + m.size()));
-        if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy); // the plan runs on a stream of its own
+        const std::vector<int> none(2 + m.size(), 0);
+        cudaError_t e = cudaMalloc((void **)&pl->act, sizeof(int) * none.size());
+        if (e == cudaSuccess) e = upload(pl->act, none.data(), sizeof(int) * none.size(), cudaStreamLegacy);
         if (e != cudaSuccess) {
             cudaGetLastError();
             fsim_set_error("plan allocation failed: %s", cudaGetErrorString(e));
@@ -928,7 +937,7 @@ fsim_status build_plan(const std::vector<fsim_sim *> &m, unsigned phases, int pf
     pl->host = ab.bytes;
     if (!ab.bytes.empty()) {
         cudaError_t e = cudaMalloc((void **)&pl->arena, ab.bytes.size());
-        if (e == cudaSuccess) e = cudaMemcpy(pl->arena, ab.bytes.data(), ab.bytes.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = upload(pl->arena, ab.bytes.data(), ab.bytes.size(), cudaStreamLegacy);
         if (e != cudaSuccess) {
             cudaGetLastError();
             fsim_set_error("plan upload failed: %s", cudaGetErrorString(e));
@@ -1180,7 +1189,7 @@ fsim_status sort_virtual(fsim_sim *h, const float *vpos_host, float4 *vpos_dev =
                {blocks_for(n, kBlock)});
     pl.host = ab.bytes;
     CK(cudaMalloc((void **)&pl.arena, ab.bytes.size()));
-    cudaError_t e = cudaMemcpy(pl.arena, ab.bytes.data(), ab.bytes.size(), cudaMemcpyHostToDevice);
+    cudaError_t e = upload(pl.arena, ab.bytes.data(), ab.bytes.size(), h->stream);
     if (e == cudaSuccess && (st = enqueue_plan(pl, h->stream, 0)) == FSIM_OK) {
         e = cudaMemsetAsync(h->v_velp, 0, sizeof(float4) * n, h->stream);
         // the normal sums the walls within R: any grid of cells >= R finds them
@@ -1269,10 +1278,10 @@ fsim_status build_solid_neighbors(fsim_sim *h, const float *ref)
     if ((st = dalloc(h, &h->s_nbr_off, (size_t)ns + 1)) || (st = dalloc(h, &h->s_nbr_orig, ne)) ||
         (st = dalloc(h, &h->s_nbr_owner, ne)) || (st = dalloc(h, &h->s_nbr_slot, ne)))
         return st;
-    CK(cudaMemcpy(h->s_nbr_off, off.data(), sizeof(int) * (ns + 1), cudaMemcpyHostToDevice));
+    CK(upload(h->s_nbr_off, off.data(), sizeof(int) * (ns + 1), h->stream));
     if (ne) {
-        CK(cudaMemcpy(h->s_nbr_orig, nbr.data(), sizeof(int) * ne, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(h->s_nbr_owner, owner.data(), sizeof(int) * ne, cudaMemcpyHostToDevice));
+        CK(upload(h->s_nbr_orig, nbr.data(), sizeof(int) * ne, h->stream));
+        CK(upload(h->s_nbr_owner, owner.data(), sizeof(int) * ne, h->stream));
     }
     return FSIM_OK;
 }
@@ -1421,11 +1430,11 @@ fsim_status create_impl(fsim_sim *h, const fsim_particles *p)
         // F = L = I, P = 0 until the first solid phase (include/host_data.cuh:95-97)
         std::vector<float> eye(9 * (size_t)ns, 0.0f);
         for (int i = 0; i < ns; ++i) eye[9 * i] = eye[9 * i + 4] = eye[9 * i + 8] = 1.0f;
-        CK(cudaMemcpy(h->s_F, eye.data(), sizeof(float) * 9 * ns, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(h->s_L, eye.data(), sizeof(float) * 9 * ns, cudaMemcpyHostToDevice));
-        CK(cudaMemset(h->s_P, 0, sizeof(float) * 9 * ns));
-        CK(cudaMemset(h->s_dudt, 0, sizeof(float4) * ns));
-        CK(cudaMemset(h->s_couple, 0, sizeof(float4) * ns));
+        CK(upload(h->s_F, eye.data(), sizeof(float) * 9 * ns, h->stream));
+        CK(upload(h->s_L, eye.data(), sizeof(float) * 9 * ns, h->stream));
+        CK(cudaMemsetAsync(h->s_P, 0, sizeof(float) * 9 * ns, h->stream));
+        CK(cudaMemsetAsync(h->s_dudt, 0, sizeof(float4) * ns, h->stream));
+        CK(cudaMemsetAsync(h->s_couple, 0, sizeof(float4) * ns, h->stream));
         h->s_mech_ok = true; // initial values, in input order (= s_orig[0])
         h->s_np_ok = true;
         if ((st = build_solid_neighbors(h, p->solid_ref_pos))) return st;
@@ -2577,10 +2586,11 @@ std::vector<SnapArray> snap_arrays(fsim_sim *h, int pf, int ps)
 fsim_status nl_restore(fsim_sim *h)
 {
     NlState saved;
-    CK(cudaMemcpy(&saved, h->nl_state, sizeof saved, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(&saved, h->nl_state, sizeof saved, cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
     NlState now = saved;
     now.rebuild = 1;
-    CK(cudaMemcpy(h->nl_state, &now, sizeof now, cudaMemcpyHostToDevice));
+    CK(upload(h->nl_state, &now, sizeof now, h->stream));
     const float4 *vpos = h->mixed ? h->v_abs : h->v_posr; // absolute wall positions
     if (h->nv) {
         launch_k_cells_of(blocks_for(h->nv, kBlock), h->stream, h->P, vpos, h->nv, h->v_icell, h->v_icxyz);
@@ -2598,8 +2608,8 @@ fsim_status nl_restore(fsim_sim *h)
                {blocks_for(h->nf, h->nf <= kNlWarpBuildMax ? kNlBuildThreads / 32 : kNlBuildThreads)}, kRebuildBuildGrid, 1);
     pl.host = ab.bytes;
     cudaError_t e = cudaMalloc((void **)&pl.arena, std::max<size_t>(ab.bytes.size(), 1));
-    if (e == cudaSuccess) e = cudaMemcpy(pl.act, only, sizeof only, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(pl.arena, ab.bytes.data(), ab.bytes.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload(pl.act, only, sizeof only, h->stream);
+    if (e == cudaSuccess) e = upload(pl.arena, ab.bytes.data(), ab.bytes.size(), h->stream);
     fsim_status st = FSIM_OK;
     if (e == cudaSuccess) st = enqueue_plan(pl, h->stream, 0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
@@ -2612,7 +2622,7 @@ fsim_status nl_restore(fsim_sim *h)
         return FSIM_ECUDA;
     }
     if (st) return st;
-    CK(cudaMemcpy(h->nl_state, &saved, sizeof saved, cudaMemcpyHostToDevice));
+    CK(upload(h->nl_state, &saved, sizeof saved, h->stream));
     return FSIM_OK;
 }
 size_t snap_payload(fsim_sim *h)
@@ -2706,7 +2716,7 @@ extern "C" fsim_status fsim_snapshot_load(const void *buf, size_t bytes, int dev
     const char *ref_src = nullptr, *orig_src = nullptr;
     cudaError_t e = cudaSuccess;
     for (const SnapArray &a : snap_arrays(h, 0, 0)) {
-        if (a.bytes && e == cudaSuccess) e = cudaMemcpy(a.dev, in + off, a.bytes, cudaMemcpyHostToDevice);
+        if (a.bytes && e == cudaSuccess) e = upload(a.dev, in + off, a.bytes, h->stream);
         if (a.dev == h->s_ref[0]) ref_src = in + off;
         if (a.dev == h->s_orig[0]) orig_src = in + off;
         off += (a.bytes + 15) & ~size_t(15);
@@ -2735,11 +2745,11 @@ extern "C" fsim_status fsim_snapshot_load(const void *buf, size_t bytes, int dev
         }
         std::vector<float> eye(9 * (size_t)ns, 0.0f);
         for (int i = 0; i < ns; ++i) eye[9 * i] = eye[9 * i + 4] = eye[9 * i + 8] = 1.0f;
-        e = cudaMemcpy(h->s_F, eye.data(), sizeof(float) * 9 * ns, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(h->s_L, eye.data(), sizeof(float) * 9 * ns, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemset(h->s_P, 0, sizeof(float) * 9 * ns);
-        if (e == cudaSuccess) e = cudaMemset(h->s_dudt, 0, sizeof(float4) * ns);
-        if (e == cudaSuccess) e = cudaMemset(h->s_couple, 0, sizeof(float4) * ns);
+        e = upload(h->s_F, eye.data(), sizeof(float) * 9 * ns, h->stream);
+        if (e == cudaSuccess) e = upload(h->s_L, eye.data(), sizeof(float) * 9 * ns, h->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(h->s_P, 0, sizeof(float) * 9 * ns, h->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(h->s_dudt, 0, sizeof(float4) * ns, h->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(h->s_couple, 0, sizeof(float4) * ns, h->stream);
         if (e != cudaSuccess || (st = build_solid_neighbors(h, ref.data()))) {
             if (!st) fsim_set_error("snapshot restore failed: %s", cudaGetErrorString(e));
             free_all(h);
@@ -2953,11 +2963,11 @@ extern "C" fsim_status fsim_create_case(const fsim_config *cfg, const fsim_case 
         }
         std::vector<float> eye(9 * (size_t)ns, 0.0f);
         for (int k = 0; k < ns; ++k) eye[9 * k] = eye[9 * k + 4] = eye[9 * k + 8] = 1.0f;
-        CK(cudaMemcpy(h->s_F, eye.data(), sizeof(float) * 9 * ns, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(h->s_L, eye.data(), sizeof(float) * 9 * ns, cudaMemcpyHostToDevice));
-        CK(cudaMemset(h->s_P, 0, sizeof(float) * 9 * ns));
-        CK(cudaMemset(h->s_dudt, 0, sizeof(float4) * ns));
-        CK(cudaMemset(h->s_couple, 0, sizeof(float4) * ns));
+        CK(upload(h->s_F, eye.data(), sizeof(float) * 9 * ns, h->stream));
+        CK(upload(h->s_L, eye.data(), sizeof(float) * 9 * ns, h->stream));
+        CK(cudaMemsetAsync(h->s_P, 0, sizeof(float) * 9 * ns, h->stream));
+        CK(cudaMemsetAsync(h->s_dudt, 0, sizeof(float4) * ns, h->stream));
+        CK(cudaMemsetAsync(h->s_couple, 0, sizeof(float4) * ns, h->stream));
         h->s_mech_ok = h->s_np_ok = true;
         if ((st = build_solid_neighbors(h, ref.data()))) return fail(st);
     }
