@@ -552,7 +552,7 @@ FSIM_BATCHED_KERNEL(kb_rank, RankArgs, rank_body, kBlock)
 // particle per step, so its cost is negligible.
 __device__ __forceinline__ float tait_pressure(const DevParams &P, float rho)
 {
-    const float p = (powf(rho * P.rho0_inv, P.gamma) - 1.0f) * P.rho2p;
+    const float p = __fmul_rn(__fsub_rn(powf(__fmul_rn(rho, P.rho0_inv), P.gamma), 1.0f), P.rho2p);
     return fmaxf(p, P.min_p);
 }
 
@@ -590,54 +590,51 @@ __device__ __forceinline__ float rcp_approx(float x)
     return y;
 }
 
+// x . y of the plain form.
+__device__ __forceinline__ float dot3(float x0, float x1, float x2, float y0, float y1, float y2)
+{
+    return __fmaf_rn(x2, y2, __fmaf_rn(x0, y0, __fmul_rn(x1, y1)));
+}
+
 // LIMITER: min(3 du, c0) (fluid, wall) or c0 (solid).  clamp_ps: P* >= 0 (wall).
 // The terms of one pair: drho += x w, a += f (dx, dy, dz).
-// EXACT (mixed form): every rounding spelled out (no contraction freedom left to
-// the compiler), so that every kernel inlining this rounds identically.
-// SPELLED: the one contraction of the plain terms that came out differently in
-// different kernels (either product of P* may be the one left unrounded, and for a
-// solid neighbour, whose density is the particle's own, both are alike to the
-// compiler): fixed for the one-instance list sweep.  The batched forms keep their
-// own, so a batch member that touches a solid can differ from its standalone run
-// in the last bit.
-template <bool LIMITER, int VISCID, bool EXACT = false, bool SPELLED = false>
+// Every rounding is spelled out (here and in the particle update), so that no
+// contraction is left to the compiler: it chose differently in different kernels
+// (which product of P* stays unrounded), and a batch member must equal its
+// standalone run, and a particle its sums, bit for bit whatever the launch form,
+// the launch shape and the lanes per particle.  MIXED and JI only choose between
+// equally good orders: that of the velocity's dot product, and which product of P*
+// is rounded by itself (JI: rho_i p_j).
+template <bool LIMITER, int VISCID, bool MIXED = false, bool JI = false>
 __device__ __forceinline__ void riemann_terms(const DevParams &P, float dx, float dy, float dz, float r2, float uix,
                                               float uiy, float uiz, float rhoi, float pi, float ujx, float ujy,
                                               float ujz, float rhoj, float pj, bool clamp_ps, float &x, float &w,
                                               float &f)
 {
-    if (EXACT) {
-        w = __fmul_rn(ex2_approx(__fmul_rn(r2, P.exp2_scale)), P.kdiff);
-        const float inv_r = rsqrt_approx(fmaxf(r2, 1e-30f));
-        const float rs_inv = rcp_approx(__fadd_rn(rhoi, rhoj));
-        const float a = fmaf(__fsub_rn(uiz, ujz), dz, fmaf(__fsub_rn(uiy, ujy), dy, __fmul_rn(__fsub_rn(uix, ujx), dx)));
-        const float du = fmaxf(__fmul_rn(a, inv_r), 0.0f);
-        const float lim = LIMITER ? fminf(__fmul_rn(3.0f, du), P.c0) : P.c0;
-        float ps = __fmul_rn(fmaf(rhoi, pj, __fmul_rn(rhoj, pi)), rs_inv);
-        ps = fmaf(__fmul_rn(__fmul_rn(__fmul_rn(rhoi, rhoj), rs_inv), du), lim, ps);
-        if (clamp_ps) ps = fmaxf(ps, 0.0f);
-        const float r = __fmul_rn(r2, inv_r);
-        x = __fmul_rn(fmaf(rhoj, a, -__fmul_rn(__fmul_rn(__fsub_rn(pi, pj), r), P.c0_inv)), rs_inv);
-        f = __fmul_rn(-2.0f, ps);
-        if (VISCID == 1 || (VISCID == 2 && P.viscid))
-            f = fmaf(__fmul_rn(P.mu10, -a), rcp_approx(__fadd_rn(r2, P.eps_h2)), f);
-        f = __fmul_rn(f, w);
-        return;
-    }
-    w = ex2_approx(r2 * P.exp2_scale) * P.kdiff;
+    w = __fmul_rn(ex2_approx(__fmul_rn(r2, P.exp2_scale)), P.kdiff);
     const float inv_r = rsqrt_approx(fmaxf(r2, 1e-30f)); // r2 = 0 (the particle itself) contributes 0
-    const float rs_inv = rcp_approx(rhoi + rhoj);
-    const float a = (uix - ujx) * dx + (uiy - ujy) * dy + (uiz - ujz) * dz;
-    const float du = fmaxf(a * inv_r, 0.0f); // only du >= 0 adds dissipation
-    const float lim = LIMITER ? fminf(3.0f * du, P.c0) : P.c0;
-    float ps = (SPELLED ? __fmaf_rn(rhoj, pi, __fmul_rn(rhoi, pj)) : rhoi * pj + rhoj * pi) * rs_inv;
-    ps = fmaf(rhoi * rhoj * rs_inv * du, lim, ps);
+    const float rs_inv = rcp_approx(__fadd_rn(rhoi, rhoj));
+    const float vx = __fsub_rn(uix, ujx), vy = __fsub_rn(uiy, ujy), vz = __fsub_rn(uiz, ujz);
+    const float a = MIXED ? __fmaf_rn(vz, dz, __fmaf_rn(vy, dy, __fmul_rn(vx, dx))) : dot3(vx, vy, vz, dx, dy, dz);
+    const float du = fmaxf(__fmul_rn(a, inv_r), 0.0f); // only du >= 0 adds dissipation
+    const float lim = LIMITER ? fminf(__fmul_rn(3.0f, du), P.c0) : P.c0;
+    float ps = JI ? __fmaf_rn(rhoj, pi, __fmul_rn(rhoi, pj)) : __fmaf_rn(rhoi, pj, __fmul_rn(rhoj, pi));
+    ps = __fmul_rn(ps, rs_inv);
+    ps = __fmaf_rn(__fmul_rn(__fmul_rn(__fmul_rn(rhoi, rhoj), rs_inv), du), lim, ps);
     if (clamp_ps) ps = fmaxf(ps, 0.0f);
-    const float r = r2 * inv_r;
-    x = (rhoj * a - (pi - pj) * r * P.c0_inv) * rs_inv;
-    f = -2.0f * ps;
-    if (VISCID == 1 || (VISCID == 2 && P.viscid)) f = fmaf(P.mu10 * -a, rcp_approx(r2 + P.eps_h2), f);
-    f *= w;
+    const float r = __fmul_rn(r2, inv_r);
+    x = __fmul_rn(__fmaf_rn(rhoj, a, -__fmul_rn(__fmul_rn(__fsub_rn(pi, pj), r), P.c0_inv)), rs_inv);
+    f = __fmul_rn(-2.0f, ps);
+    if (VISCID == 1 || (VISCID == 2 && P.viscid))
+        f = __fmaf_rn(__fmul_rn(P.mu10, -a), rcp_approx(__fadd_rn(r2, P.eps_h2)), f);
+    f = __fmul_rn(f, w);
+}
+
+// 2 (u - v) . n: the velocity u mirrored at a solid neighbour (velocity v, normal
+// n) is u - that times n (plain form).
+__device__ __forceinline__ float mirror2(float4 u, float4 v, float4 n)
+{
+    return __fmul_rn(2.0f, dot3(__fsub_rn(u.x, v.x), __fsub_rn(u.y, v.y), __fsub_rn(u.z, v.z), n.x, n.y, n.z));
 }
 
 // sum += x w with Kahan's compensation c (mixed form), where `in`
@@ -649,16 +646,16 @@ __device__ __forceinline__ void kahan_add(float x, float w, bool in, float &sum,
     c = in ? d : c;
 }
 
-// Adds one pair to the sums.  KAHAN: the density-rate sum is Kahan-compensated
-// (mixed form).
+// Adds one pair of a cell walk to the sums.  KAHAN: the density-rate sum is
+// Kahan-compensated (mixed form).
 template <bool LIMITER, int VISCID, bool KAHAN = false>
 __device__ __forceinline__ void riemann_pair(const DevParams &P, float dx, float dy, float dz, float r2, float uix,
                                              float uiy, float uiz, float rhoi, float pi, float ujx, float ujy,
                                              float ujz, float rhoj, float pj, bool clamp_ps, PairAcc &A)
 {
     float x, w, f;
-    riemann_terms<LIMITER, VISCID, KAHAN>(P, dx, dy, dz, r2, uix, uiy, uiz, rhoi, pi, ujx, ujy, ujz, rhoj, pj,
-                                          clamp_ps, x, w, f);
+    riemann_terms<LIMITER, VISCID, KAHAN, !KAHAN && LIMITER>(P, dx, dy, dz, r2, uix, uiy, uiz, rhoi, pi, ujx, ujy, ujz,
+                                                             rhoj, pj, clamp_ps, x, w, f);
     if (KAHAN) kahan_add(x, w, true, A.drho, A.drho_c);
     else A.drho = fmaf(x, w, A.drho);
     A.ax = fmaf(f, dx, A.ax);
@@ -675,24 +672,25 @@ __device__ __forceinline__ float4 fluid_update_store(const DevParams &P, const F
                                                      float4 vp, const PairAcc &acc)
 {
     const float rho_inv = __fdividef(1.0f, pr.w);
-    float drho = 2.0f * pr.w * acc.drho;
-    float ax = acc.ax * rho_inv, ay = acc.ay * rho_inv, az = acc.az * rho_inv;
+    float drho = __fmul_rn(__fmul_rn(2.0f, pr.w), acc.drho);
+    float ax = __fmul_rn(acc.ax, rho_inv), ay = __fmul_rn(acc.ay, rho_inv), az = __fmul_rn(acc.az, rho_inv);
     if (!(drho == drho)) drho = 0.0f;
     if (!(ax == ax && ay == ay && az == az)) ax = ay = az = 0.0f;
-    float x = pr.x + vp.x * P.dt, y = pr.y + vp.y * P.dt, z = pr.z + vp.z * P.dt;
-    float ux = vp.x + (ax + P.gx) * P.dt, uy = vp.y + (ay + P.gy) * P.dt, uz = vp.z + (az + P.gz) * P.dt;
-    float rho = pr.w + drho * P.dt;
+    float x = __fmaf_rn(vp.x, P.dt, pr.x), y = __fmaf_rn(vp.y, P.dt, pr.y), z = __fmaf_rn(vp.z, P.dt, pr.z);
+    float ux = __fmaf_rn(__fadd_rn(ax, P.gx), P.dt, vp.x), uy = __fmaf_rn(__fadd_rn(ay, P.gy), P.dt, vp.y),
+          uz = __fmaf_rn(__fadd_rn(az, P.gz), P.dt, vp.z);
+    float rho = __fmaf_rn(drho, P.dt, pr.w);
     rho = fminf(fmaxf(rho, P.min_rho), P.max_rho);
     const float p = tait_pressure(P, rho);
     x = fminf(fmaxf(x, P.dmin[0]), P.dmax[0]);
     y = fminf(fmaxf(y, P.dmin[1]), P.dmax[1]);
     z = fminf(fmaxf(z, P.dmin[2]), P.dmax[2]);
-    const float speed = sqrtf(ux * ux + uy * uy + uz * uz);
+    const float speed = __fsqrt_rn(dot3(ux, uy, uz, ux, uy, uz));
     if (speed > P.vmax) {
-        const float s = P.vmax / speed;
-        ux *= s;
-        uy *= s;
-        uz *= s;
+        const float s = __fdiv_rn(P.vmax, speed);
+        ux = __fmul_rn(ux, s);
+        uy = __fmul_rn(uy, s);
+        uz = __fmul_rn(uz, s);
     }
     const float4 xr = make_float4(x, y, z, rho);
     A.posr_out[i] = xr;
@@ -760,9 +758,9 @@ __device__ __forceinline__ void flush_list(const DevParams &P, const FluidSweepA
                                                       fmaf(-k2, np.x, vp.x), fmaf(-k2, np.y, vp.y),
                                                       fmaf(-k2, np.z, vp.z), pr.w, np.w, false, acc);
                 } else {
-                    const float k2 = 2.0f * ((vp.x - sv.x) * np.x + (vp.y - sv.y) * np.y + (vp.z - sv.z) * np.z);
-                    riemann_pair<false, VISCID>(P, dx, dy, dz, r2, vp.x, vp.y, vp.z, pr.w, vp.w, vp.x - k2 * np.x,
-                                                vp.y - k2 * np.y, vp.z - k2 * np.z, pr.w, np.w, false, acc);
+                    const float k2 = mirror2(vp, sv, np);
+                    riemann_pair<false, VISCID>(P, dx, dy, dz, r2, vp.x, vp.y, vp.z, pr.w, vp.w, __fmaf_rn(-k2, np.x, vp.x),
+                                                __fmaf_rn(-k2, np.y, vp.y), __fmaf_rn(-k2, np.z, vp.z), pr.w, np.w, false, acc);
                 }
             } else {
                 const float4 q = SP == kFluid ? A.posr[j] : A.v_posr[j];
@@ -1319,7 +1317,7 @@ __device__ __forceinline__ void walk_list(const FluidSweepArgs &A, int i, bool v
 }
 
 // Particle i's pairs in the plain form.
-template <int VISCID, bool CHECK, bool LANES, bool ONE>
+template <int VISCID, bool CHECK, bool LANES>
 __device__ __forceinline__ void fluid_sweep_nl_pairs(const DevParams &P, const FluidSweepArgs &A, int i, bool valid,
                                                      float4 pr, float4 vp, ListSum<LANES, false> &sum)
 {
@@ -1347,8 +1345,8 @@ __device__ __forceinline__ void fluid_sweep_nl_pairs(const DevParams &P, const F
             const float4 q = A.v_posr[j], u = A.v_velp[j];
             const float r2 = rel(q, p);
             p.in = r2 < P.R2 && (!CHECK || cells_adjacent(ci, A.nl_cxyz_v[j]));
-            riemann_terms<true, VISCID>(P, p.dx, p.dy, p.dz, r2, vp.x, vp.y, vp.z, pr.w, vp.w, u.x, u.y, u.z, q.w, u.w,
-                                        true, p.x, p.w, p.f);
+            riemann_terms<true, VISCID, false, true>(P, p.dx, p.dy, p.dz, r2, vp.x, vp.y, vp.z, pr.w, vp.w, u.x, u.y,
+                                                     u.z, q.w, u.w, true, p.x, p.w, p.f);
             return p;
         },
         [&](int j) {
@@ -1356,10 +1354,10 @@ __device__ __forceinline__ void fluid_sweep_nl_pairs(const DevParams &P, const F
             const float4 q = A.s_pos[j], np = A.s_np[j], sv = A.s_vel[j];
             const float r2 = rel(q, p);
             p.in = r2 < P.R2 && (!CHECK || cells_adjacent(ci, A.nl_cxyz_s[j]));
-            const float k2 = 2.0f * ((vp.x - sv.x) * np.x + (vp.y - sv.y) * np.y + (vp.z - sv.z) * np.z);
-            riemann_terms<false, VISCID, false, ONE>(P, p.dx, p.dy, p.dz, r2, vp.x, vp.y, vp.z, pr.w, vp.w, vp.x - k2 * np.x,
-                                                     vp.y - k2 * np.y, vp.z - k2 * np.z, pr.w, np.w, false, p.x, p.w,
-                                                     p.f);
+            const float k2 = mirror2(vp, sv, np);
+            riemann_terms<false, VISCID, false, true>(P, p.dx, p.dy, p.dz, r2, vp.x, vp.y, vp.z, pr.w, vp.w,
+                                                      __fmaf_rn(-k2, np.x, vp.x), __fmaf_rn(-k2, np.y, vp.y),
+                                                      __fmaf_rn(-k2, np.z, vp.z), pr.w, np.w, false, p.x, p.w, p.f);
             return p;
         });
 }
@@ -1371,7 +1369,7 @@ __device__ __forceinline__ float (*lane_terms())[32]
     return sweep_terms + kSweepTermRows * (threadIdx.x >> 5);
 }
 
-template <int VISCID, bool LANES, bool ONE>
+template <int VISCID, bool LANES>
 __device__ __forceinline__ void fluid_sweep_nl_lanes(const DevParams &P, const FluidSweepArgs &A, int blk)
 {
     const int t = blk * blockDim.x + threadIdx.x, sh = LANES ? A.lane_shift : 0, i = t >> sh;
@@ -1387,8 +1385,8 @@ __device__ __forceinline__ void fluid_sweep_nl_lanes(const DevParams &P, const F
         pr = A.posr[i];
         vp = A.velp[i];
     }
-    if (A.nl_cxyz_f) fluid_sweep_nl_pairs<VISCID, true, LANES, ONE>(P, A, i, valid, pr, vp, sum);
-    else fluid_sweep_nl_pairs<VISCID, false, LANES, ONE>(P, A, i, valid, pr, vp, sum);
+    if (A.nl_cxyz_f) fluid_sweep_nl_pairs<VISCID, true, LANES>(P, A, i, valid, pr, vp, sum);
+    else fluid_sweep_nl_pairs<VISCID, false, LANES>(P, A, i, valid, pr, vp, sum);
     const PairAcc acc = sum.total();
     unsigned d2bits = 0u;
     if (valid && sum.g == 0) {
@@ -1399,11 +1397,11 @@ __device__ __forceinline__ void fluid_sweep_nl_lanes(const DevParams &P, const F
     const unsigned wmax = __reduce_max_sync(kFull, d2bits);
     if ((threadIdx.x & 31) == 0 && wmax) atomicMax(&A.nl->maxd2, wmax);
 }
-template <int VISCID, bool ONE = false>
+template <int VISCID>
 __device__ __forceinline__ void fluid_sweep_nl_body(const DevParams &P, const FluidSweepArgs &A, int blk)
 {
-    if (A.lane_shift) fluid_sweep_nl_lanes<VISCID, true, ONE>(P, A, blk); // uniform over the launch
-    else fluid_sweep_nl_lanes<VISCID, false, ONE>(P, A, blk);
+    if (A.lane_shift) fluid_sweep_nl_lanes<VISCID, true>(P, A, blk); // uniform over the launch
+    else fluid_sweep_nl_lanes<VISCID, false>(P, A, blk);
 }
 
 // launch shapes of the list sweep: threads per block, minimum blocks per SM
@@ -1422,7 +1420,7 @@ template <int VISCID, class SH>
 __global__ void __launch_bounds__(SH::threads, SH::min_blocks) kb_fluid_sweep_nl_1(const DevParams P,
                                                                                    const FluidSweepArgs A)
 {
-    fluid_sweep_nl_body<VISCID, true>(P, A, (int)blockIdx.x);
+    fluid_sweep_nl_body<VISCID>(P, A, (int)blockIdx.x);
 }
 template <int VISCID, class SH>
 __global__ void __launch_bounds__(SH::threads, SH::min_blocks)
@@ -1803,21 +1801,12 @@ struct OwnMixed {
 // Every mixed-form pair test and pair term rounds it this one way.
 __device__ __forceinline__ float shifted(float ob, int o, float cdx) { return fmaf(-(float)(o + 1), cdx, ob); }
 // Cell codes (o + 1 per axis, each in {0, 1, 2} for neighbouring cells) of a
-// pair from packed coordinates (x | y << 11 | z << 21): with cb = kCellBias -
+// pair (mixed_rel) from packed coordinates (x | y << 11 | z << 21): with cb = kCellBias -
 // c_i, the fields of c_j + cb are the codes when the cells are neighbours;
 // otherwise some field exceeds 2 (a field below -1 wraps to at least 3 in its
 // own bits, given fewer than 2^11, 2^10, 2^11 cells per axis, and any borrow
 // it passes up only shows where a field has already failed).
 constexpr unsigned kCellBias = 1u | (1u << 11) | (1u << 21);
-__device__ __forceinline__ bool cell_codes(unsigned cj, unsigned cb, int &bx, int &by, int &bz)
-{
-    const unsigned d = cj + cb;
-    bx = (int)(d & 0x7ffu);
-    by = (int)((d >> 11) & 0x3ffu);
-    bz = (int)(d >> 21);
-    return bx <= 2 && by <= 2 && bz <= 2;
-}
-
 template <int SP, int VISCID>
 __device__ __forceinline__ void flush_list_m(const DevParams &P, const FluidSweepArgs &A, int (*lst)[32], int lane,
                                              int &cnt, const OwnMixed &o, float4 vp, PairAcc &acc)
@@ -1902,7 +1891,7 @@ __device__ __forceinline__ float4 fluid_update_store_m(const DevParams &P, const
                                                        float4 vp, float rho, const PairAcc &acc, int cx, int cy,
                                                        int cz)
 {
-    // explicit roundings throughout (see riemann_pair's KAHAN branch)
+    // explicit roundings throughout (see riemann_terms)
     const float rho_inv = __fdividef(1.0f, rho);
     float drho = __fmul_rn(__fmul_rn(2.0f, rho), acc.drho);
     float ax = __fmul_rn(acc.ax, rho_inv), ay = __fmul_rn(acc.ay, rho_inv), az = __fmul_rn(acc.az, rho_inv);
@@ -2009,8 +1998,8 @@ __device__ __forceinline__ void unpack_cell(unsigned c, int &cx, int &cy, int &c
     cz = (int)(c >> 21);
 }
 
-// A pair's difference vector in the mixed form from the packed codes d (as
-// cell_codes unpacks them): true when the cells are neighbours.  Where they
+// A pair's difference vector in the mixed form from the packed codes d
+// (kCellBias): true when the cells are neighbours.  Where they
 // are not, the codes come out as those of the own cell, so that what is
 // addressed by them stays in bounds.
 __device__ __forceinline__ bool mixed_rel(const DevParams &P, const OwnMixed &o, unsigned d, float4 q, float &dx,
