@@ -22,7 +22,7 @@ NVCC = os.environ.get("NVCC", "nvcc")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 CUDA_UNITS = ["fsim_kernels.cu", "fsim_sim.cu", "fsim_noalloc.cu", "fsim_probe.cu"]
 HOST_UNITS = ["fsim_host.cpp"]
-HEADERS = ["fsim_internal.h", "fsim_types.h"]
+HEADERS = ["fsim_internal.h", "fsim_span.h", "fsim_types.h"]
 # FSIM_DEVICE_CHECKS=1 in the environment compiles the kernels' index checks
 # in (a debugging build; see FSIM_DCHECK in fsim_kernels.cu)
 DEBUG_FLAGS = ["-DFSIM_DEVICE_CHECKS"] if os.environ.get("FSIM_DEVICE_CHECKS") == "1" else []

@@ -3,8 +3,10 @@
 // lists of a step, captured into CUDA graphs), batches, field I/O, snapshots
 // and the device-side case generator driver.  The kernels are in
 // fsim_kernels.cu; what both share is in fsim_types.h.
+#include "fsim_span.h"
 #include "fsim_types.h"
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
@@ -1948,9 +1950,31 @@ namespace {
 // Above, the copies of the first fields overlap the kernels of the later ones.
 constexpr size_t kStateBytes = 4u << 20;
 
+// What the driver knows of a host pointer (all zero: nothing).
+HostSpan host_span(const void *p)
+{
+    using Query = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+    static const Query query = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const cudaError_t e = cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &fn, 7000, cudaEnableDefault,
+                                                               &found);
+        return reinterpret_cast<Query>(e == cudaSuccess && found == cudaDriverEntryPointSuccess ? fn : nullptr);
+    }();
+    unsigned type = 0, managed = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *to[] = {&type, &managed, &dev, &start, &size};
+    if (!query || query(5, what, to, (CUdeviceptr)p) != CUDA_SUCCESS) return {};
+    return {type == CU_MEMORYTYPE_HOST && !managed, (uintptr_t)dev, (uintptr_t)start, size};
+}
+
 // Enqueue the copies of a call's fields between the bulk buffer and host memory:
-// one kernel if all host buffers are page-locked and mapped (so the device can
-// address them) and word-aligned, else one copy per field.
+// one kernel if every host buffer lies in one page-locked, mapped allocation (so the
+// device can address it) and is word-aligned, else one copy per field.
 fsim_status copy_fields(fsim_sim *h, int nfields, void *const *host, const size_t *bytes, bool to_host)
 {
     CopyArgs C{};
@@ -1959,19 +1983,11 @@ fsim_status copy_fields(fsim_sim *h, int nfields, void *const *host, const size_
     bool direct = true;
     for (int k = 0; k < nfields && direct; ++k) {
         if (!bytes[k]) continue;
-        cudaPointerAttributes at{};
-        direct = reinterpret_cast<uintptr_t>(host[k]) % 4 == 0 &&
-                 cudaPointerGetAttributes(&at, host[k]) == cudaSuccess && at.type == cudaMemoryTypeHost &&
-                 at.devicePointer;
-        // the whole buffer must lie in page-locked memory: its last word too
-        cudaPointerAttributes end{};
-        const char *last = static_cast<const char *>(host[k]) + bytes[k] - 4;
-        direct = direct && cudaPointerGetAttributes(&end, last) == cudaSuccess && end.type == cudaMemoryTypeHost &&
-                 static_cast<const char *>(end.devicePointer) - static_cast<const char *>(at.devicePointer) ==
-                     (ptrdiff_t)(bytes[k] - 4);
+        const HostSpan span = host_span(host[k]);
+        direct = reinterpret_cast<uintptr_t>(host[k]) % 4 == 0 && span_addressable(span, bytes[k]);
         if (!direct) break;
         unsigned *dev = reinterpret_cast<unsigned *>(static_cast<char *>(h->bulk) + off);
-        unsigned *mapped = static_cast<unsigned *>(at.devicePointer);
+        unsigned *mapped = reinterpret_cast<unsigned *>(span.dev);
         CopyArgs::Pair &p = C.pair[pairs++];
         p.dst = to_host ? mapped : dev;
         p.src = to_host ? dev : mapped;
@@ -1985,7 +2001,6 @@ fsim_status copy_fields(fsim_sim *h, int nfields, void *const *host, const size_
         CK_LAUNCH();
         return FSIM_OK;
     }
-    cudaGetLastError(); // a pageable buffer's query may have failed
     off = 0;
     for (int k = 0; k < nfields; ++k) {
         if (!bytes[k]) continue;
