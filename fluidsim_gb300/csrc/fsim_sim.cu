@@ -1974,7 +1974,8 @@ HostSpan host_span(const void *p)
 
 // Enqueue the copies of a call's fields between the bulk buffer and host memory:
 // one kernel if every host buffer lies in one page-locked, mapped allocation (so the
-// device can address it) and is word-aligned, else one copy per field.
+// device can address it), is word-aligned and, to the host, shares no bytes with
+// another, else one copy per field.
 fsim_status copy_fields(fsim_sim *h, int nfields, void *const *host, const size_t *bytes, bool to_host)
 {
     CopyArgs C{};
@@ -1985,6 +1986,9 @@ fsim_status copy_fields(fsim_sim *h, int nfields, void *const *host, const size_
         if (!bytes[k]) continue;
         const HostSpan span = host_span(host[k]);
         direct = reinterpret_cast<uintptr_t>(host[k]) % 4 == 0 && span_addressable(span, bytes[k]);
+        for (int q = 0; q < k && to_host; ++q)
+            direct = direct && !spans_overlap(reinterpret_cast<uintptr_t>(host[q]), bytes[q],
+                                              reinterpret_cast<uintptr_t>(host[k]), bytes[k]);
         if (!direct) break;
         unsigned *dev = reinterpret_cast<unsigned *>(static_cast<char *>(h->bulk) + off);
         unsigned *mapped = reinterpret_cast<unsigned *>(span.dev);

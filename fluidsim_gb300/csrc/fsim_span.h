@@ -24,4 +24,12 @@ inline bool span_addressable(const HostSpan &s, size_t bytes)
     return s.host && s.dev && s.start <= s.dev && s.size >= bytes && s.dev - s.start <= s.size - bytes;
 }
 
+// Whether the buffers [p, p + bytes) overlap: what a call leaves in buffers that
+// share bytes is the last field's, which copies one after another give and copies
+// side by side do not.
+inline bool spans_overlap(uintptr_t p, size_t pbytes, uintptr_t q, size_t qbytes)
+{
+    return pbytes && qbytes && (p < q ? q - p < pbytes : p - q < qbytes);
+}
+
 } // namespace fsim_rt
