@@ -3734,7 +3734,7 @@ fsim_status enqueue_plan(const Plan &pl, cudaStream_t main_st, int shape_arg, cu
         const int g = L.blocks, n = L.ninst;
         cudaStream_t st = main_st;
         if (side) {
-            if (fsim_status r = join(L.join)) return r;
+            if (fsim_status r = join(launch_joins(L, sweep0 != nullptr))) return r;
             if (L.branch) {
                 const int b = L.branch - 1;
                 if (!(open & (1u << b))) {

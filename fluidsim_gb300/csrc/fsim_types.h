@@ -535,6 +535,14 @@ struct Launch {
     unsigned join = 0;                    // side streams (bits) this launch waits for
 };
 
+// Side streams (bits) that a launch waits for in a capture.  A sweep that is timed
+// waits for all of them: its time is the sweep's alone, whatever runs beside it in a
+// step that is not timed.
+inline unsigned launch_joins(const Launch &L, bool sweep_timed)
+{
+    return L.kind == L_SWEEP && sweep_timed ? ~0u : L.join;
+}
+
 struct Plan {
     int device = 0;
     int pf = 0, ps = 0;           // buffer parities at the start

@@ -300,7 +300,9 @@ fsim_status fsim_time_steps(fsim_handle h, int nsteps, float *ms);
 /* Instrumented timing: run nsteps as CUDA-graph replays of the step graph
  * with event nodes around the fluid sweep launch (launch by launch while the
  * sweep's launch shape is still being tuned); *total_ms = elapsed device time
- * of the nsteps, *sweep_ms = summed device time of the nsteps sweep launches. */
+ * of the nsteps, *sweep_ms = summed device time of the nsteps sweep launches.
+ * Nothing runs beside a timed sweep: the graph's parallel branches are joined
+ * before it, which can make these steps a little longer than fsim_step's. */
 fsim_status fsim_time_sweep(fsim_handle h, int nsteps, float *total_ms, float *sweep_ms);
 /* Per-phase device time: run nsteps launch by launch with CUDA events around
  * every launch; ms[p] = summed time of phase p (FSIM_PHASE_CELL .. SOLID) for
