@@ -2262,7 +2262,7 @@ extern "C" fsim_status fsim_list_stats(fsim_handle h, int *enabled, int *builds,
     }
     if (enabled) *enabled = h->nl ? 1 : 0;
     if (builds) *builds = b;
-    if (capacity) *capacity = h->nl ? h->nl_cap : 0;
+    if (capacity) *capacity = h->nl ? h->nl_cap - kNlPad : 0; // without the filling at the species' boundaries
     if (check) *check = h->nl_check ? 1 : 0;
     return FSIM_OK;
 }
