@@ -342,8 +342,7 @@ FSIM_REBUILD_KERNEL(kg_scan_apply, ScanArgs, scan_apply_body, kScanThreads, bloc
 // 131,072 counts, 16 consecutive ones per thread, exchange their totals through
 // distributed shared memory and carry the sum to the next chunk.  One launch
 // instead of the three above, which at a few ten thousand cells are nothing but
-// launch latency (5.3 + 4.2 + 4.4 us); above kClusterScanMax cells, whose
-// chunks one cluster would walk one after another, the three passes are faster.
+// launch latency (5.3 + 4.2 + 4.4 us); scan_by_clusters says where it is taken.
 __global__ void __cluster_dims__(kScanCluster, 1, 1) __launch_bounds__(kScanThreads)
     kb_scan_cluster(const Item<ScanArgs> *__restrict__ items)
 {

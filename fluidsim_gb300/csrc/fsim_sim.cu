@@ -369,20 +369,36 @@ void add_sweep_launch(Plan &pl, ArenaBuilder &ab, const std::vector<Item<FluidSw
     pl.launches.push_back(L);
 }
 
+// One cluster per array of cell counts, or three passes over all of them (`arrays` of
+// them, the longest `most` counts, `total` together).  Step times in us, three passes
+// against clusters, for (cells, arrays): the cluster saves two launches while a chunk
+// holds the array: (2,160, 2) 112.9 / 107.4, (12,789, 2) 119.4 / 115.7, (67,392, 2)
+// 118.5 / 117.0, (12,789, 16) 146.1 / 145.0; then it walks its chunks one after another
+// and needs company: (181,984, 2) 121.1 / 125.4, (494,832, 2) 118.3 / 127.5 and (494,832,
+// 4) 159.2 / 163.9, but (234,256, 8) 184.0 / 175.3, (494,832, 8) 209.1 / 203.0, (67,392,
+// 64) 317.6 / 316.0, (494,832, 64) 802.4 / 743.9.  Many short arrays are worse, each
+// taking 8 blocks of 1024 threads: (2,160, 64) 163.3 / 172.6, (12,789, 64) 218.5 / 226.7.
+bool scan_by_clusters(size_t arrays, int most, long long total)
+{
+    if (most <= kClusterScanChunk && arrays <= 16) return true;
+    return arrays >= 8 && most <= kClusterScanMax && total >= 1ll << 20;
+}
+
 // The scans of the items' cell counts (blocks per item of the tile passes in sb,
-// of the partials pass in sp; 0: not scanned): one cluster per item, or three
-// passes where an item has too many cells for that.
+// of the partials pass in sp; 0: not scanned).
 void add_scan(Plan &pl, ArenaBuilder &ab, const std::vector<Item<ScanArgs>> &items, const std::vector<int> &sb,
               const std::vector<int> &sp)
 {
     std::vector<Item<ScanArgs>> scanned;
     int most = 0;
+    long long total = 0;
     for (size_t k = 0; k < items.size(); ++k)
         if (sp[k]) {
             scanned.push_back(items[k]);
             most = std::max(most, items[k].A.n);
+            total += items[k].A.n;
         }
-    if (most <= kClusterScanMax) {
+    if (scan_by_clusters(scanned.size(), most, total)) {
         add_launch(pl, ab, L_SCAN, scanned, std::vector<int>(scanned.size(), 1));
         return;
     }
