@@ -3354,13 +3354,12 @@ __global__ void k_offsets_in_cells(const DevParams P, float4 *__restrict__ pos, 
     pos[s] = p;
 }
 // Absolute position, density and pressure of a mixed-form particle, and back.  The
-// three read conversions carry about 46 bits as sums of two floats (Dekker's and
-// Knuth's exact sum and product) and round once: FP64 has 2 lanes an SM here, and
-// reading 4.2 M particles took 165 us for positions, 42 for densities and 383 for
-// pressures (expm1, log1p); now 33, 17 and 26, what their bytes take (the plain
-// form's 31 and 17).  On the CPU, 8 M draws of each over |delta| 1e-6 to 1 and gamma
-// 1 to 16, the largest error is 0.500000 ulp both ways and at most 2 values differ
-// from the doubles'.
+// three read conversions are those of FP64, rounded once; FP64 has 2 lanes an SM here
+// (4.2 M particles read 165 us of positions, 42 of densities, 383 of pressures, with
+// their expm1 and log1p), so they are first formed as sums of two floats (Dekker's and
+// Knuth's exact sum and product) within a known error, and only where that leaves the
+// rounding open (Ziv's test) in FP64: 35, 15 and 27 us, what their bytes take (the plain
+// form's 31 and 17).  The result is FP64's bit for bit.
 struct FloatPair {
     float hi, lo;
 };
@@ -3374,35 +3373,63 @@ __device__ __forceinline__ FloatPair exact_product(float a, float b)
     const float p = __fmul_rn(a, b);
     return {p, __fmaf_rn(a, b, -p)};
 }
-// an infinite sum has no error term (it would be NaN)
-__device__ __forceinline__ float rounded(float hi, float lo)
+// True where every value within t of hi + lo rounds to the same float, and that float.
+// (False for infinities and NaN, which have no error term, and where t is so small that
+// the error terms may have lost bits to underflow.)
+__device__ __forceinline__ bool rounds_alike(float hi, float lo, float t, float &out)
 {
-    return isinf(hi) ? hi : __fadd_rn(hi, lo);
+    out = __fadd_rn(hi, __fsub_rn(lo, t));
+    return out == __fadd_rn(hi, __fadd_rn(lo, t)) && t > 0x1p-124f;
 }
-__device__ __forceinline__ float from_cell(float cmin, float cdx, int c, float off)
+// (Calls, so that no FP64 is executed where it is not asked for: inlined, the few
+// instructions ran for every particle, 163 us of positions and 40 of densities.)
+__device__ __noinline__ float from_cell_fp64(float cmin, float cdx, int c, float off)
 {
+    return (float)((double)cmin + (double)c * (double)cdx + (double)off);
+}
+__device__ __noinline__ float density_fp64(float rho0, float delta) { return (float)((double)rho0 * (1.0 + (double)delta)); }
+// A position is the sum of three terms whose last places lie within 2^52 of the sum of
+// their sizes, so that FP64 forms it exactly, and so do two floats, unless a term's
+// error or a tiny offset leaves that open.  (An error bound alone would not do: offsets
+// have only some seven bits more than positions, so every hundredth sum is the middle
+// of two floats.)
+__device__ __forceinline__ float from_cell(const DevParams &P, int axis, int c, float off)
+{
+    const float cmin = P.cmin[axis], cdx = P.cdx[axis];
     const FloatPair p = exact_product((float)c, cdx), s = exact_sum(cmin, p.hi), u = exact_sum(s.hi, off);
-    return rounded(u.hi, __fadd_rn(__fadd_rn(s.lo, p.lo), u.lo));
+    const FloatPair l = exact_sum(s.lo, p.lo), m = exact_sum(l.hi, u.lo);
+    const float least = __fmul_rn(__fadd_rn(__fadd_rn(fabsf(cmin), fabsf(p.hi)), fabsf(off)), 0x1p-28f);
+    const bool exact = l.lo == 0.0f && m.lo == 0.0f && cdx >= least && (fabsf(cmin) >= least || cmin == 0.0f) &&
+                       (fabsf(off) >= least || off == 0.0f) && least > 0x1p-60f;
+    return exact ? __fadd_rn(u.hi, m.hi) : from_cell_fp64(cmin, cdx, c, off);
 }
 __device__ __forceinline__ float4 mixed_position(const DevParams &P, float4 off, int cell)
 {
     int cx, cy, cz;
     cell_xyz(P, cell, cx, cy, cz);
-    return make_float4(from_cell(P.cmin[0], P.cdx[0], cx, off.x), from_cell(P.cmin[1], P.cdx[1], cy, off.y),
-                       from_cell(P.cmin[2], P.cdx[2], cz, off.z), 0.0f);
+    return make_float4(from_cell(P, 0, cx, off.x), from_cell(P, 1, cy, off.y), from_cell(P, 2, cz, off.z), 0.0f);
 }
+// The pair's error is a rounding of terms below 2^-23 of the operands' sum, so below
+// 2^-46 of it, and FP64's below 2^-51.
+constexpr float kSumSlack = 0x1p-44f;
 __device__ __forceinline__ float mixed_density(const DevParams &P, float delta)
 {
     const FloatPair p = exact_product(P.rho0, delta), s = exact_sum(P.rho0, p.hi);
-    return rounded(s.hi, __fadd_rn(s.lo, p.lo));
+    const float t = __fmul_rn(__fadd_rn(fabsf(P.rho0), fabsf(p.hi)), kSumSlack);
+    float rho;
+    if (rounds_alike(s.hi, __fadd_rn(s.lo, p.lo), t, rho)) return rho;
+    return density_fp64(P.rho0, delta);
 }
 // Whole exponents up to 16 and |delta| < 1: q = (1 + delta)^gamma - 1 by
 // q <- q (1 + delta) + delta from q = delta, whose terms have one sign (nothing
-// cancels).  Any other exponent or delta takes the functions in FP64.
-constexpr float kWholeGammaMax = 16.0f;
+// cancels): each step adds at most 10 roundings of 2^-48 to q's relative error, all 15
+// of them less than 2^-40.  Any other exponent or delta takes the functions in FP64.
+constexpr float kWholeGammaMax = 16.0f, kPowerSlack = 0x1p-40f;
 __device__ __forceinline__ float mixed_pressure(const DevParams &P, float delta)
 {
-    if (P.gamma >= 1.0f && P.gamma <= kWholeGammaMax && P.gamma == truncf(P.gamma) && fabsf(delta) < 1.0f) {
+    if (delta == 0.0f) return fmaxf(__fmul_rn(P.rho2p, delta), P.min_p);
+    if (P.gamma >= 1.0f && P.gamma <= kWholeGammaMax && P.gamma == truncf(P.gamma) && fabsf(delta) < 1.0f &&
+        fabsf(delta) > 0x1p-80f) {
         const FloatPair t = exact_sum(1.0f, delta);
         FloatPair q = {delta, 0.0f};
         for (int k = (int)P.gamma; k > 1; --k) {
@@ -3412,7 +3439,9 @@ __device__ __forceinline__ float mixed_pressure(const DevParams &P, float delta)
             q.lo = __fsub_rn(e, __fsub_rn(q.hi, s.hi));
         }
         const FloatPair p = exact_product(P.rho2p, q.hi);
-        return fmaxf(rounded(p.hi, __fmaf_rn(P.rho2p, q.lo, p.lo)), P.min_p);
+        float pr;
+        if (rounds_alike(p.hi, __fmaf_rn(P.rho2p, q.lo, p.lo), __fmul_rn(fabsf(p.hi), kPowerSlack), pr))
+            return fmaxf(pr, P.min_p);
     }
     const double pr = (double)P.rho2p * expm1((double)P.gamma * log1p((double)delta));
     return (float)fmax(pr, (double)P.min_p);
