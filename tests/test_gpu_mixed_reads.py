@@ -1,7 +1,7 @@
 """The mixed form's positions, densities and pressures are read as FP64 forms them
 from what is held, rounded once: bit for bit, NaN and infinities included.
 
-The densities listed per exponent are states (of 33 million that FP32 densities can
+The densities listed per exponent are states (of 17 million that FP32 densities can
 reach) whose pressure lies so near the middle of two floats that a sum of two floats
 alone rounds to the other one.
 """
