@@ -2588,7 +2588,7 @@ constexpr int kForceAhead = 2; // list entries a lane of the force sweep loads a
 //
 // With pos_out the particle is also advanced, into the other of the solid's two
 // buffers (its neighbours still read this one): one launch fewer per sub-step.
-template <bool MIXED, int FLIST = 0>
+template <bool MIXED, int FLIST = 0, int AHEAD = kForceAhead>
 __device__ __forceinline__ void solid_force_body(const DevParams &P, const SolidArgs &S, int blk)
 {
     const int t = blk * blockDim.x + threadIdx.x;
@@ -2708,19 +2708,19 @@ __device__ __forceinline__ void solid_force_body(const DevParams &P, const Solid
         }
         const float4 ri = S.ref[i];
         const int o = S.orig[i];
-        // kForceAhead entries' loads in flight together, summed in list order
-        for (int e0 = S.nbr_off[o] + g, ee = S.nbr_off[o + 1]; e0 < ee; e0 += kForceAhead * kSolidGroup) {
-            int js[kForceAhead];
-            float4 q0[kForceAhead], q1[kForceAhead], q2[kForceAhead], q3[kForceAhead];
-            float2 q4[kForceAhead];
+        // AHEAD entries' loads in flight together, summed in list order
+        for (int e0 = S.nbr_off[o] + g, ee = S.nbr_off[o + 1]; e0 < ee; e0 += AHEAD * kSolidGroup) {
+            int js[AHEAD];
+            float4 q0[AHEAD], q1[AHEAD], q2[AHEAD], q3[AHEAD];
+            float2 q4[AHEAD];
 #pragma unroll
-            for (int u = 0; u < kForceAhead; ++u) {
+            for (int u = 0; u < AHEAD; ++u) {
                 const int e = e0 + u * kSolidGroup;
                 js[u] = e < ee ? S.nbr_slot[e] : -1;
                 FSIM_DCHECK(js[u] < S.n, 2048u, js[u] = -1);
             }
 #pragma unroll
-            for (int u = 0; u < kForceAhead; ++u) {
+            for (int u = 0; u < AHEAD; ++u) {
                 const int j = js[u] < 0 ? i : js[u];
                 const float *rec = S.PL + kPLStride * j;
                 load_solid_record(rec, q0[u], q1[u]);
@@ -2728,7 +2728,7 @@ __device__ __forceinline__ void solid_force_body(const DevParams &P, const Solid
                 q4[u] = *reinterpret_cast<const float2 *>(rec + 16);
             }
 #pragma unroll
-            for (int u = 0; u < kForceAhead; ++u) {
+            for (int u = 0; u < AHEAD; ++u) {
                 const bool in = js[u] >= 0;
                 const float4 xj = q3[u]; // position; velocity x
                 const float dX = __fsub_rn(q2[u].y, ri.x), dY = __fsub_rn(q2[u].z, ri.y), dZ = __fsub_rn(q2[u].w, ri.z);
@@ -2954,6 +2954,10 @@ __global__ void k_probe(const DevParams P, const ProbeArgs A)
 // every CTA resident at once; the barrier still gives up after a bounded wait
 // (FLAG_BARRIER_TIMEOUT on every instance, reported as FSIM_ETIMEOUT) instead
 // of spinning for ever.
+// Three CTAs of 256 threads an SM leave 80 registers a thread, and the force's two
+// entries ahead do not fit beside the walk of the 27 cells: with one, a step's solid
+// phase takes 311 us instead of 350 (27,000 particles, 5 sub-steps; 338 before there
+// were entries ahead), 179 instead of 194 (18,960) and 80 instead of 84 (128).
 constexpr unsigned kBarrierSpinLimit = 1u << 22; // x ~64 ns sleeps: about a quarter of a second and more
 
 // `limit`: polls before giving up (kBarrierSpinLimit unless the configuration
@@ -3014,7 +3018,7 @@ __global__ void __launch_bounds__(kBlock, 3) kb_solid_fused(const Item<SolidArgs
             const int inst = locate_instance(F.bstart_w, F.ninst, b);
             if (k >= items[inst].A.nsub) continue;
             const DevParams P = items[inst].P;
-            solid_force_body<MIXED>(P, items[inst].A, b - F.bstart_w[inst]);
+            solid_force_body<MIXED, 0, 1>(P, items[inst].A, b - F.bstart_w[inst]);
         }
         grid_sync(F.barrier, ok, F.polls);
         if (!ok) break;
