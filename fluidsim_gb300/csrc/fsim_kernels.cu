@@ -2558,13 +2558,15 @@ __device__ __forceinline__ void solid_update_particle(const DevParams &P, const 
     vel[i] = v;
 }
 
-// 32 bytes of a solid record with one load (an ordinary one: in the fused launch
-// the same kernel wrote them).
+// 32 bytes of a solid record with one load (an ordinary one, and one that the
+// compiler keeps behind earlier stores and barriers: in the fused launch the same
+// kernel wrote them).
 __device__ __forceinline__ void load_solid_record(const float *p, float4 &a, float4 &b)
 {
     asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-                 : "l"(p));
+                 : "l"(p)
+                 : "memory");
 }
 
 constexpr int kForceAhead = 2; // list entries a lane of the force sweep loads ahead
