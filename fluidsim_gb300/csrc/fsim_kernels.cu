@@ -2223,7 +2223,7 @@ FSIM_BATCHED_KERNEL(kb_virt_mixed, VirtArgs, virt_mixed_body, kBlock)
 // its z cell from the row's cell boundaries, its position relative to the
 // solid particle from the offset.
 struct RowMixed {
-    int b1, b2, z0;  // start of the row's 2nd and 3rd cell, first cell
+    int b1, b2;      // start of the row's 2nd and 3rd cell
     float sx, sy;    // solid offset minus the row's x/y cell shift
 };
 __device__ __forceinline__ int fluid_rel(const DevParams &P, const RowMixed &R, int t, float sz0, float4 q, float &dx,
@@ -2264,7 +2264,6 @@ __device__ __forceinline__ void solid_fluid_walk_m(const DevParams &P, const int
 #pragma unroll
     for (int r = 0; r < 9; ++r) {
         RowMixed R;
-        R.z0 = W.z0;
         R.b1 = W.b1[r];
         R.b2 = W.b2[r];
         R.sx = fmaf(-(float)(r / 3 - 1), P.cdx[0], sox);

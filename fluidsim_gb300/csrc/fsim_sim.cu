@@ -717,8 +717,13 @@ void plan_virt(Plan &pl, ArenaBuilder &ab, const std::vector<fsim_sim *> &m, int
 // of the whole plan.  One lane walks a list of ~12 groups, a chain of memory
 // latencies: while the particles leave most of the GPU's 152 x 2048 threads idle
 // more lanes shorten it, and beyond that they only repeat the per-particle work.
-// Sweep with 1 / 4 / 8 / 16 lanes: 1.4 k particles 26 / 22 / 17 / 14 us, 32 k 29 /
-// 31 / 38 / 55 us (64 and 63 us before the branch-free walk).
+// Sweep in us with 1 / 4 / 8 / 16 lanes, plain: 1,440 particles 22.4 / 21.8 / 16.3 /
+// 12.1, 4,096 24.4 / 21.9 / 16.6 / 14.3, 8,000 26.0 / 22.5 / 18.3 / 20.2, 12,000 23.5 /
+// 23.5 / 19.4 / 25.4, 16,250 25.5 / 23.5 / 23.4 / 30.2, 18,928 25.5 / 24.2 / 25.5 / 33.9,
+// 32,768 25.5 / 28.8 / 37.1 / 52.2; mixed: 1,440 35.7 / 29.6 / 23.7 / 19.6, 8,000 37.8 /
+// 31.6 / 25.5 / 23.5, 12,000 37.8 / 31.6 / 27.6 / 35.8, 16,250 40.6 / 34.2 / 30.3 / 39.8,
+// 32,768 38.4 / 39.8 / 50.0 / 67.8.  No choice here is slower than one lane; eight
+// lanes, which it does not offer, would be up to 5 us better from 8,000 to 16,000.
 int sweep_lane_shift(long long n)
 {
     return n <= 8192 ? 4 : n <= 16384 ? 2 : 0;
@@ -1962,8 +1967,11 @@ namespace {
 // Up to this many bytes the fields of a call move through one kernel over the
 // state and, to or from page-locked host memory, one that copies them all: with a
 // launch, an event, a stream switch and a copy per field they were host and launch
-// latency (42 us to read and 51 us to write the six fields of 32,000 particles).
-// Above, the copies of the first fields overlap the kernels of the later ones.
+// latency.  Six fields read / written in us, field by field against together, page-locked:
+// 59 kB 42 / 49 and 25 / 24, 1 MB 43 / 51 and 31 / 31, 4 MB 56 / 63 and 49 / 47; pageable
+// 4 MB 119 / 104 and 97 / 87.  The gain fades with the size (16 MB 123 / 123 and 119 /
+// 117, and in another run of half a million particles 118 / 115 and 128 / 124): above
+// 4 MB the copies of the first fields overlap the kernels of the later ones.
 constexpr size_t kStateBytes = 4u << 20;
 
 // What the driver knows of a host pointer (all zero: nothing).
@@ -2623,9 +2631,6 @@ fsim_status nl_restore(fsim_sim *h)
     NlState saved;
     CK(cudaMemcpyAsync(&saved, h->nl_state, sizeof saved, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    NlState now = saved;
-    now.rebuild = 1;
-    CK(upload(h->nl_state, &now, sizeof now, h->stream));
     const float4 *vpos = h->mixed ? h->v_abs : h->v_posr; // absolute wall positions
     if (h->nv) {
         launch_k_cells_of(blocks_for(h->nv, kBlock), h->stream, h->P, vpos, h->nv, h->v_icell, h->v_icxyz);

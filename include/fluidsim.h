@@ -312,13 +312,14 @@ fsim_status fsim_time_phases(fsim_handle h, int nsteps, float *ms, int n);
 fsim_status fsim_launches_per_step(fsim_handle h, int *n);
 
 /* Launch-shape autotuner of the fluid sweep (no counterpart in the reference).
- * The sweep has FSIM_SWEEP_SHAPES launch shapes (warps per block / per-lane
- * neighbour-list capacity in shared memory: 0 = 4/48, 1 = 4/32, 2 = 8/32), all
- * giving bit-identical results.  The first FSIM_SWEEP_SHAPES steps of a handle
- * (or of a batch) run one shape each, launch by launch, with CUDA events around
- * the sweep; the fastest is then used for the CUDA graph of every later step.
- * *chosen = the chosen shape (-1 while tuning), ms[k] = the timed sweep of
- * shape k (0 if not yet timed), for k < n. */
+ * The sweep has FSIM_SWEEP_SHAPES launch shapes, all giving bit-identical results:
+ * of the cell walk, warps per block / per-lane neighbour-list capacity in shared
+ * memory (0 = 4/48, 1 = 4/32, 2 = 8/32), of the list sweep, warps per block / blocks
+ * per SM (4/8, 4/9, 8/4; mixed form 4/8, 4/7, 8/3).  The first step of a handle (or
+ * of a batch) runs launch by launch and sweeps twice with each shape, with CUDA
+ * events around the sweeps; the fastest is then used for the CUDA graph of every
+ * later step.  *chosen = the chosen shape (-1 while tuning), ms[k] = the timed sweep
+ * of shape k (0 if not yet timed), for k < n. */
 #define FSIM_SWEEP_SHAPES 3
 fsim_status fsim_sweep_tuning(fsim_handle h, int *chosen, float *ms, int n);
 
