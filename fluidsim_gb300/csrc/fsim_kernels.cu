@@ -1165,8 +1165,8 @@ FSIM_REBUILD_KERNEL(kg_nl_build, NlBuildArgs, nl_build_body, kNlBuildWarps * 32,
 // fluidUpdate (src/fluid.cu:234-269) as in the stream sweep; the particle's
 // squared displacement since the build goes into the instance's running maximum.
 // With one lane per particle the plain form is bound by the L1's wavefronts (a
-// scattered 32-byte record per entry, 21-28 wavefronts per warp and entry of a
-// possible 8) and the mixed form by issue (110 instructions an entry).  Measured,
+// scattered 32-byte record per entry, 26 wavefronts per warp and entry of a
+// possible 8) and the mixed form by issue (104 instructions an entry).  Measured,
 // 4.2 M / 1 M / 32 k particles: plain 1.16 / 0.31 / 0.060 ms with a test and branch
 // per entry, 1.08 / 0.28 / 0.028 ms branch-free with the next group prefetched;
 // mixed 1.59 -> 1.38 ms at 4.2 M.
